@@ -135,17 +135,18 @@ size_t lsmf_operator_memory_consumption(const lsmf_op *op);
  * ExcNotImplemented).  Synchronous (one value copied to the host). */
 lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
 /* execution options (no reference counterpart; defaults are the fast path):
- * LSMF_OPT_BULK_PIPELINE: depth 1..3 of the shared-memory ring through which
- *   each warp streams its cell records with bulk copies; 0 = plain coalesced
- *   loads; -1 (default) = measured choice: 1 for tensor4, tensor4_ns and
- *   scalar_referential of degree 1 or 2 while a cell record fits in 24 KB,
- *   else 0.  The
- *   depth is reduced when the ring would not fit in shared memory.
+ * LSMF_OPT_BULK_PIPELINE: depth 1..3 of the shared-memory ring (2..4 record
+ *   slices, a slice holding one point of every x line of a warp's cells)
+ *   through which each warp streams its cell records with bulk copies; 0 =
+ *   plain coalesced loads; -1 (default) = measured choice: 2 slices, 3 for
+ *   tensor2 and scalar_referential of degree 4, plain loads for the scalar
+ *   variants of degree 2 and more.  The depth is reduced when the ring would
+ *   not fit in shared memory; cell lists (colour8) use plain loads.
  * LSMF_OPT_BASIC_KERNEL: 1 = the basic vmult kernel (per-warp shared-memory
  *   sweeps, plain loads); the stage mask of vmult always uses it.
- * LSMF_OPT_MAX_WARPS: cap on warps per block of the vmult kernel (1..8;
- *   0 = default: 8 for FP64 tensor2 and scalar, 2 for FP64
- *   scalar_referential, 4 otherwise).
+ * LSMF_OPT_MAX_WARPS: cap on warps per block of the vmult kernel (1..8, the
+ *   kernel uses at most 4; 0 = default: 4 at degree 4, 1 for tensor4_ns of
+ *   degree 1 and 2, 2 otherwise).
  * LSMF_OPT_WAIT_TRIES: bound of the pipelined kernel's wait for a cell
  *   record (mbarrier try_wait calls; -1 = default 2^22, seconds).  A wait
  *   that runs out sets the operator's device error word, lets every copy
@@ -164,16 +165,12 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   diagonal and the other cell loops of a nodesum operator use the
  *   colours).
  * LSMF_OPT_RECORD_PREFETCH: with plain record loads, 1 issues an L1
- *   prefetch of the cell's record before its sum-factorisation sweeps, 2 of
- *   the next cell's record, 0 none; -1 (default): 1, except 0 for the FP64
- *   scalar variant (measured).
- * LSMF_OPT_CELL_PAIRS: FP32 operators only: 1 = the vmult cell loop takes
- *   two cells per warp and runs their sum factorisation and point physics
- *   as the two halves of packed FP32x2 registers (one sm_100 f32x2
- *   instruction for both cells); 0 = one cell per warp; -1 (default) =
- *   measured choice (pairs for Q1 tensor2 / scalar formulation 1, Q2
- *   tensor2 / scalar formulation 1 / scalar_referential, Q4
- *   scalar_referential).  Ignored for FP64 operators.
+ *   prefetch of the records of a warp's cells before its sum-factorisation
+ *   sweeps, 2 of the next cells' records, 0 none; -1 (default): 1.
+ * LSMF_OPT_CELL_PAIRS: accepted (-1, 0, 1) and reported back, without effect:
+ *   FP32 tables interleave two cells, and the FP32 cell loop always runs the
+ *   sum factorisation and point physics of both as the halves of packed
+ *   FP32x2 registers (one sm_100 f32x2 instruction for both cells).
  * LSMF_OPT_CHUNKS: the atomic-scatter vmult cell loop split into 2..8
  *   contiguous cell chunks on streams of the operator's own, forked from
  *   and joined back into its stream: each chunk zeroes its range of dst and
@@ -182,8 +179,8 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   ends of the chunks' launches overlap other chunks' cell loops (levels
  *   with fewer than 1024 cells per chunk run in one piece); 1 = one launch;
  *   -1 (default) = measured choice: from 131,072 cells 8 for
- *   scalar_referential and tensor4_ns, 2 for tensor2, 4 otherwise; from
- *   32,768 cells 2; below that 1.  The operators a GMG object or a problem
+ *   scalar_referential and tensor4_ns, 4 otherwise; from 32,768 cells 2;
+ *   below that, and for tensor2, 1.  The operators a GMG object or a problem
  *   creates start at 1 (measured faster inside the Newton solve).  The
  *   chunks' streams and events are created by lsmf_operator_cache (and by
  *   this option on a cached operator), not by the vmult.

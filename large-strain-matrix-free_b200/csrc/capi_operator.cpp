@@ -1,4 +1,6 @@
 // C ABI: status strings, mesh and operator entry points (include/lsmf.h).
+#include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <new>
 #include <string>
@@ -179,23 +181,23 @@ lsmf_status lsmf_operator_create(lsmf_mesh *m, int level, lsmf_caching caching, 
   op->mesh = m; op->level = level; op->caching = caching; op->formulation = formulation;
   op->precision = precision;
   if (cudaGetDevice(&op->device) != cudaSuccess) { delete op; set_error("cudaGetDevice failed"); return LSMF_ERR_CUDA; }
-  op->ncomp = table_components(caching, formulation, precision);
   const Level &L = op->L();
   // scalar caching on affine cells: the reference inverse Jacobian is one
-  // 3x3 block per cell after the 11 per-point values (c, Eulerian inverse
-  // Jacobian, JxW); otherwise ncomp values per point.  Every record is
-  // padded at its end to a multiple of 16 bytes (bulk copies and aligned
-  // records), never with whole components.
+  // 3x3 block per cell beside the 11 per-point values (c, Eulerian inverse
+  // Jacobian, JxW).  The documented tables of tensor4 and tensor4_ns hold
+  // full tensors; the stored records keep the upper triangles and use the
+  // front of the buffer.
   op->ref_per_cell = caching == LSMF_CACHE_SCALAR && L.affine;
-  const int al = 16 / (int)op->elem();
-  if (op->ref_per_cell) {
-    op->ncomp = 11;
-    op->rec_elems = (11 * L.nq() + 9 + al - 1) / al * al;
-  } else {
-    op->rec_elems = (op->ncomp * L.nq() + al - 1) / al * al;
-  }
+  const int al = 16 / (int)op->elem(), extra = op->ref_per_cell ? 9 : 0;
+  auto padded = [&](int n) { return (n + al - 1) / al * al; };
+  const int stored = op->ref_per_cell ? 11 : record_components(caching);
+  const int documented = op->ref_per_cell ? 11 : table_components(caching);
+  const int B = cells_per_batch(L.p, precision), n_batches = (L.n_cells + B - 1) / B;
+  op->slice_elems = padded(stored * L.q * L.q * B);
+  op->batch_elems = L.q * op->slice_elems + padded(extra * B);
+  op->table_bytes = (size_t)L.n_cells * padded(documented * L.nq() + extra) * op->elem();
   lsmf_status s;
-  if ((s = op->d_table.alloc((size_t)L.n_cells * op->rec_elems * op->elem())) != LSMF_OK ||
+  if ((s = op->d_table.alloc(std::max(op->table_bytes, (size_t)n_batches * op->batch_elems * op->elem()))) != LSMF_OK ||
       (s = op->d_diag.alloc((size_t)L.n_dofs() * op->elem())) != LSMF_OK ||
       (s = op->d_inv_diag.alloc((size_t)L.n_dofs() * op->elem())) != LSMF_OK ||
       (s = op->d_flag.alloc(1)) != LSMF_OK) {
@@ -386,7 +388,7 @@ size_t lsmf_operator_memory_consumption(const lsmf_op *op) {
   // mf_nh_operator.h:300-328)
   if (!op) return 0;
   const Level &L = op->L();
-  return op->d_table.n + L.d_cell_nodes.n * sizeof(int) + L.d_X.n * sizeof(double);
+  return op->table_bytes + L.d_cell_nodes.n * sizeof(int) + L.d_X.n * sizeof(double);
 }
 
 lsmf_status lsmf_operator_get_table(lsmf_op *op, int which, double *host, size_t *count) {
@@ -421,7 +423,10 @@ lsmf_status lsmf_operator_get_table(lsmf_op *op, int which, double *host, size_t
   for (int cell = 0; cell < L.n_cells; ++cell)
     for (int q = 0; q < nq; ++q)
       for (int k = 0; k < nk; ++k) {
-        const size_t src = (size_t)cell * op->rec_elems + (size_t)(c0 + k) * nq + q;
+        // the full matrices of tables 3 and 7 from their stored upper triangles
+        const int N = which == 3 ? 6 : 9, i = k / N, j = k % N;
+        const int kk = which == 3 || which == 7 ? std::min(i, j) * N - std::min(i, j) * (std::min(i, j) - 1) / 2 + std::abs(j - i) : k;
+        const size_t src = record_index(op, cell, c0 + kk, q);
         const double v = op->precision == LSMF_FP64 ? ((const double *)raw.data())[src]
                                                     : (double)((const float *)raw.data())[src];
         host[((size_t)cell * nq + q) * nk + k] = v;

@@ -1,11 +1,13 @@
 // Device building blocks of the cell kernels: warp-cooperative sum
 // factorisation and the quadrature-point physics of the Neo-Hookean tangent.
 //
-// Execution model: one warp owns one cell at a time.  Lanes stride over the
-// work items of each tensor-product sweep; intermediate tensors live in a
-// per-warp shared-memory slab, so only __syncwarp() separates the sweeps.
-// Quadrature point q belongs to lane q % 32 (QPL = ceil(Q^3/32) points per
-// lane), so everything per quadrature point stays in registers.
+// Execution model of the production kernels (SFC): a cell is worked on by
+// Q^2 lanes of a warp, each holding whole lines of the cell (a z line of
+// nodes, then a z line of points by x / y, finally an x line of quadrature
+// points), so a warp carries 32 / Q^2 cells (8, 3, 2, 1 for Q = 2..5) and
+// only the two transposes between the three sweeps go through a per-warp
+// shared-memory slab.  The basic kernel (SF) keeps one cell per warp with
+// lanes striding over the work items of each sweep.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -20,25 +22,62 @@ enum Variant {
 };
 __host__ __device__ constexpr bool variant_referential(int v) { return v == VAR_SCALAR_REF || v == VAR_TENSOR4_NS; }
 
-// Record layout per cell: [comp][qp], ncomp * Q^3 values, the record padded
-// at its end to a multiple of 16 bytes.  The first 9 components are the
-// inverse Jacobian (row-major) of the frame the variant integrates in:
-// Eulerian for tensor4 / tensor2 / scalar, reference for scalar_referential
-// and tensor4_ns.  The point result of tensor4, tensor2 and tensor4_ns is
-// linear in their cached coefficients, so those are stored multiplied by
-// JxW and follow from component 9: tensor4 JxW tau/J (6) + JxW C (36);
-// tensor2 JxW c1, JxW c2, JxW tau/J (6); tensor4_ns JxW dP/dF (81).  The
-// scalar variants keep JxW as component 9, then: scalar c + reference
-// inverse Jacobian (9); scalar_referential c + u at the point (3).
+// Components of the cell record.  The first 9 are the inverse Jacobian
+// (row-major) of the frame the variant integrates in: Eulerian for tensor4 /
+// tensor2 / scalar, reference for scalar_referential and tensor4_ns.  The
+// point result of tensor4, tensor2 and tensor4_ns is linear in their cached
+// coefficients, so those are stored multiplied by JxW and follow from
+// component 9: tensor4 JxW tau/J (6) + JxW C (21: the 6x6 matrix acting on
+// sym(g) is symmetric, its upper triangle is kept); tensor2 JxW c1, JxW c2,
+// JxW tau/J (6); tensor4_ns JxW dP/dF (45: the 9x9 matrix of a hyperelastic
+// material is symmetric, its upper triangle is kept).  The scalar variants
+// keep JxW as component 9, then: scalar c + reference inverse Jacobian (9);
+// scalar_referential c + u at the point (3).
+// The records are interleaved over the cells a warp works on together, see
+// RecLayout.
 constexpr int C_JINV = 0, C_JXW = 9, C_VAR = 10;
 __host__ __device__ constexpr bool variant_folds_jxw(int v) {
   return v == VAR_TENSOR4 || v == VAR_TENSOR2 || v == VAR_TENSOR4_NS;
 }
 // first coefficient component
 __host__ __device__ constexpr int variant_cvar(int v) { return variant_folds_jxw(v) ? C_JXW : C_VAR; }
+// components a point keeps (scalar on affine cells: 11, and the reference
+// inverse Jacobian once per cell)
 __host__ __device__ constexpr int variant_ncomp(int v) {
-  return v == VAR_TENSOR4 ? 51 : v == VAR_TENSOR2 ? 17 : v == VAR_SCALAR_REF ? 14 : v == VAR_TENSOR4_NS ? 90 : 20;
+  return v == VAR_TENSOR4 ? 36 : v == VAR_TENSOR2 ? 17 : v == VAR_SCALAR_REF ? 14 : v == VAR_TENSOR4_NS ? 54 : 20;
 }
+
+// The cell records of the device table.  A batch of B consecutive cells (the
+// cells one warp works on at a time: CPW groups of L = Q^2 lanes, and for
+// FP32 tables TH = 2 cells per lane, the halves of a packed register) is
+// stored as Q slices, one per point of the lanes' x lines, each
+// [component][lane][half]: a component's load is one contiguous 256-byte
+// (216 at Q = 3) access of the warp, and a slice is one contiguous block for
+// the bulk-copy ring.  With [cell][comp][point] records the three cells of a
+// Q2 warp would touch three 72-byte pieces per load.  A slice takes
+// slice_elems values (its components, padded to 16 bytes), a batch
+// batch_elems (Q slices, then for scalar caching on affine cells the
+// reference inverse Jacobians of its cells, padded to 16 bytes).
+template <int P, int Q, int TH>
+struct RecLayout {
+  static constexpr int L = Q * Q, CPW = 32 / L, LW = CPW * L, B = CPW * TH;
+  static constexpr int TS = TH, CS = LW * TH;  // strides of lane, component
+  static constexpr int RS = CPW * TH;          // stride of the entries of the reference inverse Jacobian
+  // first value of a cell (slice 0, component 0, lane 0)
+  static __host__ __device__ __forceinline__ size_t base(int cell, int batch_elems) {
+    const int b = cell / B, e = cell - b * B;
+    return (size_t)b * batch_elems + (e / TH) * (L * TH) + e % TH;
+  }
+  // offset of point q = (qz Q + qy) Q + qx
+  static __host__ __device__ __forceinline__ int q_off(int q, int slice_elems) {
+    return (q % Q) * slice_elems + (q / Q) * TS;
+  }
+  // first entry of a cell's reference inverse Jacobian
+  static __host__ __device__ __forceinline__ size_t ref(int cell, int batch_elems, int slice_elems) {
+    const int b = cell / B, e = cell - b * B;
+    return (size_t)b * batch_elems + (size_t)Q * slice_elems + e;
+  }
+};
 
 template <int P, int Q>
 struct Tab {
@@ -55,25 +94,26 @@ struct TabT {
   T Dc[Q][Q];  // collocation derivative on the Gauss points
 };
 
-// scalar_referential: F = I + Grad u from the displacement stored at the
-// points of the cell record (collocation derivative, the
-// FEEvaluationImplCollocation step of mf_nh_operator.h:1271-1300) and the
-// reference inverse Jacobian
-// (R: the record, a pointer or an accessor with operator[] and + offset)
-template <int Q, typename T, typename DC, typename R>
-__device__ __forceinline__ void collocation_F(const R &rec, int q, const DC &Dc, const T Ji[3][3], T F[3][3]) {
-  constexpr int NQ = Q * Q * Q;
-  const int qx = q % Q, qy = (q / Q) % Q, qz = q / (Q * Q);
+// scalar_referential: F = I + Grad u at point (qx, qy, qz) from the
+// displacement stored at the points of the cell record (collocation
+// derivative, the FEEvaluationImplCollocation step of
+// mf_nh_operator.h:1271-1300) and the reference inverse Jacobian.
+// ux[c][m]: values along the point's x line; slice: the cell's record at the
+// point's slice and lane 0 (a pointer, or an accessor with operator[] and
+// + offset); CS, TS: its component and lane strides.
+template <int Q, int CS, int TS, typename T, typename DC, typename R>
+__device__ __forceinline__ void collocation_F(const T ux[3][Q], const R &slice, int qx, int qy, int qz, const DC &Dc,
+                                              const T Ji[3][3], T F[3][3]) {
   T G[3][3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const auto u = rec + (C_VAR + 1 + c) * NQ;
+    const auto u = slice + (C_VAR + 1 + c) * CS;
     T gx = 0, gy = 0, gz = 0;
 #pragma unroll
     for (int m = 0; m < Q; ++m) {
-      gx += T(Dc[qx][m]) * u[(qz * Q + qy) * Q + m];
-      gy += T(Dc[qy][m]) * u[(qz * Q + m) * Q + qx];
-      gz += T(Dc[qz][m]) * u[(m * Q + qy) * Q + qx];
+      gx += T(Dc[qx][m]) * ux[c][m];
+      gy += T(Dc[qy][m]) * u[(qz * Q + m) * TS];
+      gz += T(Dc[qz][m]) * u[(m * Q + qy) * TS];
     }
     G[c][0] = gx; G[c][1] = gy; G[c][2] = gz;
   }
@@ -84,328 +124,210 @@ __device__ __forceinline__ void collocation_F(const R &rec, int q, const DC &Dc,
       F[c][d] = G[c][0] * Ji[0][d] + G[c][1] * Ji[1][d] + G[c][2] * Ji[2][d] + (c == d ? T(1) : T(0));
 }
 
-// Shared-memory layout of the row sweeps, chosen per (degree, element size)
-// by a wavefront count of every warp access of the sweeps (32 banks of 4
-// bytes; 8-byte words served per half warp) so that the transposes between
-// sweeps are free of bank conflicts where the unpadded tensors allow it:
-//   X0..X2: order in which the x sweep (and the gather / scatter) enumerates
-//           its rows (c, k, j) over the lanes, fastest first (ids 0 = c,
-//           1 = k, 2 = j);
-//   Y0..Y2: the same for the y sweep rows (0 = c, 1 = k, 2 = qx);
-//   Z0..Z2: the same for the z sweep rows (0 = c, 1 = qy, 2 = qx);
-//   AC, AK, AJ, AQ: strides of the x-sweep output A[c][k][j][qx] (and of
-//           the y-sweep output of integrate);
-//   BC, BK, BY, BX: strides of the y-sweep output B[c][k][qy][qx] (and of
-//           the z-sweep output of integrate);
-//   NQP:    stride of the 9 per-point blocks (c, e) of the point tensor.
-template <int P, int ES>
-struct SFRLayout {  // generic: the natural orders, no padding
-  static constexpr int N1 = P + 1;
-  static constexpr int X0 = 2, X1 = 1, X2 = 0, Y0 = 2, Y1 = 1, Y2 = 0, Z0 = 2, Z1 = 1, Z2 = 0;
-  static constexpr int AC = N1 * N1 * N1, AK = N1 * N1, AJ = N1, AQ = 1;
-  static constexpr int BC = N1 * N1 * N1, BK = N1 * N1, BY = N1, BX = 1;
-  static constexpr int NQP = N1 * N1 * N1;
-};
-// Q1 / Q2 with 8-byte (FP64) and 4-byte (FP32) entries.  Wavefronts per
-// cell of the sweeps and point accesses, natural -> chosen: Q2 FP64 306 ->
-// 192 and Q2 FP32 162 -> 96 (both conflict-free), Q1 FP64 122 -> 110.  For
-// Q3 / Q4 the best orders with unpadded A / B save under 10 % of the
-// wavefronts and measured slower (FP32 Q4 0.73 -> 1.08 ms), so they keep the
-// natural layout.
-template <int P, int Y0_, int Y1_, int Y2_, int Z0_, int Z1_, int Z2_, int NQP_>
-struct SFRLayoutYZ : SFRLayout<P, 0> {
-  static constexpr int Y0 = Y0_, Y1 = Y1_, Y2 = Y2_, Z0 = Z0_, Z1 = Z1_, Z2 = Z2_, NQP = NQP_;
-};
-template <> struct SFRLayout<1, 8> : SFRLayoutYZ<1, 0, 1, 2, 0, 1, 2, 9> {};
-template <> struct SFRLayout<1, 4> : SFRLayoutYZ<1, 0, 1, 2, 0, 1, 2, 8> {};
-template <> struct SFRLayout<2, 8> : SFRLayoutYZ<2, 1, 0, 2, 0, 2, 1, 41> {};
-// FP32 Q2: x rows with the component fastest (the three components of a node
-// are gathered by neighbouring lanes), A[j][c][k][qx], B[k][c][qx][qy]
-template <> struct SFRLayout<2, 4> : SFRLayoutYZ<2, 0, 1, 2, 0, 1, 2, 29> {
-  static constexpr int X0 = 0, X1 = 1, X2 = 2;
-  static constexpr int AC = 9, AK = 3, AJ = 27, AQ = 1;
-  static constexpr int BC = 9, BK = 27, BY = 1, BX = 3;
-};
-// Q4 FP32: conflict-free sweeps with reordered intermediate tensors
-// (A[qx][c][k][j], B[qy][qx][c][k]).  The conflict-free orders found for Q3
-// and for Q4 FP64 measured slower for tensor4 (FP64 Q4 1.36 -> 1.98 ms), so
-// those keep the natural layout.
-template <> struct SFRLayout<4, 4> : SFRLayoutYZ<4, 1, 0, 2, 0, 2, 1, 153> {
-  static constexpr int AC = 25, AK = 5, AJ = 1, AQ = 75;
-  static constexpr int BC = 5, BK = 1, BY = 75, BX = 15;
-};
-
-// row -> its three indices (by id) for an enumeration (I0 fastest, I2
-// slowest) over index ranges D[id]
-template <int I0, int I1, int I2, int DA, int DB, int DC>
-__device__ __forceinline__ void decode_row(int row, int idx[3]) {
-  constexpr int D[3] = {DA, DB, DC};
-  idx[I0] = row % D[I0];
-  idx[I1] = (row / D[I0]) % D[I1];
-  idx[I2] = row / (D[I0] * D[I1]);
-}
-
-// Visit the rows lane, lane + 32, ... of a sweep with NR rows: f(row, act).
-// CLAMP with NR <= 32: every lane takes one row, lanes past the end repeat
-// the last row (act = false: they compute, but store nothing), so the sweep
-// has no divergent branch.
-template <int NR, bool CLAMP, typename F>
-__device__ __forceinline__ void rows_of_lane(int lane, F &&f) {
-  if constexpr (CLAMP && NR <= 32) {
-    f(lane < NR ? lane : NR - 1, lane < NR);
-  } else {
-    for (int row = lane; row < NR; row += 32) f(row, true);
+// Place of a lane in its warp: cell slot r, line (a, b) of the cell, and the
+// lane id clamped to the working lanes.  At Q = 3 / 5 the lanes 27..31 /
+// 25..31 repeat the last working lane: they read and write the same
+// shared-memory words with the same values, so the sweeps need no branches;
+// only stores to global memory test `act`.
+template <int Q>
+struct LanePos {
+  static constexpr int L = Q * Q, CPW = 32 / L, LW = CPW * L;
+  int ln, r, t, a, b;
+  bool act;
+  __device__ __forceinline__ LanePos() {
+    const int lane = threadIdx.x & 31;
+    act = lane < LW;
+    ln = act ? lane : LW - 1;
+    r = ln / L;
+    t = ln - r * L;
+    a = t / Q;
+    b = t - a * Q;
   }
-}
+};
 
-// Sum factorisation with one 1D line per lane ("row" sweeps).  Each sweep
-// maps lane -> row of the tensor it produces and unrolls the 1D contraction
-// completely; shared memory only carries the transposes between sweeps.
-//   eval:      src rows (c,k,j) in registers -> A (x) -> B (y) -> G (z) ->
-//              per-point gradient registers
-//   integrate: per-point H -> Z (z) -> Y (y) -> per-row nodal values (x)
-// Slab layout (elements of T): [9*NQ points][2*NA][3*NB].
-// CLAMP: with at most 32 rows / points per sweep, the lanes past the end
-// repeat the last row or point and only their stores are skipped (no
-// divergent branches; measured faster for the scalar variants, whose
-// kernels carry the most registers, and slower for tensor2)
-template <int P, int Q, typename T, bool CLAMP = false>
-struct SFR {
-  using LY = SFRLayout<P, (int)sizeof(T)>;
+// Sum factorisation with whole lines per lane, Q^2 lanes per cell.
+//   eval:      lane (j, i) holds the nodes k = 0..P of its z line; the z
+//              sweep runs in registers, its two fields (value, derivative)
+//              are transposed to lanes (qz, i) for the y sweep, and its
+//              three fields to lanes (qz, qy) for the x sweep, which leaves
+//              the reference gradients of an x line of points in registers.
+//   integrate: the transpose, back to nodal values of z lines.
+// Per cell and direction 2 * 3 + 3 * 3 words per lane go through shared
+// memory each way; the row-per-lane form this replaces also moved the 9
+// gradient components of every point (96 against 60 shared-memory accesses
+// per lane and cell at Q = 3), and its kernels were bound by exactly that
+// traffic.  The slab rows are 32 + Q (z / y transposes) and 33 (y / x)
+// entries apart: = Q and = 1 modulo 16 and 32, which makes every access of
+// both sides of a transpose conflict-free for 8- and 4-byte entries.
+template <int P, int Q, typename T>
+struct SFC {
   static constexpr int N1 = P + 1, NN = N1 * N1 * N1, NQ = Q * Q * Q;
-  static constexpr int NQP = (Q == P + 1) ? LY::NQP : NQ;  // point-block stride
-  static constexpr int QPL = (NQ + 31) / 32;
-  static constexpr int XR = 3 * N1 * N1;      // x rows (c,k,j)
-  static constexpr int YR = 3 * N1 * Q;       // y rows (c,k,qx)
-  static constexpr int ZR = 3 * Q * Q;        // z rows (c,qy,qx)
-  static constexpr int RPL = (XR + 31) / 32;  // x rows per lane
-  static constexpr int NA = 3 * N1 * N1 * Q;
-  static constexpr int NB = 3 * N1 * Q * Q;
-  static constexpr int SZP = 9 * NQP;
-  static constexpr int SZ = SZP + 2 * NA + 3 * NB;
+  static_assert(N1 == Q, "q = p + 1");
+  static constexpr int L = Q * Q, CPW = 32 / L, LW = CPW * L;
+  static constexpr int RA = 32 + Q, RB = 33;
+  static constexpr int BA = Q * RA, BB = Q * RB;              // one component of one field
+  static constexpr int SZ = 6 * BA > 9 * BB ? 6 * BA : 9 * BB;  // per-warp slab (elements of T)
 
-  // v[r][i]: value of component c at node (i, j, k) for x row r = lane + 32 r;
-  // the reference gradients are left in the point block of the slab,
-  // Pt[(c * 3 + e) * NQP + q]
-  // x row (component c, node line (k, j)) of a lane: row -> (c, k, j)
-  static __device__ __forceinline__ void x_row(int row, int &c, int &k, int &j) {
-    int ix[3];
-    decode_row<LY::X0, LY::X1, LY::X2, 3, N1, N1>(row, ix);
-    c = ix[0]; k = ix[1]; j = ix[2];
-  }
-  static __device__ __forceinline__ int a_at(int c, int k, int j, int qx) {
-    return c * LY::AC + k * LY::AK + j * LY::AJ + qx * LY::AQ;
-  }
-  static __device__ __forceinline__ int b_at(int c, int k, int qy, int qx) {
-    return c * LY::BC + k * LY::BK + qy * LY::BY + qx * LY::BX;
-  }
-
-  static __device__ __forceinline__ void eval_pt(const TabT<P, Q, T> &t, const T v[RPL][N1], T *slab, int lane) {
-    T *Pt = slab, *A = slab + SZP, *B = A + 2 * NA;
+  // v[c][k]: value of component c at node k of the lane's z line ->
+  // G[s][c][e]: reference gradient at point s of the lane's x line, and with
+  // Vq the values Vq[s][c] there
+  static __device__ __forceinline__ void eval(const TabT<P, Q, T> &tb, const T v[3][N1], T *slab, const LanePos<Q> &lp,
+                                              T G[Q][3][3], T (*Vq)[3] = nullptr) {
+    __syncwarp();  // the slab's previous readers are done
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row0 = lane + 32 * r;
-      if ((CLAMP && XR <= 32) || row0 < XR) {
-        const bool act = row0 < XR;
-        int c, k, j;
-        x_row(act ? row0 : XR - 1, c, k, j);
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int qx = 0; qx < Q; ++qx) {
-          T s0 = 0, s1 = 0;
+      for (int qz = 0; qz < Q; ++qz) {
+        T s0 = 0, s1 = 0;
 #pragma unroll
-          for (int i = 0; i < N1; ++i) {
-            s0 += t.N[qx][i] * v[r][i];
-            s1 += t.D[qx][i] * v[r][i];
-          }
-          if (act) {
-            A[a_at(c, k, j, qx)] = s0;
-            A[NA + a_at(c, k, j, qx)] = s1;
-          }
+        for (int k = 0; k < N1; ++k) {
+          s0 += tb.N[qz][k] * v[c][k];
+          s1 += tb.D[qz][k] * v[c][k];
         }
+        slab[c * BA + qz * RA + lp.ln] = s0;
+        slab[(3 + c) * BA + qz * RA + lp.ln] = s1;
       }
+    __syncwarp();
+    // lane (qz, i) = (a, b)
+    T a0[3][N1], a1[3][N1];
+    {
+      const T *A = slab + lp.r * L + lp.b + lp.a * RA;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int j = 0; j < N1; ++j) {
+          a0[c][j] = A[c * BA + j * Q];
+          a1[c][j] = A[(3 + c) * BA + j * Q];
+        }
     }
     __syncwarp();
-    rows_of_lane<YR, CLAMP>(lane, [&](int row, bool act) {
-      int ix[3];
-      decode_row<LY::Y0, LY::Y1, LY::Y2, 3, N1, Q>(row, ix);
-      const int c = ix[0], k = ix[1], qx = ix[2];
-      T a0[N1], a1[N1];
 #pragma unroll
-      for (int j = 0; j < N1; ++j) {
-        a0[j] = A[a_at(c, k, j, qx)];
-        a1[j] = A[NA + a_at(c, k, j, qx)];
-      }
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
       for (int qy = 0; qy < Q; ++qy) {
         T s00 = 0, s01 = 0, s10 = 0;
 #pragma unroll
         for (int j = 0; j < N1; ++j) {
-          s00 += t.N[qy][j] * a0[j];
-          s01 += t.D[qy][j] * a0[j];
-          s10 += t.N[qy][j] * a1[j];
+          s00 += tb.N[qy][j] * a0[c][j];
+          s01 += tb.D[qy][j] * a0[c][j];
+          s10 += tb.N[qy][j] * a1[c][j];
         }
-        const int b = b_at(c, k, qy, qx);
-        if (act) {
-          B[b] = s00;
-          B[NB + b] = s01;
-          B[2 * NB + b] = s10;
-        }
+        slab[c * BB + qy * RB + lp.ln] = s00;
+        slab[(3 + c) * BB + qy * RB + lp.ln] = s01;
+        slab[(6 + c) * BB + qy * RB + lp.ln] = s10;
       }
-    });
     __syncwarp();
-    rows_of_lane<ZR, CLAMP>(lane, [&](int row, bool act) {
-      int ix[3];
-      decode_row<LY::Z0, LY::Z1, LY::Z2, 3, Q, Q>(row, ix);
-      const int qyx = ix[1] * Q + ix[2], c = ix[0];
-      T b00[N1], b01[N1], b10[N1];
+    // lane (qz, qy) = (a, b)
+    const T *B = slab + lp.r * L + lp.a * Q + lp.b * RB;
 #pragma unroll
-      for (int k = 0; k < N1; ++k) {
-        const int b = b_at(c, k, ix[1], ix[2]);
-        b00[k] = B[b];
-        b01[k] = B[NB + b];
-        b10[k] = B[2 * NB + b];
+    for (int c = 0; c < 3; ++c) {
+      T b0[N1], by[N1], bz[N1];
+#pragma unroll
+      for (int i = 0; i < N1; ++i) {
+        b0[i] = B[c * BB + i];
+        by[i] = B[(3 + c) * BB + i];
+        bz[i] = B[(6 + c) * BB + i];
       }
 #pragma unroll
-      for (int qz = 0; qz < Q; ++qz) {
+      for (int s = 0; s < Q; ++s) {
         T gx = 0, gy = 0, gz = 0;
 #pragma unroll
-        for (int k = 0; k < N1; ++k) {
-          gx += t.N[qz][k] * b10[k];
-          gy += t.N[qz][k] * b01[k];
-          gz += t.D[qz][k] * b00[k];
+        for (int i = 0; i < N1; ++i) {
+          gx += tb.D[s][i] * b0[i];
+          gy += tb.N[s][i] * by[i];
+          gz += tb.N[s][i] * bz[i];
         }
-        const int q = qz * Q * Q + qyx;
-        if (act) {
-          Pt[(c * 3 + 0) * NQP + q] = gx;
-          Pt[(c * 3 + 1) * NQP + q] = gy;
-          Pt[(c * 3 + 2) * NQP + q] = gz;
+        G[s][c][0] = gx;
+        G[s][c][1] = gy;
+        G[s][c][2] = gz;
+        if (Vq) {
+          T x = 0;
+#pragma unroll
+          for (int i = 0; i < N1; ++i) x += tb.N[s][i] * b0[i];
+          Vq[s][c] = x;
         }
       }
-    });
-    __syncwarp();
+    }
   }
 
-  // eval_pt, then the gradients of the points lane + 32 l into registers
-  static __device__ __forceinline__ void eval(const TabT<P, Q, T> &t, const T v[RPL][N1], T *slab, int lane,
-                                              T G[QPL][3][3]) {
-    eval_pt(t, v, slab, lane);
-    const T *Pt = slab;
+  // H[s][c][e] at the points of the lane's x line -> out[c][k]: nodal value
+  // of component c at node k of the lane's z line
+  static __device__ __forceinline__ void integrate(const TabT<P, Q, T> &tb, const T H[Q][3][3], T *slab,
+                                                   const LanePos<Q> &lp, T out[3][N1]) {
+    __syncwarp();
 #pragma unroll
-    for (int l = 0; l < QPL; ++l) {
-      // lanes past the last point read the last point (no divergent branch)
-      const int q = (CLAMP && NQ <= 32) ? (lane < NQ ? lane : NQ - 1) : lane + 32 * l;
-      if ((CLAMP && NQ <= 32) || q < NQ) {
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+      for (int i = 0; i < N1; ++i) {
+        T zx = 0, zy = 0, zz = 0;
 #pragma unroll
-          for (int e = 0; e < 3; ++e) G[l][c][e] = Pt[(c * 3 + e) * NQP + q];
+        for (int s = 0; s < Q; ++s) {
+          zx += tb.D[s][i] * H[s][c][0];
+          zy += tb.N[s][i] * H[s][c][1];
+          zz += tb.N[s][i] * H[s][c][2];
+        }
+        slab[c * BB + i * RB + lp.ln] = zx;
+        slab[(3 + c) * BB + i * RB + lp.ln] = zy;
+        slab[(6 + c) * BB + i * RB + lp.ln] = zz;
+      }
+    __syncwarp();
+    // lane (qz, i) = (a, b)
+    T o1[3][N1], o2[3][N1];
+    {
+      const T *Z = slab + lp.r * L + lp.a * Q + lp.b * RB;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        T zx[Q], zy[Q], zz[Q];
+#pragma unroll
+        for (int qy = 0; qy < Q; ++qy) {
+          zx[qy] = Z[c * BB + qy];
+          zy[qy] = Z[(3 + c) * BB + qy];
+          zz[qy] = Z[(6 + c) * BB + qy];
+        }
+#pragma unroll
+        for (int j = 0; j < N1; ++j) {
+          T s1 = 0, s2 = 0;
+#pragma unroll
+          for (int qy = 0; qy < Q; ++qy) {
+            s1 += tb.N[qy][j] * zx[qy];
+            s1 += tb.D[qy][j] * zy[qy];
+            s2 += tb.N[qy][j] * zz[qy];
+          }
+          o1[c][j] = s1;
+          o2[c][j] = s2;
+        }
       }
     }
     __syncwarp();
-  }
-
-  // per-point H -> out[r][i] for x row r (component c, node (i, j, k))
-  static __device__ __forceinline__ void integrate(const TabT<P, Q, T> &t, const T H[QPL][3][3], T *slab, int lane,
-                                                   T out[RPL][N1]) {
-    T *Pt = slab;
 #pragma unroll
-    for (int l = 0; l < QPL; ++l) {
-      const int q = lane + 32 * l;
-      if (q < NQ) {
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int e = 0; e < 3; ++e) Pt[(c * 3 + e) * NQP + q] = H[l][c][e];
+      for (int j = 0; j < N1; ++j) {
+        slab[c * BA + j * RA + lp.ln] = o1[c][j];
+        slab[(3 + c) * BA + j * RA + lp.ln] = o2[c][j];
       }
-    }
-    integrate_pt(t, slab, lane, out);
-  }
-
-  // the same with H already in the point block of the slab
-  static __device__ __forceinline__ void integrate_pt(const TabT<P, Q, T> &t, T *slab, int lane, T out[RPL][N1]) {
-    T *Pt = slab, *Y = slab + SZP, *Z = Y + 2 * NA;
     __syncwarp();
-    rows_of_lane<ZR, CLAMP>(lane, [&](int row, bool act) {
-      int ix[3];
-      decode_row<LY::Z0, LY::Z1, LY::Z2, 3, Q, Q>(row, ix);
-      const int qyx = ix[1] * Q + ix[2], c = ix[0];
-      T hx[Q], hy[Q], hz[Q];
+    // lane (j, i) = (a, b)
+    const T *Y = slab + lp.r * L + lp.b + lp.a * RA;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      T y1[Q], y2[Q];
 #pragma unroll
       for (int qz = 0; qz < Q; ++qz) {
-        const int q = qz * Q * Q + qyx;
-        hx[qz] = Pt[(c * 3 + 0) * NQP + q];
-        hy[qz] = Pt[(c * 3 + 1) * NQP + q];
-        hz[qz] = Pt[(c * 3 + 2) * NQP + q];
+        y1[qz] = Y[c * BA + qz * Q];
+        y2[qz] = Y[(3 + c) * BA + qz * Q];
       }
 #pragma unroll
       for (int k = 0; k < N1; ++k) {
-        T sx = 0, sy = 0, sz = 0;
+        T s = 0;
 #pragma unroll
         for (int qz = 0; qz < Q; ++qz) {
-          sx += t.N[qz][k] * hx[qz];
-          sy += t.N[qz][k] * hy[qz];
-          sz += t.D[qz][k] * hz[qz];
+          s += tb.N[qz][k] * y1[qz];
+          s += tb.D[qz][k] * y2[qz];
         }
-        const int z = b_at(c, k, ix[1], ix[2]);
-        if (act) {
-          Z[z] = sx;
-          Z[NB + z] = sy;
-          Z[2 * NB + z] = sz;
-        }
-      }
-    });
-    __syncwarp();
-    rows_of_lane<YR, CLAMP>(lane, [&](int row, bool act) {
-      int ix[3];
-      decode_row<LY::Y0, LY::Y1, LY::Y2, 3, N1, Q>(row, ix);
-      const int c = ix[0], k = ix[1], qx = ix[2];
-      T zx[Q], zy[Q], zz[Q];
-#pragma unroll
-      for (int qy = 0; qy < Q; ++qy) {
-        const int z = b_at(c, k, qy, qx);
-        zx[qy] = Z[z];
-        zy[qy] = Z[NB + z];
-        zz[qy] = Z[2 * NB + z];
-      }
-#pragma unroll
-      for (int j = 0; j < N1; ++j) {
-        T sx = 0, so = 0;
-#pragma unroll
-        for (int qy = 0; qy < Q; ++qy) {
-          sx += t.N[qy][j] * zx[qy];
-          so += t.D[qy][j] * zy[qy] + t.N[qy][j] * zz[qy];
-        }
-        const int y = a_at(c, k, j, qx);
-        if (act) {
-          Y[y] = sx;
-          Y[NA + y] = so;
-        }
-      }
-    });
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row0 = lane + 32 * r;
-      // lanes past the last row compute the last row (their out is unused)
-      if ((CLAMP && XR <= 32) || row0 < XR) {
-        int c, k, j;
-        x_row(row0 < XR ? row0 : XR - 1, c, k, j);
-        T yx[Q], yo[Q];
-#pragma unroll
-        for (int qx = 0; qx < Q; ++qx) {
-          yx[qx] = Y[a_at(c, k, j, qx)];
-          yo[qx] = Y[NA + a_at(c, k, j, qx)];
-        }
-#pragma unroll
-        for (int i = 0; i < N1; ++i) {
-          T s = 0;
-#pragma unroll
-          for (int qx = 0; qx < Q; ++qx) s += t.D[qx][i] * yx[qx] + t.N[qx][i] * yo[qx];
-          out[r][i] = s;
-        }
+        out[c][k] = s;
       }
     }
-    __syncwarp();
   }
 };
 
@@ -578,11 +500,16 @@ struct ScalarState {
   T det;
 };
 
+// upper triangle of a symmetric N x N matrix, row by row
+__host__ __device__ constexpr int tri_index(int N, int i, int j) {
+  return i <= j ? i * N - i * (i - 1) / 2 + (j - i) : j * N - j * (j - 1) / 2 + (i - j);
+}
+
 // Q(g) of do_operation_on_cell (mf_nh_operator.h:922-1499) for the point
-// whose record is rec[comp * NQ] (rec already offset by q; a pointer, or an
+// whose record is rec[comp * CS] (rec already offset to the point; a pointer, or an
 // accessor with operator[] such as the record pair of two cells); for the
 // variants that fold JxW into their coefficients Q(g) comes out times JxW.
-template <typename T, int VAR, int NQ, typename R>
+template <typename T, int VAR, int CS, typename R>
 __device__ __forceinline__ void physics(const T g[3][3], const R &rec, T mu, T lambda, T kappa,
                                         const ScalarState<T> &st, T Qm[3][3]) {
   constexpr int CV = variant_cvar(VAR);
@@ -594,13 +521,13 @@ __device__ __forceinline__ void physics(const T g[3][3], const R &rec, T mu, T l
     // g * (tau/J) + C : sym(g)     (mf_nh_operator.h:1425-1440)
     T Ts[6];
 #pragma unroll
-    for (int I = 0; I < 6; ++I) Ts[I] = rec[(CV + I) * NQ];
+    for (int I = 0; I < 6; ++I) Ts[I] = rec[(CV + I) * CS];
     T cs[6];
 #pragma unroll
     for (int I = 0; I < 6; ++I) {
       T a = 0;
 #pragma unroll
-      for (int J = 0; J < 6; ++J) a += rec[(CV + 6 + I * 6 + J) * NQ] * s[J];
+      for (int J = 0; J < 6; ++J) a += rec[(CV + 6 + tri_index(6, I, J)) * CS] * s[J];
       cs[I] = a;
     }
     const T T00 = Ts[0], T11 = Ts[1], T22 = Ts[2], T01 = Ts[3], T02 = Ts[4], T12 = Ts[5];
@@ -616,9 +543,9 @@ __device__ __forceinline__ void physics(const T g[3][3], const R &rec, T mu, T l
     Qm[1][2] += cs[5]; Qm[2][1] += cs[5];
   } else if (VAR == VAR_TENSOR2) {
     // c1 sym(g) + c2 tr(g) I + g * (tau/J)   (mf_nh_operator.h:1401-1424)
-    const T c1 = rec[CV * NQ], c2 = rec[(CV + 1) * NQ];
-    const T T00 = rec[(CV + 2) * NQ], T11 = rec[(CV + 3) * NQ], T22 = rec[(CV + 4) * NQ];
-    const T T01 = rec[(CV + 5) * NQ], T02 = rec[(CV + 6) * NQ], T12 = rec[(CV + 7) * NQ];
+    const T c1 = rec[CV * CS], c2 = rec[(CV + 1) * CS];
+    const T T00 = rec[(CV + 2) * CS], T11 = rec[(CV + 3) * CS], T22 = rec[(CV + 4) * CS];
+    const T T01 = rec[(CV + 5) * CS], T02 = rec[(CV + 6) * CS], T12 = rec[(CV + 7) * CS];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       Qm[i][0] = g[i][0] * T00 + g[i][1] * T01 + g[i][2] * T02;
@@ -642,13 +569,13 @@ __device__ __forceinline__ void physics(const T g[3][3], const R &rec, T mu, T l
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
-          for (int l = 0; l < 3; ++l) a += rec[(CV + ((i * 3 + j) * 3 + k) * 3 + l) * NQ] * g[k][l];
+          for (int l = 0; l < 3; ++l) a += rec[(CV + tri_index(9, i * 3 + j, k * 3 + l)) * CS] * g[k][l];
         Qm[i][j] = a;
       }
   } else if (VAR == VAR_SCALAR_REF) {
     // mf_nh_operator.h:1255-1400: g = Grad v; grad_x v = Grad v F^-1; the
     // scalar-variant physics; submitted as (jc + grad_x v tau) F^-T
-    const T c = rec[C_VAR * NQ];
+    const T c = rec[C_VAR * CS];
     T Fi[3][3];
     inv3(st.F, Fi);
     T gx[3][3];
@@ -681,7 +608,7 @@ __device__ __forceinline__ void physics(const T g[3][3], const R &rec, T mu, T l
       for (int j = 0; j < 3; ++j) Qm[i][j] = qd[i][0] * Fi[j][0] + qd[i][1] * Fi[j][1] + qd[i][2] * Fi[j][2];
   } else if (VAR == VAR_SCALAR_F1) {
     // mf_nh_operator.h:1182-1254: tau = mu b - c I, jc = 2c sym + 2 lambda tr I
-    const T c = rec[C_VAR * NQ];
+    const T c = rec[C_VAR * CS];
     T jc[6];
 #pragma unroll
     for (int I = 0; I < 6; ++I) jc[I] = T(2) * c * s[I] + (I < 3 ? T(2) * lambda * tr : T(0));
@@ -713,7 +640,7 @@ __device__ __forceinline__ void physics(const T g[3][3], const R &rec, T mu, T l
       for (int j = 0; j < 3; ++j) Qm[i][j] *= idet;
   } else {
     // formulation 0 (vol/iso split), mf_nh_operator.h:1001-1181
-    const T Jm13 = rec[C_VAR * NQ];
+    const T Jm13 = rec[C_VAR * CS];
     const T det_F = st.det;
     T bbar[3][3];
 #pragma unroll

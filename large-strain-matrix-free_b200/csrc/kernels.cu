@@ -86,16 +86,38 @@ __global__ void node_sum_kernel(T *dst, const T *__restrict__ buf, const int *__
 
 }  // namespace
 
-// Components per quadrature point of the cell record (the record's length
-// is rounded up to 16 bytes at its end, for the bulk-copy engine).
-int table_components(int caching, int formulation, lsmf_precision precision) {
-  (void)formulation;
-  (void)precision;
+int record_components(int caching) {
   if (caching == LSMF_CACHE_TENSOR4) return variant_ncomp(VAR_TENSOR4);
   if (caching == LSMF_CACHE_TENSOR2) return variant_ncomp(VAR_TENSOR2);
   if (caching == LSMF_CACHE_SCALAR_REFERENTIAL) return variant_ncomp(VAR_SCALAR_REF);
   if (caching == LSMF_CACHE_TENSOR4_NS) return variant_ncomp(VAR_TENSOR4_NS);
   return variant_ncomp(VAR_SCALAR_F1);
+}
+
+// metric 9 + tau/J 6 + the full 6x6 C; metric 9 + the full 9x9 dP/dF
+int table_components(int caching) {
+  if (caching == LSMF_CACHE_TENSOR4) return 9 + 6 + 36;
+  if (caching == LSMF_CACHE_TENSOR4_NS) return 9 + 81;
+  return record_components(caching);
+}
+
+int cells_per_batch(int p, lsmf_precision precision) {
+  const int halves = precision == LSMF_FP32 ? 2 : 1;
+  return 32 / ((p + 1) * (p + 1)) * halves;
+}
+
+size_t record_index(const lsmf_op *op, int cell, int comp, int q) {
+  auto at = [&](auto layout) -> size_t {
+    using RL = decltype(layout);
+    return RL::base(cell, op->batch_elems) + (size_t)comp * RL::CS + RL::q_off(q, op->slice_elems);
+  };
+  const bool f = op->precision == LSMF_FP32;
+  switch (op->L().p) {
+    case 1: return f ? at(RecLayout<1, 2, 2>{}) : at(RecLayout<1, 2, 1>{});
+    case 2: return f ? at(RecLayout<2, 3, 2>{}) : at(RecLayout<2, 3, 1>{});
+    case 3: return f ? at(RecLayout<3, 4, 2>{}) : at(RecLayout<3, 4, 1>{});
+    default: return f ? at(RecLayout<4, 5, 2>{}) : at(RecLayout<4, 5, 1>{});
+  }
 }
 
 lsmf_status launch_cache(lsmf_op *op) {
@@ -186,22 +208,17 @@ lsmf_status set_scatter_mode(lsmf_op *op, int mode) {
 }
 
 // Chunks of an operator's atomic-scatter cell loop: the option, or the
-// measured choice.  Swept on B200 over 1 / 2 / 4 / 6 / 8 chunks for every
-// variant and precision at 64^3 Q2 and for tensor4 at 32^3 / 40^3 Q2 and
-// 48^3 Q3 / Q4 (vmult time against one launch): from 131,072 cells 8 for
-// the referential variants (scalar_referential FP64 -7 %, tensor4_ns FP64 /
-// FP32 -4 / -6 %), 2 for tensor2 (-1 / -2 %), 4 for the others (tensor4
-// FP64 / FP32 -3.5 / -4 %, scalar -2 %); from 32,768 cells 2 (32^3 Q2
-// tensor4 FP64 / FP32 -4.5 / -10 %, 48^3 Q3 / Q4 under -1 %); fewer cells
-// run in one launch.
+// measured choice (vmult time on B200 against one launch, at 60^3 Q2, 96^3
+// Q1, 40^3 Q3 and 36^3 Q4): from 131,072 cells 8 for the referential variants
+// (scalar_referential -3 %, tensor4_ns -2 %), 4 for the others (tensor4
+// -0.5 %, scalar -2 %; degree 4 -2 to -4 %), from 32,768 cells 2; tensor2 and
+// fewer cells run in one launch (60^3 Q2 tensor2 229 us against 235 in 4).
 static int chunk_count(const lsmf_op *op) {
   if (op->chunks > 0) return op->chunks;
   const int n = op->L().n_cells;
-  if (n >= 131072) {
-    if (op->caching == LSMF_CACHE_TENSOR4_NS || op->caching == LSMF_CACHE_SCALAR_REFERENTIAL) return 8;
-    return op->caching == LSMF_CACHE_TENSOR2 ? 2 : 4;
-  }
-  return n >= 32768 ? 2 : 1;
+  if (op->caching == LSMF_CACHE_TENSOR2 || n < 32768) return 1;
+  if (n < 131072) return 2;
+  return op->caching == LSMF_CACHE_TENSOR4_NS || op->caching == LSMF_CACHE_SCALAR_REFERENTIAL ? 8 : 4;
 }
 
 // The operator's plan for k chunks (*out = nullptr where it does not apply:
@@ -225,7 +242,9 @@ static lsmf_status chunk_plan(const lsmf_op *op, int k, const ChunkPlan **out) {
     plan->cell0.resize(k + 1);
     plan->node0.resize(k + 1);
     std::vector<int> nmax(k);
-    for (int c = 0; c <= k; ++c) plan->cell0[c] = (int)((long long)L.n_cells * c / k);
+    // chunks start at whole batches of the cell records
+    const int B = cells_per_batch(L.p, op->precision);
+    for (int c = 0; c <= k; ++c) plan->cell0[c] = c == k ? L.n_cells : (int)((long long)L.n_cells * c / k) / B * B;
     for (int c = 0; c < k; ++c) {
       int lo = L.n_nodes, hi = -1;
       for (size_t i = (size_t)plan->cell0[c] * ncn; i < (size_t)plan->cell0[c + 1] * ncn; ++i) {

@@ -3,7 +3,7 @@
 //   cell_nodes  int32 [n_cells][(p+1)^3], node id | (constrained comps << 29)
 //   X           double [n_nodes][3] reference node coordinates
 //   vectors     Number [n_nodes][3] (dof = 3*node + comp)
-//   cache table Number [n_cells][n_comp][Q^3] (one contiguous record per cell)
+//   cache table Number, cell records interleaved by batches (RecLayout, cell_kernels.cuh)
 #pragma once
 #include <cuda_runtime.h>
 
@@ -212,23 +212,23 @@ struct lsmf_op {
   int level = 0;
   int caching = LSMF_CACHE_TENSOR4, formulation = 1;
   lsmf_precision precision = LSMF_FP64;
-  int ncomp = 0;                     // table components per qp
-  int rec_elems = 0;                 // values per cell record (ncomp * nq, plus per-cell values and padding)
+  int slice_elems = 0, batch_elems = 0;  // strides of the record table (RecLayout)
+  size_t table_bytes = 0;            // size of the tables as documented per caching (memory_consumption)
   bool ref_per_cell = false;         // scalar caching on affine cells: reference metric once per cell
   double nu = 0.3;
   std::vector<double> mu_host;
   lsmf::DevBuf<double> d_mu;         // per cell
-  lsmf::DevBuf<char> d_table;        // [cell][ncomp][nq] of Number
+  lsmf::DevBuf<char> d_table;        // cell records of Number (RecLayout)
   lsmf::DevBuf<char> d_diag, d_inv_diag;
   lsmf::DevBuf<int> d_flag;          // device error word
   const void *d_u = nullptr;         // borrowed displacement
   bool cached = false, have_diag = false;
-  int stages = -1;                   // bulk-copy (TMA) ring depth of the vmult kernel (0 = plain loads, -1 auto)
+  int stages = -1;                   // bulk-copy (TMA) ring depth of the vmult kernel: depth + 1 slices (0 = plain loads, -1 auto)
   bool basic = false;                // use the basic (smem-sweep) vmult kernel
   int max_warps = 0;                 // warps per block cap of the vmult kernel (<= 8, 0 auto)
   int wait_tries = -1;               // bulk-copy wait bound (try_wait calls; -1 = default 2^22)
   int prefetch = -1;                 // plain-load kernels: L1 prefetch of the record (0, 1 this cell, 2 next; -1 auto)
-  int pairs = -1;                    // FP32 vmult: two cells per warp in packed f32x2 arithmetic (0 off, 1 on, -1 auto)
+  int pairs = -1;                    // LSMF_OPT_CELL_PAIRS as set (no effect: FP32 always runs packed pairs)
   int device = 0;                    // CUDA device the operator's buffers live on
   int scatter = LSMF_SCATTER_ATOMIC; // cell-loop scatter: atomics, the 8 colour launches, or node sums
   lsmf::DevBuf<char> d_cellbuf;      // node-sum scatter: per-cell results [cell][local node][component]
@@ -258,5 +258,12 @@ lsmf_status set_scatter_mode(lsmf_op *op, int mode);
 // chunks the operator's next full vmult cell loop runs in (1: one launch)
 lsmf_status effective_chunks(const lsmf_op *op, int *k);
 lsmf_status upload_basis_tables(const Basis &b);
-int table_components(int caching, int formulation, lsmf_precision precision);
+// components of a point in the documented table and in the stored record
+// (tensor4 / tensor4_ns store the upper triangle of their symmetric matrices)
+int table_components(int caching);
+int record_components(int caching);
+// cells whose records are interleaved (RecLayout::B), and the index of value
+// (comp, point q) of a cell in the table
+int cells_per_batch(int p, lsmf_precision precision);
+size_t record_index(const lsmf_op *op, int cell, int comp, int q);
 }  // namespace lsmf

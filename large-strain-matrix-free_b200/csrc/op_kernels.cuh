@@ -3,7 +3,7 @@
 //   cache_kernel       NeoHookOperator::cache + Eulerian MatrixFree metric
 //   apply_kernel       NeoHookOperator::vmult_add cell loop, basic form with
 //                      the MFMask stage switches
-//   apply_fast_kernel  the production vmult cell loop
+//   apply_line_kernel  the production vmult cell loop
 //   diagonal_kernel    NeoHookOperator::compute_diagonal
 // Every cell loop runs either over all cells with atomic scatter, or over
 // one colour of the lattice (a list of cells no two of which share a node)
@@ -28,8 +28,8 @@ template <typename T>
 struct KArgs {
   const int *cell_nodes;
   int n_cells;
-  int ncomp;
-  int rec_elems;         // values per cell record
+  int slice_elems, batch_elems;  // record layout (RecLayout)
+  int ring;              // slices of the bulk-copy ring
   int ref_per_cell;      // scalar caching: reference inverse Jacobian once per cell
   T *table;              // cache records (written by cache, read by apply/diag)
   const T *src;
@@ -41,7 +41,7 @@ struct KArgs {
   int *flag;             // device error word
   unsigned mask;
   int wait_tries;        // try_wait calls before a bulk-copy wait gives up
-  int prefetch;          // plain loads: L1 prefetch of the record (0 off, 1 this cell, 2 the next cell)
+  int prefetch;          // plain loads: L1 prefetch of the records (0 off, 1 this unit, 2 the next unit)
   const int *cells;      // cell list of one colour (nullptr: all n_cells cells)
   int plain;             // scatter with plain adds (colour launches) instead of atomics
   T *cellbuf;            // node-sum scatter: per-cell results [cell][local node][component]
@@ -102,8 +102,7 @@ __device__ __forceinline__ void atomic_add(T *a, T v) { atomicAdd(a, v); }
 // ------------------------------------------------ bulk-copy (TMA) helpers
 // One-dimensional cp.async.bulk from this GPU's global memory into the
 // issuing CTA's own shared memory with mbarrier completion (no tensor map):
-// each cell record is one contiguous, 16-byte aligned block of
-// ncomp * Q^3 values.
+// the records of a warp's cells are one contiguous, 16-byte aligned block.
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -156,107 +155,154 @@ constexpr int FLAG_DETF = 1, FLAG_TIMEOUT = 2, FLAG_SMEM = 4;
 // internal stage bit: gather constrained entries instead of zeroing them
 constexpr unsigned MASK_INHOM = MASK_INHOM_BIT;
 
+// --------------------------------------------------- cells of a warp
+// The number type of a kernel, the scalar it is made of and how many cells a
+// lane carries: double and float one, f2 (packed FP32x2, pair.cuh) two.
+template <typename T>
+struct Num {
+  using S = T;
+  static constexpr int H = 1;
+};
+template <>
+struct Num<f2> {
+  using S = float;
+  static constexpr int H = 2;
+};
+// cells per lane group in the table of a scalar type: FP32 tables interleave
+// two cells, the halves of an f2
+template <typename S>
+__host__ __device__ constexpr int table_halves() { return sizeof(S) == 4 ? 2 : 1; }
+
+// List entries of a warp's unit of work w: entry i0 (and i0 + 1 of an f2
+// pair).  Contiguous loops follow the table: a double / f2 unit is one batch,
+// a float unit (diagonal) one half of a batch; lists are taken in order.
+// Entries past the end repeat the last one (pair) and are not stored.
+template <int P, int Q, typename T, bool LIST>
+struct UnitMap {
+  using S = typename Num<T>::S;
+  static constexpr int H = Num<T>::H, TH = table_halves<S>();
+  static constexpr int CPW = 32 / (Q * Q);
+  static constexpr bool HALF = !LIST && H == 1 && TH == 2;  // float over a paired table
+  static __host__ __device__ __forceinline__ int units(int n) {
+    return HALF ? 2 * ((n + 2 * CPW - 1) / (2 * CPW)) : (n + CPW * H - 1) / (CPW * H);
+  }
+  static __device__ __forceinline__ int entry(int w, int r) {
+    return HALF ? ((w >> 1) * CPW + r) * 2 + (w & 1) : (w * CPW + r) * H;
+  }
+};
+
 // ------------------------------------------------------------ cache kernel
+// NeoHookOperator::cache and the Eulerian metric: gathers X and u, evaluates
+// both gradients, and writes the cell records in FP64 arithmetic.  Lanes own
+// lines of cells (SFC), so every store of a component is one contiguous
+// access of the warp.  FP32 tables hold two cells per lane slot; their two
+// halves are worked on one after the other.
 template <int P, int Q, typename T, int VAR>
-__global__ void __launch_bounds__(256) cache_kernel(KArgs<T> a, Tab<P, Q> tab) {
-  using S = SF<P, Q, double>;
-  constexpr int NN = S::NN, NQ = S::NQ, QPL = S::QPL;
+__global__ void __launch_bounds__(128) cache_kernel(KArgs<T> a, TabT<P, Q, double> tabt, Tab<P, Q> tab) {
+  using S = SFC<P, Q, double>;
+  constexpr int N1 = P + 1, NN = S::NN, L = S::L, CPW = S::CPW, TH = table_halves<T>();
+  using RL = RecLayout<P, Q, TH>;
   const int WPB = blockDim.x >> 5;
   extern __shared__ __align__(16) unsigned char smem[];
-  double *sN = (double *)smem, *sD = sN + Q * (P + 1);
-  load_tables<P, Q, double>(tab, sN, sD);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double *slab = sD + Q * (P + 1) + warp * S::SZ;
-  double *V = slab, *A = slab + S::SZ1, *B = A + S::SZ2;
+  const int warp = threadIdx.x >> 5;
+  double *slab = (double *)smem + warp * S::SZ;
+  const LanePos<Q> lp;
   const int gw = blockIdx.x * WPB + warp, nw = gridDim.x * WPB;
+  const int n_units = TH * ((a.n_cells + RL::B - 1) / RL::B);
   int bad = 0;
-  for (int cell = gw; cell < a.n_cells; cell += nw) {
+  for (int w = gw; w < n_units; w += nw) {
+    const int e = ((w / TH) * CPW + lp.r) * TH + w % TH;
+    const bool valid = lp.act && e < a.n_cells;
+    const int cell = e < a.n_cells ? e : a.n_cells - 1;
     const int *cn = a.cell_nodes + (size_t)cell * NN;
-    double GX[QPL][3][3], GU[QPL][3][3];
-    gather<NN>(cn, a.X, false, V, lane);
-    S::eval(sN, sD, V, A, B, lane, GX);
-    gather<NN>(cn, a.u, false, V, lane);
-    S::eval(sN, sD, V, A, B, lane, GU);
+    double GX[Q][3][3], GU[Q][3][3], UV[Q][3];
+    {
+      double vx[3][N1], vu[3][N1];
+#pragma unroll
+      for (int k = 0; k < N1; ++k) {
+        const size_t d = 3 * (size_t)(__ldg(cn + k * L + lp.t) & NODE_MASK);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          vx[c][k] = __ldg(a.X + d + c);
+          vu[c][k] = (double)__ldg(a.u + d + c);
+        }
+      }
+      S::eval(tabt, vx, slab, lp, GX);
+      S::eval(tabt, vu, slab, lp, GU, VAR == VAR_SCALAR_REF ? UV : nullptr);
+    }
     const double mu = a.mu[cell];
     const double lambda = (2.0 * mu * a.nu) / (1.0 - 2.0 * a.nu);
-    T *rec = a.table + (size_t)cell * a.rec_elems;
-#pragma unroll
-    for (int l = 0; l < QPL; ++l) {
-      const int q = lane + 32 * l;
-      if (q >= NQ) continue;
-      const double w = tab.w[q % Q] * tab.w[(q / Q) % Q] * tab.w[q / (Q * Q)];
+    T *rec = a.table + RL::base(cell, a.batch_elems) + lp.t * RL::TS;
+    constexpr int CS = RL::CS;
+#pragma unroll(Q <= 3 ? Q : 1)
+    for (int s = 0; s < Q; ++s) {
+      const double w3 = tab.w[s] * tab.w[lp.b] * tab.w[lp.a];
       double Jr[3][3], Jc[3][3], Jri[3][3], Jci[3][3];
 #pragma unroll
       for (int d = 0; d < 3; ++d)
 #pragma unroll
-        for (int e = 0; e < 3; ++e) {
-          Jr[d][e] = GX[l][d][e];
-          Jc[d][e] = GX[l][d][e] + GU[l][d][e];
+        for (int e2 = 0; e2 < 3; ++e2) {
+          Jr[d][e2] = GX[s][d][e2];
+          Jc[d][e2] = GX[s][d][e2] + GU[s][d][e2];
         }
       inv3(Jr, Jri);
       const double dc = inv3(Jc, Jci);
-      T *r = rec + q;
+      T *r = rec + s * a.slice_elems;
+      auto put = [&](int comp, double x) {
+        if (valid) r[comp * CS] = T(x);
+      };
       // scalar_referential / tensor4_ns integrate in the reference frame
-      const double jxw = variant_referential(VAR) ? det3(Jr) * w : dc * w;
+      const double jxw = variant_referential(VAR) ? det3(Jr) * w3 : dc * w3;
 #pragma unroll
-      for (int i = 0; i < 9; ++i)
-        r[(C_JINV + i) * NQ] = T(variant_referential(VAR) ? Jri[i / 3][i % 3] : Jci[i / 3][i % 3]);
+      for (int i = 0; i < 9; ++i) put(C_JINV + i, variant_referential(VAR) ? Jri[i / 3][i % 3] : Jci[i / 3][i % 3]);
       // tensor4 / tensor2 / tensor4_ns store their coefficients times JxW
       constexpr int CV = variant_cvar(VAR);
       const double fw = variant_folds_jxw(VAR) ? jxw : 1.0;
-      if (!variant_folds_jxw(VAR)) r[C_JXW * NQ] = T(jxw);
+      if (!variant_folds_jxw(VAR)) put(C_JXW, jxw);
       // F = I + Grad u (reference configuration, mf_nh_operator.h:462-476)
       double F[3][3];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-          F[c][d] = GU[l][c][0] * Jri[0][d] + GU[l][c][1] * Jri[1][d] + GU[l][c][2] * Jri[2][d] + (c == d ? 1.0 : 0.0);
+          F[c][d] = GU[s][c][0] * Jri[0][d] + GU[s][c][1] * Jri[1][d] + GU[s][c][2] * Jri[2][d] + (c == d ? 1.0 : 0.0);
       const double det_F = det3(F);
       if (!(det_F > 0.0)) bad = 1;
       if (VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1) {
-        const double c = (VAR == VAR_SCALAR_F0) ? pow(det_F, -1.0 / 3.0) : mu - 2.0 * lambda * log(det_F);
-        r[C_VAR * NQ] = T(c);
+        put(C_VAR, (VAR == VAR_SCALAR_F0) ? pow(det_F, -1.0 / 3.0) : mu - 2.0 * lambda * log(det_F));
         if (a.ref_per_cell) {
           // affine cell: the reference metric of the first point stands for all
-          if (q == 0)
+          if (s == 0 && lp.t == 0 && valid) {
+            T *ref = a.table + RL::ref(cell, a.batch_elems, a.slice_elems);
 #pragma unroll
-            for (int i = 0; i < 9; ++i) rec[(C_VAR + 1) * NQ + i] = T(Jri[i / 3][i % 3]);
+            for (int i = 0; i < 9; ++i) ref[i * RL::RS] = T(Jri[i / 3][i % 3]);
+          }
         } else {
 #pragma unroll
-          for (int i = 0; i < 9; ++i) r[(C_VAR + 1 + i) * NQ] = T(Jri[i / 3][i % 3]);
+          for (int i = 0; i < 9; ++i) put(C_VAR + 1 + i, Jri[i / 3][i % 3]);
         }
         continue;
       }
       const double scalar = mu - 2.0 * lambda * log(det_F);
       if (VAR == VAR_SCALAR_REF) {
         // c and the displacement values at the point (phi_reference.begin_values())
-        r[C_VAR * NQ] = T(scalar);
-        const int qx = q % Q, qy = (q / Q) % Q, qz = q / (Q * Q);
+        put(C_VAR, scalar);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          double v = 0;
-          for (int kz = 0; kz <= P; ++kz)
-            for (int jy = 0; jy <= P; ++jy)
-              for (int ix = 0; ix <= P; ++ix)
-                v += sN[qx * (P + 1) + ix] * sN[qy * (P + 1) + jy] * sN[qz * (P + 1) + kz] *
-                     V[c * NN + (kz * (P + 1) + jy) * (P + 1) + ix];
-          r[(C_VAR + 1 + c) * NQ] = T(v);
-        }
+        for (int c = 0; c < 3; ++c) put(C_VAR + 1 + c, UV[s][c]);
         continue;
       }
       if (VAR == VAR_TENSOR4_NS) {
         // 2 lambda F^-T (x) F^-T + (mu - 2 lambda ln J) F^-T_il F^-1_jk + mu I_ik I_jl
         double Fi[3][3];
         inv3(F, Fi);
-        const double lnJ = log(det_F);
-        for (int i = 0; i < 3; ++i)
-          for (int j = 0; j < 3; ++j)
-            for (int k = 0; k < 3; ++k)
-              for (int l = 0; l < 3; ++l)
-                r[(CV + ((i * 3 + j) * 3 + k) * 3 + l) * NQ] =
-                    T(fw * (2.0 * lambda * Fi[j][i] * Fi[l][k] + (mu - 2.0 * lambda * lnJ) * Fi[l][i] * Fi[j][k] +
-                            (i == k && j == l ? mu : 0.0)));
+#pragma unroll
+        for (int m = 0; m < 9; ++m)
+#pragma unroll
+          for (int n = m; n < 9; ++n) {
+            const int i = m / 3, j = m % 3, k = n / 3, l = n % 3;
+            put(CV + tri_index(9, m, n), fw * (2.0 * lambda * Fi[j][i] * Fi[l][k] + scalar * Fi[l][i] * Fi[j][k] +
+                                               (i == k && j == l ? mu : 0.0)));
+          }
         continue;
       }
       const double idet = 1.0 / det_F;
@@ -268,23 +314,22 @@ __global__ void __launch_bounds__(256) cache_kernel(KArgs<T> a, Tab<P, Q> tab) {
         tau[I] = mu * b - (i == j ? scalar : 0.0);
       }
       if (VAR == VAR_TENSOR2) {
-        r[CV * NQ] = T(fw * scalar * 2.0 * idet);
-        r[(CV + 1) * NQ] = T(fw * 2.0 * lambda * idet);
+        put(CV, fw * scalar * 2.0 * idet);
+        put(CV + 1, fw * 2.0 * lambda * idet);
 #pragma unroll
-        for (int I = 0; I < 6; ++I) r[(CV + 2 + I) * NQ] = T(fw * tau[I] * idet);
+        for (int I = 0; I < 6; ++I) put(CV + 2 + I, fw * tau[I] * idet);
       } else {
 #pragma unroll
-        for (int I = 0; I < 6; ++I) r[(CV + I) * NQ] = T(fw * tau[I] * idet);
+        for (int I = 0; I < 6; ++I) put(CV + I, fw * tau[I] * idet);
         // C = (2c/J) S + (2 lambda/J) I (x) I  (mf_nh_operator.h:542-546)
         const double ca = scalar * 2.0 * idet, cb = lambda * 2.0 * idet;
 #pragma unroll
         for (int I = 0; I < 6; ++I)
 #pragma unroll
-          for (int J = 0; J < 6; ++J)
-            r[(CV + 6 + I * 6 + J) * NQ] = T(fw * ((I == J ? ca : 0.0) + (I < 3 && J < 3 ? cb : 0.0)));
+          for (int J = I; J < 6; ++J)
+            put(CV + 6 + tri_index(6, I, J), fw * ((I == J ? ca : 0.0) + (I < 3 && J < 3 ? cb : 0.0)));
       }
     }
-    __syncwarp();
   }
   if (bad) atomicOr(a.flag, 1);
 }
@@ -298,6 +343,8 @@ __global__ void __launch_bounds__(256) apply_kernel(KArgs<T> a, Tab<P, Q> tab) {
   constexpr int NN = S::NN, NQ = S::NQ, QPL = S::QPL;
   const int WPB = blockDim.x >> 5;
   constexpr bool SCALAR = (VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1);
+  using RL = RecLayout<P, Q, table_halves<T>()>;
+  constexpr int CS = RL::CS;
   extern __shared__ __align__(16) unsigned char smem[];
   T *sN = (T *)smem, *sD = sN + Q * (P + 1);
   load_tables<P, Q, T>(tab, sN, sD);
@@ -310,7 +357,8 @@ __global__ void __launch_bounds__(256) apply_kernel(KArgs<T> a, Tab<P, Q> tab) {
   for (int ic = gw; ic < a.n_cells; ic += nw) {
     const int cell = cell_of(a, ic);
     const int *cn = a.cell_nodes + (size_t)cell * NN;
-    const T *rec = a.table + (size_t)cell * a.rec_elems;
+    const T *rec = a.table + RL::base(cell, a.batch_elems);
+    const T *ref = a.table + RL::ref(cell, a.batch_elems, a.slice_elems);
     T G[QPL][3][3], GU[QPL][3][3];
     if (SCALAR) {
       if (rw) gather<NN>(cn, a.u, false, V, lane);   // read_dof_values_plain(u)
@@ -341,11 +389,11 @@ __global__ void __launch_bounds__(256) apply_kernel(KArgs<T> a, Tab<P, Q> tab) {
 #pragma unroll
         for (int e = 0; e < 3; ++e) H[l][c][e] = T(0);
       if (q >= NQ || !qd) continue;
-      const T *r = rec + q;
+      const T *r = rec + RL::q_off(q, a.slice_elems);
       T Ji[3][3];
 #pragma unroll
-      for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * NQ];
-      const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * NQ]);
+      for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * CS];
+      const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * CS]);
       T g[3][3];
 #pragma unroll
       for (int c = 0; c < 3; ++c)
@@ -356,7 +404,7 @@ __global__ void __launch_bounds__(256) apply_kernel(KArgs<T> a, Tab<P, Q> tab) {
         T Jr[3][3];
 #pragma unroll
         for (int i = 0; i < 9; ++i)
-          Jr[i / 3][i % 3] = a.ref_per_cell ? rec[(C_VAR + 1) * NQ + i] : r[(C_VAR + 1 + i) * NQ];
+          Jr[i / 3][i % 3] = a.ref_per_cell ? ref[i * RL::RS] : r[(C_VAR + 1 + i) * CS];
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -365,11 +413,16 @@ __global__ void __launch_bounds__(256) apply_kernel(KArgs<T> a, Tab<P, Q> tab) {
         st.det = det3(st.F);
       }
       if (VAR == VAR_SCALAR_REF) {
-        collocation_F<Q>(rec, q, tab.Dc, Ji, st.F);
+        T ux[3][Q];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+          for (int m = 0; m < Q; ++m) ux[c][m] = rec[m * a.slice_elems + (C_VAR + 1 + c) * CS + (q / Q) * RL::TS];
+        collocation_F<Q, CS, RL::TS>(ux, rec + (q % Q) * a.slice_elems, q % Q, (q / Q) % Q, q / (Q * Q), tab.Dc, Ji, st.F);
         st.det = det3(st.F);
       }
       T Qm[3][3];
-      physics<T, VAR, NQ>(g, r, mu, lambda, kappa, st, Qm);
+      physics<T, VAR, CS>(g, r, mu, lambda, kappa, st, Qm);
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -401,471 +454,329 @@ __global__ void __launch_bounds__(256) apply_kernel(KArgs<T> a, Tab<P, Q> tab) {
 }
 
 
-// --------------------------------------------- apply kernel, fast path
-// The production vmult cell loop.  One warp per cell; row-per-lane sum
-// factorisation (SFR) with the 1D matrices as constant operands; the
-// gather of the next cell (node ids, src, and u for the scalar variants) is
-// prefetched into registers while the current cell is computed; with
-// STAGES == 2 each warp streams its cell records through a two-stage
-// shared-memory ring filled by cp.async.bulk (evict-first in L2), with
-// STAGES == 0 the record is read with plain coalesced loads.  SC (scatter):
-// SC_ATOMIC loops over all cells and adds with atomics; SC_COLOUR over the
-// cell list of one lattice colour (a.cells, a.n_cells entries) with plain
-// adds; SC_CELLBUF over all cells, storing every cell's results to
+// ---------------------------------------- apply kernel, production path
+// The production vmult cell loop.  Q^2 lanes per cell, CPW cells per warp
+// (SFC), for f2 two cells per lane; the gather of the next unit (node ids,
+// src, and u for the scalar variants) is prefetched into registers while the
+// current one is computed; with RING each warp streams the record slices of
+// its units through a shared-memory ring of a.ring slices filled by
+// cp.async.bulk (evict-first in L2): a slice's place is refilled as soon as
+// the slice's points are done, so copies stay in flight through the whole
+// unit; without it the records are read with plain coalesced loads.
+// SC (scatter): SC_ATOMIC loops over all cells and adds with atomics;
+// SC_COLOUR over the cell list of one lattice colour (a.cells, a.n_cells
+// entries; no two of them share a node) with plain adds; SC_CELLBUF over all
+// cells, storing every cell's results to
 // a.cellbuf[cell][local node][component] (constrained rows as zero) for the
 // node sum that follows; SC_PEER as SC_ATOMIC, with the neighbour part's
 // nodes (PEER_BIT in the index map) gathered from a.psrc / a.pu and added to
 // a.pdst over peer memory: the partitioned vmult's ghost update and
 // compress(add) done by the cell loop itself.
+// Bound: HBM for the record-heavy variants (60^3 Q2 tensor4 FP64: 303 us for
+// 1.79 GB, 0.90 of the measured copy bandwidth; tensor4_ns 406 us, 0.99),
+// else shared-memory wavefronts and the latency of the sweeps (tensor2 229
+// us, 0.60).  One cell per warp with row-per-lane sweeps, 51 / 90 values per
+// point, took 397 / 654 / 274 us; 96^3 Q1 formulation 0 1167 -> 349 us, 36^3
+// Q4 tensor4 504 -> 376 us.
 constexpr int SC_ATOMIC = 0, SC_COLOUR = 1, SC_CELLBUF = 2, SC_PEER = 3;
-template <int P, int Q, typename T, int VAR, int STAGES, int SC>
-__global__ void __launch_bounds__(256) apply_fast_kernel(KArgs<T> a, TabT<P, Q, T> tab) {
+
+// per-warp shared memory: the ring's slices and barriers, the slab, and for
+// the scalar variants the displacement gradients of the unit's points
+// (kept there while the source's sweeps run: two gradient sets in registers
+// left 8 warps per SM and spilled from Q = 4 on)
+template <int P, int Q, typename T, bool SCALAR>
+__host__ __device__ __forceinline__ size_t line_warp_bytes(int ring, size_t slice_bytes) {
+  using S = SFC<P, Q, T>;
+  return (ring * slice_bytes + 16 * ((ring + 1) / 2) + (S::SZ + (SCALAR ? 9 * Q * S::LW : 0)) * sizeof(T) + 127) / 128 * 128;
+}
+
+// the cells' values as one number of the kernel's type
+template <typename T>
+__device__ __forceinline__ T join_of(const typename Num<T>::S *h, int stride) {
+  if constexpr (Num<T>::H == 2) return pack2(h[0], h[stride]);
+  else return h[0];
+}
+
+// Blocks of 128 threads the register allocation leaves room for: three (168
+// registers, 12 warps per SM) up to degree 2, where the working set fits
+// (60^3 Q2 FP64: tensor4 311 -> 303 us, scalar 367 -> 348, scalar_referential
+// 338 -> 329; 96^3 Q1 scalar 331 -> 315, formulation 0 387 -> 349; four
+// blocks, 128 registers, spill: tensor4 363), and for tensor2 at degree 3
+// (167 -> 161); two from there on (255 registers; 36^3 Q4 tensor4 376
+// against 438 us) and for the FP32 scalar_referential Q2 kernel (194 against
+// 210 us).
+template <int P, int VAR, bool FP32>
+constexpr int line_min_blocks() {
+  if (P == 2 && VAR == VAR_SCALAR_REF && FP32) return 2;
+  return P <= 2 || (P == 3 && VAR == VAR_TENSOR2) ? 3 : 2;
+}
+
+template <int P, int Q, typename T, int VAR, bool RING, int SC>
+__global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()) apply_line_kernel(KArgs<typename Num<T>::S> a, TabT<P, Q, T> tab) {
+  using E = typename Num<T>::S;
+  constexpr int H = Num<T>::H, TH = table_halves<E>();
   constexpr bool COL = SC == SC_COLOUR;
   constexpr bool SCALAR = (VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1);
-  // branch-free sweeps and point loop for the scalar variants (48^3 / 64^3
-  // Q2: scalar -7 % FP64 / -10 % FP32, scalar_referential -4 % / -17 %;
-  // tensor2 +4-6 % and tensor4 +1 %, so those keep the divergent form)
-  constexpr bool CLAMP = SCALAR || VAR == VAR_SCALAR_REF;
-  using S = SFR<P, Q, T, CLAMP>;
-  constexpr int N1 = P + 1, NN = S::NN, NQ = S::NQ, QPL = S::QPL, RPL = S::RPL, XR = S::XR;
-  // several points per lane (Q^3 > 32): the gradients stay in the slab's
-  // point block and each point is read, transformed and overwritten there
-  // in turn, instead of holding 2 x 9 x QPL values in registers (the FP64 Q4
-  // kernel otherwise runs out of registers); the scalar variants also need
-  // the displacement gradients and keep the register form
-  constexpr bool PT_SMEM = !SCALAR && QPL >= 2;
+  static_assert(H == TH, "one number holds the cells of a table entry");
+  static_assert(!(RING && COL), "the ring streams whole batches");
+  using S = SFC<P, Q, T>;
+  using UM = UnitMap<P, Q, T, COL>;
+  using RL = RecLayout<P, Q, TH>;
+  constexpr int N1 = P + 1, NN = S::NN, L = S::L, CPW = S::CPW, LW = S::LW;
+  // record access in numbers of T; the pairs of a cell list are put together
+  // from their two cells, in scalars
+  constexpr int U = COL ? TH : 1, TS = U, CS = LW * U, RS = CPW * U;
+  const int SS = a.slice_elems / (COL ? 1 : H);
   const int WPB = blockDim.x >> 5;
   extern __shared__ __align__(128) unsigned char smem[];
-  const int rec_elems = a.rec_elems;
-  const uint32_t rec_bytes = (uint32_t)(rec_elems * sizeof(T));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const size_t warp_bytes = ((STAGES * (size_t)rec_bytes + 8 * (STAGES > 0 ? STAGES : 1) + S::SZ * sizeof(T) + 127) / 128) * 128;
-  unsigned char *wbase = smem + warp * warp_bytes;
-  constexpr int NS = STAGES > 0 ? STAGES : 1;
-  T *stage[NS];
-#pragma unroll
-  for (int s = 0; s < NS; ++s) stage[s] = (T *)(wbase + s * rec_bytes);
-  uint64_t *bar = (uint64_t *)(wbase + STAGES * rec_bytes);
-  T *slab = (T *)(wbase + STAGES * rec_bytes + 8 * NS);
+  const LanePos<Q> lp;
+  const int D = RING ? a.ring : 0;
+  const uint32_t slice_bytes = (uint32_t)(a.slice_elems * sizeof(E));
+  unsigned char *wbase = smem + warp * line_warp_bytes<P, Q, T, SCALAR>(D, slice_bytes);
+  uint64_t *bar = (uint64_t *)(wbase + D * slice_bytes);
+  T *slab = (T *)(wbase + D * slice_bytes + 16 * ((D + 1) / 2));
+  T *park = slab + S::SZ + lp.ln;  // entry (s, c, e) at ((s * 3 + c) * 3 + e) * LW
   const int gw = blockIdx.x * WPB + warp, nw = gridDim.x * WPB;
+  const int n_units = UM::units(a.n_cells);
   // list entry -> cell
   auto cid = [&](int i) -> int { return COL ? __ldg(a.cells + i) : a.cell0 + i; };
+  // batch of a contiguous unit (a.cell0 is a multiple of the batch size)
+  auto batch_ptr = [&](int w) -> const E * { return a.table + (size_t)(a.cell0 / RL::B + w) * a.batch_elems; };
   uint64_t pol = 0;
-  if (STAGES > 0) {
+  auto copy_slice = [&](int w, int s, int place) {
+    mbar_expect_tx(&bar[place], slice_bytes);
+    bulk_g2s(wbase + place * slice_bytes, batch_ptr(w) + (size_t)s * a.slice_elems, slice_bytes, &bar[place], pol);
+  };
+  if (RING) {
     pol = evict_first_policy();
     if (lane == 0) {
-#pragma unroll
-      for (int s = 0; s < NS; ++s) mbar_init(&bar[s], 1);
+      for (int d = 0; d < D; ++d) mbar_init(&bar[d], 1);
       mbar_init_fence();
     }
     __syncwarp();
-    if (lane == 0) {
-#pragma unroll
-      for (int s = 0; s < NS; ++s) {
-        const int c = gw + s * nw;
-        if (c < a.n_cells) {
-          mbar_expect_tx(&bar[s], rec_bytes);
-          bulk_g2s(stage[s], a.table + (size_t)cid(c) * rec_elems, rec_bytes, &bar[s], pol);
-        }
-      }
-    }
+    if (lane == 0)
+      for (int d = 0; d < D; ++d)
+        if (gw + (d / Q) * nw < n_units) copy_slice(gw + (d / Q) * nw, d % Q, d);
   }
-  // gather registers of the x rows (c, k, j) owned by this lane
-  int pk[RPL][N1];
-  T pv[RPL][N1], pu[RPL][N1];
-  auto prefetch = [&](int c) {
-    const int *cn = a.cell_nodes + (size_t)cid(c) * NN;
+  int place = 0;        // ring place of the next slice, and the parity its
+  uint32_t parity = 0;  // copy completes
+  // cells of the lane: c[h]; ok[h]: stored by this lane
+  auto cells_of = [&](int w, int c[H], bool ok[H]) {
+    const int e0 = UM::entry(w, lp.r);
+    const int last = a.n_cells - 1;
+    const int f = e0 < a.n_cells ? e0 : last - last % H;
+    c[0] = cid(f);
+    ok[0] = lp.act && e0 < a.n_cells;
+    if (H == 2) {
+      c[H - 1] = f + 1 < a.n_cells ? cid(f + 1) : c[0];
+      ok[H - 1] = lp.act && e0 + 1 < a.n_cells;
+    }
+  };
+  // gather registers of the lane's z line of nodes, and the cells' mu
+  int pk[H][N1];
+  E pv[H][3][N1], pu[H][3][N1];
+  double pmu[H], cmu[H];
+  auto prefetch = [&](int w) {
+    int c[H];
+    bool ok[H];
+    cells_of(w, c, ok);
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      // (CLAMP) lanes past the last row load the last row again
-      if ((CLAMP && XR <= 32) || row < XR) {
-        int comp, xk, xj;
-        S::x_row(row < XR ? row : XR - 1, comp, xk, xj);
-        const int kj = xk * N1 + xj;
+    for (int h = 0; h < H; ++h) {
+      const int *cn = a.cell_nodes + (size_t)c[h] * NN + lp.t;
+      if (SCALAR || VAR == VAR_SCALAR_REF) pmu[h] = __ldg(a.mu + c[h]);
 #pragma unroll
-        for (int i = 0; i < N1; ++i) {
-          const int packed = __ldg(cn + kj * N1 + i);
-          pk[r][i] = packed;
-          if (SC == SC_PEER) {
-            const bool pe = packed & PEER_BIT;
-            const size_t dof = 3 * (size_t)(packed & PEER_NODE_MASK) + comp;
-            pv[r][i] = __ldg((pe ? a.psrc : a.src) + dof);
-            if (SCALAR) pu[r][i] = __ldg((pe ? a.pu : a.u) + dof);
-          } else {
-            const size_t dof = 3 * (size_t)(packed & NODE_MASK) + comp;
-            pv[r][i] = __ldg(a.src + dof);
-            if (SCALAR) pu[r][i] = __ldg(a.u + dof);
-          }
+      for (int k = 0; k < N1; ++k) pk[h][k] = __ldg(cn + k * L);
+#pragma unroll
+      for (int k = 0; k < N1; ++k) {
+        const int packed = pk[h][k];
+        const bool pe = SC == SC_PEER && (packed & PEER_BIT);
+        const size_t dof = 3 * (size_t)(packed & (SC == SC_PEER ? PEER_NODE_MASK : NODE_MASK));
+        const E *sv = (pe ? a.psrc : a.src) + dof, *su = (pe ? a.pu : a.u) + dof;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          pv[h][i][k] = __ldg(sv + i);
+          if (SCALAR) pu[h][i][k] = __ldg(su + i);
         }
       }
     }
   };
-  if (gw < a.n_cells) prefetch(gw);
-  int it = 0;
-  for (int cell = gw; cell < a.n_cells; cell += nw, ++it) {
-    const int s = it % NS;
-    const uint32_t parity = (it / NS) & 1;
-    int ck[RPL][N1];
-    T v[RPL][N1], vu[RPL][N1];
+  // the reference metric of a batch into L1, ahead of its use
+  auto prefetch_ref = [&](int w) {
+    if (SCALAR && !COL && a.ref_per_cell && lane * 128 < 9 * RL::B * (int)sizeof(E))
+      asm volatile("prefetch.global.L1 [%0];" ::"l"((const char *)(batch_ptr(w) + (size_t)Q * a.slice_elems) + lane * 128));
+  };
+  if (gw < n_units) {
+    prefetch(gw);
+    prefetch_ref(gw);
+  }
+  for (int w = gw; w < n_units; w += nw) {
+    int ck[H][N1];
+    T G[Q][3][3];
+    int c[H];
+    bool ok[H];
+    cells_of(w, c, ok);
+    // the cell's record at lane 0 of the cell, and its reference metric
+    auto rec_at = [&](size_t (*at)(int, int, int)) {
+      if constexpr (COL && H == 2)
+        return RecPair{a.table + at(c[0], a.batch_elems, a.slice_elems), a.table + at(c[H - 1], a.batch_elems, a.slice_elems)};
+      else return (const T *)(a.table + at(c[0], a.batch_elems, a.slice_elems));
+    };
+    const auto rec = rec_at([](int cell, int be, int) { return RL::base(cell, be); });
+    T ux[3][Q];  // scalar_referential: displacement along the x line
+    if (VAR == VAR_SCALAR_REF) {
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      int comp = 0, xk, xj;
-      // (CLAMP: the lanes past the last row carry a copy of it; the sweeps
-      // store nothing from them and the scatter skips them)
-      if ((CLAMP && XR <= 32) || row < XR) S::x_row(row < XR ? row : XR - 1, comp, xk, xj);
-      if (!(CLAMP && XR <= 32) && row >= XR) {
+      for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int i = 0; i < N1; ++i) { ck[r][i] = 0; v[r][i] = T(0); vu[r][i] = T(0); }
-        continue;
-      }
-#pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        ck[r][i] = pk[r][i];
-        // read_dof_values(src): constrained entries read as zero
-        v[r][i] = ((pk[r][i] >> (NODE_BITS + comp)) & 1) ? T(0) : pv[r][i];
-        if (SCALAR) vu[r][i] = pu[r][i];  // read_dof_values_plain(u)
-      }
+        for (int m = 0; m < Q; ++m) ux[i][m] = rec[m * SS + (C_VAR + 1 + i) * CS + lp.t * TS];
     }
-    if (cell + nw < a.n_cells) prefetch(cell + nw);
-    if (STAGES == 0 && a.prefetch) {
-      // one 128-byte line of the record per lane into L1, issued before the
-      // sweeps so that the point loop's loads find it there
-      const int pc = a.prefetch == 2 ? cell + nw : cell;
-      if (pc < a.n_cells) {
-        const char *base = (const char *)(a.table + (size_t)cid(pc) * rec_elems);
-        const int nbytes = rec_elems * (int)sizeof(T);
-        for (int off = lane * 128; off < nbytes; off += 32 * 128)
-          asm volatile("prefetch.global.L1 [%0];" ::"l"(base + off));
+    {
+      T v[3][N1], vu[3][N1];
+#pragma unroll
+      for (int k = 0; k < N1; ++k) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) ck[h][k] = pk[h][k];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          // read_dof_values(src): constrained entries read as zero
+          E x[H];
+#pragma unroll
+          for (int h = 0; h < H; ++h) x[h] = ((pk[h][k] >> (NODE_BITS + i)) & 1) ? E(0) : pv[h][i][k];
+          v[i][k] = join_of<T>(x, H - 1);
+          if (SCALAR) {  // read_dof_values_plain(u)
+#pragma unroll
+            for (int h = 0; h < H; ++h) x[h] = pu[h][i][k];
+            vu[i][k] = join_of<T>(x, H - 1);
+          }
+        }
       }
-    }
-    T G[QPL][3][3], GU[QPL][3][3];
-    if (SCALAR) S::eval(tab, vu, slab, lane, GU);
-    if (PT_SMEM) S::eval_pt(tab, v, slab, lane);
-    else S::eval(tab, v, slab, lane, G);
-    const T *rec;
-    if (STAGES > 0) {
-      if (!mbar_wait_bounded(&bar[s], parity, a.wait_tries)) {
-        if (lane == 0) atomicOr(a.flag, FLAG_TIMEOUT);
-        // every copy this warp issued is still owed to a stage of its
-        // shared memory: the one given up on (k = 0) and those of the next
-        // NS - 1 cells.  Let each land (long bound) before the block exits,
-        // so no copy writes shared memory that a later block owns.
-        for (int k = 0; k < NS; ++k)
-          if (cell + k * nw < a.n_cells) mbar_wait_bounded(&bar[(it + k) % NS], ((it + k) / NS) & 1);
-        return;
+#pragma unroll
+      for (int h = 0; h < H; ++h) cmu[h] = pmu[h];
+      if (w + nw < n_units) {
+        prefetch(w + nw);
+        prefetch_ref(w + nw);
       }
-      rec = stage[s];
-    } else {
-      rec = a.table + (size_t)cid(cell) * rec_elems;
-    }
-    T mu = 0, lambda = 0, kappa = 0;
-    if (SCALAR || VAR == VAR_SCALAR_REF) material<T>(a.mu[cid(cell)], a.nu, mu, lambda, kappa);
-    T H[QPL][3][3];
-#pragma unroll(PT_SMEM ? 1 : QPL)
-    for (int l = 0; l < QPL; ++l) {
-      // (CLAMP: the lanes past the last point repeat it; their H is never
-      // stored)
-      const int q = (CLAMP && NQ <= 32) ? (lane < NQ ? lane : NQ - 1) : lane + 32 * l;
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) H[l][c][e] = T(0);
-      if (!(CLAMP && NQ <= 32) && q >= NQ) continue;
-      const T *r = rec + q;
-      T Ji[3][3];
-#pragma unroll
-      for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * NQ];
-      const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * NQ]);
-      T Gq[3][3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) Gq[c][e] = PT_SMEM ? slab[(c * 3 + e) * S::NQP + q] : G[l][c][e];
-      T g[3][3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) g[c][d] = Gq[c][0] * Ji[0][d] + Gq[c][1] * Ji[1][d] + Gq[c][2] * Ji[2][d];
-      ScalarState<T> st;
+      if (!RING && !COL && a.prefetch) {
+        // one 128-byte line of the records per lane into L1, issued before
+        // the sweeps so that the point loop's loads find it there
+        const int pw = a.prefetch == 2 ? w + nw : w;
+        if (pw < n_units) {
+          const char *base = (const char *)batch_ptr(pw);
+          for (int off = lane * 128; off < Q * (int)slice_bytes; off += 32 * 128)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(base + off));
+        }
+      }
       if (SCALAR) {
-        T Jr[3][3];
+        S::eval(tab, vu, slab, lp, G);
 #pragma unroll
-        for (int i = 0; i < 9; ++i)
-          Jr[i / 3][i % 3] = a.ref_per_cell ? rec[(C_VAR + 1) * NQ + i] : r[(C_VAR + 1 + i) * NQ];
+        for (int s = 0; s < Q; ++s)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            st.F[c][d] = GU[l][c][0] * Jr[0][d] + GU[l][c][1] * Jr[1][d] + GU[l][c][2] * Jr[2][d] + (c == d ? T(1) : T(0));
-        st.det = det3(st.F);
+          for (int i = 0; i < 9; ++i) park[(s * 9 + i) * LW] = G[s][i / 3][i % 3];
       }
-      if (VAR == VAR_SCALAR_REF) {
-        collocation_F<Q>(rec, q, tab.Dc, Ji, st.F);
-        st.det = det3(st.F);
-      }
-      T Qm[3][3];
-      physics<T, VAR, NQ>(g, r, mu, lambda, kappa, st, Qm);
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-          const T h0 = Qm[c][0] * Ji[e][0] + Qm[c][1] * Ji[e][1] + Qm[c][2] * Ji[e][2];
-          const T h = variant_folds_jxw(VAR) ? h0 : T(h0 * jxw);
-          // each lane overwrites only its own points
-          if (PT_SMEM) slab[(c * 3 + e) * S::NQP + q] = h;
-          else H[l][c][e] = h;
-        }
+      S::eval(tab, v, slab, lp, G);
     }
-    if (STAGES > 0) {
-      __syncwarp();  // every lane is done reading stage[s]
-      if (lane == 0) {
-        const int next = cell + NS * nw;
-        if (next < a.n_cells) {
-          fence_proxy_async_smem();
-          mbar_expect_tx(&bar[s], rec_bytes);
-          bulk_g2s(stage[s], a.table + (size_t)cid(next) * rec_elems, rec_bytes, &bar[s], pol);
-        }
-      }
-    }
-    T out[RPL][N1];
-    if (PT_SMEM) S::integrate_pt(tab, slab, lane, out);
-    else S::integrate(tab, H, slab, lane, out);
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      if (row < XR) {
-        int comp, xk, xj;
-        S::x_row(row, comp, xk, xj);
-#pragma unroll
-        for (int i = 0; i < N1; ++i) {
-          // distribute_local_to_global: constrained rows skipped
-          const bool con = (ck[r][i] >> (NODE_BITS + comp)) & 1;
-          if (SC == SC_CELLBUF) {
-            a.cellbuf[((size_t)cell * NN + (xk * N1 + xj) * N1 + i) * 3 + comp] = con ? T(0) : out[r][i];
-          } else if (SC == SC_PEER) {
-            if (!con) {
-              const int k = ck[r][i];
-              atomic_add(((k & PEER_BIT) ? a.pdst : a.dst) + 3 * (size_t)(k & PEER_NODE_MASK) + comp, out[r][i]);
-            }
-          } else if (!con) {
-            T *d = a.dst + 3 * (size_t)(ck[r][i] & NODE_MASK) + comp;
-            if (COL) *d += out[r][i];
-            else atomic_add(d, out[r][i]);
-          }
-        }
-      }
-    }
-  }
-}
-
-// ------------------------------------------------ FP32 cell-pair kernel
-// The plain-load cell loop of apply_fast_kernel for FP32 operators with two
-// cells per warp: list entries 2i and 2i + 1 go through the sweeps and the
-// point physics together as the two halves of packed f32x2 registers
-// (pair.cuh), so one issued arithmetic or shared-memory instruction serves
-// both cells.  Gathers, record loads and the scatter stay per cell.  With an
-// odd count the last pair repeats its first cell and scatters it once.
-// per-warp shared memory of the pair kernel (8 bytes, then the slab of the
-// 8-byte-entry sweep layout), used by the kernel and by its launcher
-template <int P, int Q>
-__host__ __device__ constexpr size_t pair_warp_bytes() {
-  return ((8 + SFR<P, Q, f2>::SZ * sizeof(f2) + 127) / 128) * 128;
-}
-
-template <int P, int Q, int VAR, int SC>
-__global__ void __launch_bounds__(256) apply_pair_kernel(KArgs<float> a, TabT<P, Q, f2> tab) {
-  using T = f2;
-  constexpr bool COL = SC == SC_COLOUR;
-  constexpr bool SCALAR = (VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1);
-  constexpr bool CLAMP = SCALAR || VAR == VAR_SCALAR_REF;
-  using S = SFR<P, Q, T, CLAMP>;
-  constexpr int N1 = P + 1, NN = S::NN, NQ = S::NQ, QPL = S::QPL, RPL = S::RPL, XR = S::XR;
-  constexpr bool PT_SMEM = !SCALAR && QPL >= 2;
-  const int WPB = blockDim.x >> 5;
-  extern __shared__ __align__(128) unsigned char smem[];
-  const int rec_elems = a.rec_elems;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr size_t warp_bytes = pair_warp_bytes<P, Q>();
-  {
-    // the launch must provide every warp's slab; otherwise do nothing
-    unsigned dyn;
-    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-    if ((size_t)WPB * warp_bytes > dyn) {
-      if (threadIdx.x == 0) atomicOr(a.flag, FLAG_SMEM);
-      return;
-    }
-  }
-  T *slab = (T *)(smem + warp * warp_bytes + 8);
-  const int gw = blockIdx.x * WPB + warp, nw = gridDim.x * WPB;
-  const int n_pairs = (a.n_cells + 1) >> 1;
-  auto cid = [&](int i) -> int { return COL ? __ldg(a.cells + i) : a.cell0 + i; };
-  // gather registers of the x rows (c, k, j) owned by this lane, both cells
-  int pk0[RPL][N1], pk1[RPL][N1];
-  float pv0[RPL][N1], pv1[RPL][N1], pu0[RPL][N1], pu1[RPL][N1];
-  auto prefetch = [&](int pi) {
-    const int e0 = 2 * pi, e1 = (2 * pi + 1 < a.n_cells) ? 2 * pi + 1 : 2 * pi;
-    const int *cn0 = a.cell_nodes + (size_t)cid(e0) * NN, *cn1 = a.cell_nodes + (size_t)cid(e1) * NN;
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      if ((CLAMP && XR <= 32) || row < XR) {
-        int comp, xk, xj;
-        S::x_row(row < XR ? row : XR - 1, comp, xk, xj);
-        const int kj = xk * N1 + xj;
-#pragma unroll
-        for (int i = 0; i < N1; ++i) {
-          const int k0 = __ldg(cn0 + kj * N1 + i), k1 = __ldg(cn1 + kj * N1 + i);
-          pk0[r][i] = k0;
-          pk1[r][i] = k1;
-          const size_t d0 = 3 * (size_t)(k0 & NODE_MASK) + comp, d1 = 3 * (size_t)(k1 & NODE_MASK) + comp;
-          pv0[r][i] = __ldg(a.src + d0);
-          pv1[r][i] = __ldg(a.src + d1);
-          if (SCALAR) {
-            pu0[r][i] = __ldg(a.u + d0);
-            pu1[r][i] = __ldg(a.u + d1);
-          }
-        }
-      }
-    }
-  };
-  if (gw < n_pairs) prefetch(gw);
-  for (int pi = gw; pi < n_pairs; pi += nw) {
-    const int e0 = 2 * pi;
-    const bool two = 2 * pi + 1 < a.n_cells;
-    const int e1 = two ? e0 + 1 : e0;
-    const int c0 = cid(e0), c1 = cid(e1);
-    int ck0[RPL][N1], ck1[RPL][N1];
-    T v[RPL][N1], vu[RPL][N1];
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      int comp = 0, xk, xj;
-      if ((CLAMP && XR <= 32) || row < XR) S::x_row(row < XR ? row : XR - 1, comp, xk, xj);
-      if (!(CLAMP && XR <= 32) && row >= XR) {
-#pragma unroll
-        for (int i = 0; i < N1; ++i) { ck0[r][i] = 0; ck1[r][i] = 0; v[r][i] = T(0); vu[r][i] = T(0); }
-        continue;
-      }
-#pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        ck0[r][i] = pk0[r][i];
-        ck1[r][i] = pk1[r][i];
-        // read_dof_values(src): constrained entries read as zero
-        v[r][i] = pack2(((pk0[r][i] >> (NODE_BITS + comp)) & 1) ? 0.f : pv0[r][i],
-                        ((pk1[r][i] >> (NODE_BITS + comp)) & 1) ? 0.f : pv1[r][i]);
-        if (SCALAR) vu[r][i] = pack2(pu0[r][i], pu1[r][i]);
-      }
-    }
-    if (pi + nw < n_pairs) prefetch(pi + nw);
-    if (a.prefetch) {
-      // both records into L1 before the sweeps
-      const char *b0 = (const char *)(a.table + (size_t)c0 * rec_elems);
-      const char *b1 = (const char *)(a.table + (size_t)c1 * rec_elems);
-      const int nbytes = rec_elems * (int)sizeof(float);
-      for (int off = lane * 128; off < nbytes; off += 32 * 128) {
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(b0 + off));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(b1 + off));
-      }
-    }
-    T G[QPL][3][3], GU[QPL][3][3];
-    if (SCALAR) S::eval(tab, vu, slab, lane, GU);
-    if (PT_SMEM) S::eval_pt(tab, v, slab, lane);
-    else S::eval(tab, v, slab, lane, G);
-    const RecPair rec{a.table + (size_t)c0 * rec_elems, a.table + (size_t)c1 * rec_elems};
     T mu = 0, lambda = 0, kappa = 0;
     if (SCALAR || VAR == VAR_SCALAR_REF) {
-      float m0, l0, k0, m1, l1, k1;
-      material<float>(a.mu[c0], a.nu, m0, l0, k0);
-      material<float>(a.mu[c1], a.nu, m1, l1, k1);
-      mu = pack2(m0, m1);
-      lambda = pack2(l0, l1);
-      kappa = pack2(k0, k1);
+      E m[3][H];
+#pragma unroll
+      for (int h = 0; h < H; ++h) material<E>(cmu[h], a.nu, m[0][h], m[1][h], m[2][h]);
+      mu = join_of<T>(m[0], H - 1);
+      lambda = join_of<T>(m[1], H - 1);
+      kappa = join_of<T>(m[2], H - 1);
     }
-    T H[QPL][3][3];
-#pragma unroll(PT_SMEM ? 1 : QPL)
-    for (int l = 0; l < QPL; ++l) {
-      const int q = (CLAMP && NQ <= 32) ? (lane < NQ ? lane : NQ - 1) : lane + 32 * l;
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) H[l][c][e] = T(0);
-      if (!(CLAMP && NQ <= 32) && q >= NQ) continue;
-      const RecPair r = rec + q;
+    const auto ref = rec_at([](int cell, int be, int se) { return RL::ref(cell, be, se); });
+    // one point: G[s] becomes H[s]; slice: the record at the point's slice
+    // and lane 0 of the cell
+    auto point = [&](int s, auto slice) {
+      const auto r = slice + lp.t * TS;
       T Ji[3][3];
 #pragma unroll
-      for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * NQ];
-      const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * NQ]);
-      T Gq[3][3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) Gq[c][e] = PT_SMEM ? slab[(c * 3 + e) * S::NQP + q] : G[l][c][e];
+      for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * CS];
+      const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * CS]);
       T g[3][3];
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
+      for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) g[c][d] = Gq[c][0] * Ji[0][d] + Gq[c][1] * Ji[1][d] + Gq[c][2] * Ji[2][d];
+        for (int d = 0; d < 3; ++d) g[i][d] = G[s][i][0] * Ji[0][d] + G[s][i][1] * Ji[1][d] + G[s][i][2] * Ji[2][d];
       ScalarState<T> st;
       if (SCALAR) {
         T Jr[3][3];
 #pragma unroll
-        for (int i = 0; i < 9; ++i)
-          Jr[i / 3][i % 3] = a.ref_per_cell ? rec[(C_VAR + 1) * NQ + i] : r[(C_VAR + 1 + i) * NQ];
+        for (int i = 0; i < 9; ++i) Jr[i / 3][i % 3] = a.ref_per_cell ? T(ref[i * RS]) : T(r[(C_VAR + 1 + i) * CS]);
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+        for (int i = 0; i < 3; ++i) {
+          const T u0 = park[(s * 9 + 3 * i) * LW], u1 = park[(s * 9 + 3 * i + 1) * LW], u2 = park[(s * 9 + 3 * i + 2) * LW];
 #pragma unroll
           for (int d = 0; d < 3; ++d)
-            st.F[c][d] = GU[l][c][0] * Jr[0][d] + GU[l][c][1] * Jr[1][d] + GU[l][c][2] * Jr[2][d] + (c == d ? T(1) : T(0));
+            st.F[i][d] = u0 * Jr[0][d] + u1 * Jr[1][d] + u2 * Jr[2][d] + (i == d ? T(1) : T(0));
+        }
         st.det = det3(st.F);
       }
       if (VAR == VAR_SCALAR_REF) {
-        collocation_F<Q>(rec, q, tab.Dc, Ji, st.F);
+        collocation_F<Q, CS, TS>(ux, slice, s, lp.b, lp.a, tab.Dc, Ji, st.F);
         st.det = det3(st.F);
       }
       T Qm[3][3];
-      physics<T, VAR, NQ>(g, r, mu, lambda, kappa, st, Qm);
+      physics<T, VAR, CS>(g, r, mu, lambda, kappa, st, Qm);
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
+      for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int e = 0; e < 3; ++e) {
-          const T h0 = Qm[c][0] * Ji[e][0] + Qm[c][1] * Ji[e][1] + Qm[c][2] * Ji[e][2];
-          const T h = variant_folds_jxw(VAR) ? h0 : T(h0 * jxw);
-          if (PT_SMEM) slab[(c * 3 + e) * S::NQP + q] = h;
-          else H[l][c][e] = h;
+          const T h0 = Qm[i][0] * Ji[e][0] + Qm[i][1] * Ji[e][1] + Qm[i][2] * Ji[e][2];
+          G[s][i][e] = variant_folds_jxw(VAR) ? h0 : T(h0 * jxw);
         }
+    };
+#pragma unroll
+    for (int s = 0; s < Q; ++s) {
+      if constexpr (RING) {
+        if (!mbar_wait_bounded(&bar[place], parity, a.wait_tries)) {
+          if (lane == 0) atomicOr(a.flag, FLAG_TIMEOUT);
+          // every copy this warp issued is still owed to a place of its
+          // shared memory: the one given up on (k = 0) and those of the next
+          // D - 1 slices.  Let each land (long bound) before the block
+          // exits, so no copy writes shared memory that a later block owns.
+          for (int k = 0; k < D; ++k) {
+            if (w + ((s + k) / Q) * nw < n_units) mbar_wait_bounded(&bar[place], parity);
+            if (++place == D) { place = 0; parity ^= 1; }
+          }
+          return;
+        }
+        point(s, (const T *)(wbase + place * slice_bytes) + lp.r * L);
+        __syncwarp();  // every lane is done reading the slice
+        const int wn = w + ((s + D) / Q) * nw;
+        if (lane == 0 && wn < n_units) {
+          fence_proxy_async_smem();
+          copy_slice(wn, (s + D) % Q, place);
+        }
+        if (++place == D) { place = 0; parity ^= 1; }
+      } else {
+        point(s, rec + s * SS);
+      }
     }
-    T out[RPL][N1];
-    if (PT_SMEM) S::integrate_pt(tab, slab, lane, out);
-    else S::integrate(tab, H, slab, lane, out);
+    T out[3][N1];
+    S::integrate(tab, G, slab, lp, out);
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      if (row < XR) {
-        int comp, xk, xj;
-        S::x_row(row, comp, xk, xj);
+    for (int h = 0; h < H; ++h) {
+      if (!ok[h]) continue;
 #pragma unroll
-        for (int i = 0; i < N1; ++i) {
-          float o0, o1;
-          unpack2(out[r][i], o0, o1);
+      for (int k = 0; k < N1; ++k) {
+        const int packed = ck[h][k];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          E o;
+          if constexpr (H == 2) o = h ? hi2(out[i][k]) : lo2(out[i][k]);
+          else o = out[i][k];
           // distribute_local_to_global: constrained rows skipped
-          const bool con0 = (ck0[r][i] >> (NODE_BITS + comp)) & 1, con1 = (ck1[r][i] >> (NODE_BITS + comp)) & 1;
+          const bool con = (packed >> (NODE_BITS + i)) & 1;
           if (SC == SC_CELLBUF) {
-            const int local = (xk * N1 + xj) * N1 + i;
-            a.cellbuf[((size_t)e0 * NN + local) * 3 + comp] = con0 ? 0.f : o0;
-            if (two) a.cellbuf[((size_t)e1 * NN + local) * 3 + comp] = con1 ? 0.f : o1;
-          } else {
-            if (!con0) {
-              float *d = a.dst + 3 * (size_t)(ck0[r][i] & NODE_MASK) + comp;
-              if (COL) *d += o0;
-              else atomicAdd(d, o0);
-            }
-            if (two && !con1) {
-              float *d = a.dst + 3 * (size_t)(ck1[r][i] & NODE_MASK) + comp;
-              if (COL) *d += o1;
-              else atomicAdd(d, o1);
-            }
+            a.cellbuf[((size_t)c[h] * NN + k * L + lp.t) * 3 + i] = con ? E(0) : o;
+          } else if (SC == SC_PEER) {
+            if (!con)
+              atomic_add(((packed & PEER_BIT) ? a.pdst : a.dst) + 3 * (size_t)(packed & PEER_NODE_MASK) + i, o);
+          } else if (!con) {
+            E *d = a.dst + 3 * (size_t)(packed & NODE_MASK) + i;
+            if (COL) *d += o;
+            else atomic_add(d, o);
           }
         }
       }
@@ -874,111 +785,259 @@ __global__ void __launch_bounds__(256) apply_pair_kernel(KArgs<float> a, TabT<P,
 }
 
 // --------------------------------------------------------- diagonal kernel
-// diag(a,c) = sum_q JxW n^T B_c n with n = grad_x N_a and
-// B_c[d][l] = Q(e_c (x) e_l)[c][d]: identical to applying the cell operator
+// diag(a, c) = sum_q JxW n^T D_c n with n = grad_x N_a and
+// D_c[d][l] = Q(e_c (x) e_l)[c][d]: identical to applying the cell operator
 // to unit vectors (mf_nh_operator.h:881-899) and keeping the diagonal entry.
+// Pulled back, M_c = J^-1 D_c J^-T JxW is a symmetric 3x3 matrix per point
+// and n^T D_c n = sum_ef M_c[e][f] d_e N_a d_f N_a, whose factors are
+// products of the 1D tables N N, N D and D D: six fields per component go
+// through the three transposed sweeps, in place of a sum over all points
+// for every node.
+template <int P, int Q, typename T>
+struct TabSq {
+  T NN[Q][P + 1], ND[Q][P + 1], DD[Q][P + 1];
+};
+
+// D_c (symmetric) for row c of the tangent at a point; for the variants that
+// fold JxW into their coefficients it comes out times JxW.  order of the six
+// entries: 00, 11, 22, 01, 02, 12
+template <typename T, int VAR, int CS, typename R>
+__device__ __forceinline__ void diag_block(int c, const R &rec, T mu, T lambda, T kappa, const ScalarState<T> &st, T D[6]) {
+  constexpr int CV = variant_cvar(VAR);
+  if (VAR == VAR_TENSOR4_NS) {
+#pragma unroll
+    for (int I = 0; I < 6; ++I) D[I] = rec[(CV + tri_index(9, c * 3 + sym_i(I), c * 3 + sym_j(I))) * CS];
+    return;
+  }
+  if (VAR == VAR_TENSOR4 || VAR == VAR_TENSOR2) {
+    T c1 = 0, c2 = 0;
+    if (VAR == VAR_TENSOR2) {
+      c1 = rec[CV * CS];
+      c2 = rec[(CV + 1) * CS];
+    }
+#pragma unroll
+    for (int I = 0; I < 6; ++I) {
+      const int d = sym_i(I), l = sym_j(I);
+      T x = rec[(CV + (VAR == VAR_TENSOR2 ? 2 : 0) + I) * CS];
+      if (VAR == VAR_TENSOR2) {
+        x += c1 * (T(0.5) * T((d == l) + (d == c && l == c))) + (d == c && l == c ? c2 : T(0));
+      } else {
+        // entry (c, d), (c, l) of the 6x6 matrix acting on sym(e_c (x) e_l)
+        const int Id = c == d ? c : (c + d) + 2, Il = c == l ? c : (c + l) + 2;  // (0,1) 3, (0,2) 4, (1,2) 5
+        x += rec[(CV + 6 + tri_index(6, Id, Il)) * CS] * (c == l ? T(1) : T(0.5));
+      }
+      D[I] = x;
+    }
+    return;
+  }
+  T b[6];
+#pragma unroll
+  for (int I = 0; I < 6; ++I) {
+    const int i = sym_i(I), j = sym_j(I);
+    b[I] = st.F[i][0] * st.F[j][0] + st.F[i][1] * st.F[j][1] + st.F[i][2] * st.F[j][2];
+  }
+  const T x0 = rec[C_VAR * CS];
+  if (VAR == VAR_SCALAR_F0) {
+    // formulation 0 (mf_nh_operator.h:1001-1181), x0 = J^(-1/3)
+    const T det = st.det, idet = T(1) / det;
+    const T dPsi = (kappa / T(2)) * (det - idet), d2Psi = (kappa / T(2)) * (T(1) + idet * idet);
+#pragma unroll
+    for (int I = 0; I < 6; ++I) b[I] = b[I] * x0 * x0 * mu;  // tau_bar
+    const T trb = b[0] + b[1] + b[2], trd = trb * T(1.0 / 3.0), two3 = T(2.0 / 3.0);
+#pragma unroll
+    for (int I = 0; I < 6; ++I) {
+      const int d = sym_i(I), l = sym_j(I);
+      auto iso = [&](int i, int j) -> T { return b[i == j ? i : i + j + 2] - (i == j ? trd : T(0)); };
+      T v = (two3 * trb - T(2) * dPsi * det) * (T(0.5) * T((d == l) + (d == c && l == c)));
+      if (d == c && l == c) v += det * (dPsi + det * d2Psi) - (two3 * trb) * T(1.0 / 3.0);
+      if (l == c) v -= two3 * iso(c, d);
+      if (d == c) v -= two3 * iso(c, l);
+      v += b[I] + (d == l ? dPsi * det - trd : T(0));
+      D[I] = v * idet;
+    }
+    return;
+  }
+  // formulation 1: W = c (I + e_c e_c^T) + 2 lambda e_c e_c^T + tau, over J
+  // in the Eulerian frame
+  const T f = VAR == VAR_SCALAR_F1 ? T(T(1) / st.det) : T(1);
+#pragma unroll
+  for (int I = 0; I < 6; ++I) {
+    const int d = sym_i(I), l = sym_j(I);
+    T v = mu * b[I];  // tau = mu b - x0 I cancels the x0 I of the first term
+    if (d == c && l == c) v += x0 + T(2) * lambda;
+    D[I] = v * f;
+  }
+}
+
 template <int P, int Q, typename T, int VAR>
-__global__ void __launch_bounds__(128) diagonal_kernel(KArgs<T> a, Tab<P, Q> tab) {
-  using S = SF<P, Q, T>;
-  constexpr int N1 = P + 1, NN = S::NN, NQ = S::NQ, QPL = S::QPL;
-  const int WPB = blockDim.x >> 5;
+__global__ void __launch_bounds__(128) diagonal_kernel(KArgs<T> a, TabT<P, Q, T> tab, TabSq<P, Q, T> sq) {
+  using S = SFC<P, Q, T>;
+  constexpr int TH = table_halves<T>();
+  using RL = RecLayout<P, Q, TH>;
+  constexpr int N1 = P + 1, NN = S::NN, L = S::L, CPW = S::CPW, CS = RL::CS;
+  constexpr int RA = S::RA, RB = S::RB, BA = S::BA, BB = S::BB;
   constexpr bool SCALAR = (VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1);
-  constexpr int SZD = S::SZ + 36 * NQ;
   extern __shared__ __align__(16) unsigned char smem[];
-  T *sN = (T *)smem, *sD = sN + Q * N1;
-  load_tables<P, Q, T>(tab, sN, sD);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  T *slab = sD + Q * N1 + warp * SZD;
-  T *V = slab, *A = slab + S::SZ1, *B = A + S::SZ2;
-  T *Bq = slab + S::SZ;  // [q][27] then [q][9] inverse Jacobian
-  T *Jq = Bq + 27 * NQ;
+  const int WPB = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  T *slab = (T *)smem + warp * S::SZ;
+  const LanePos<Q> lp;
   const int gw = blockIdx.x * WPB + warp, nw = gridDim.x * WPB;
-  for (int ic = gw; ic < a.n_cells; ic += nw) {
-    const int cell = cell_of(a, ic);
-    const int *cn = a.cell_nodes + (size_t)cell * NN;
-    const T *rec = a.table + (size_t)cell * a.rec_elems;
-    T GU[QPL][3][3];
+  const bool list = a.cells != nullptr;
+  const int n_units = list ? UnitMap<P, Q, T, true>::units(a.n_cells) : UnitMap<P, Q, T, false>::units(a.n_cells);
+  for (int w = gw; w < n_units; w += nw) {
+    const int e = list ? UnitMap<P, Q, T, true>::entry(w, lp.r) : UnitMap<P, Q, T, false>::entry(w, lp.r);
+    const bool valid = lp.act && e < a.n_cells;
+    const int cell = cell_of(a, e < a.n_cells ? e : a.n_cells - 1);
+    const int *cn = a.cell_nodes + (size_t)cell * NN + lp.t;
+    const T *cr = a.table + RL::base(cell, a.batch_elems), *ref = a.table + RL::ref(cell, a.batch_elems, a.slice_elems);
+    int ck[N1];
+#pragma unroll
+    for (int k = 0; k < N1; ++k) ck[k] = __ldg(cn + k * L);
+    T GU[Q][3][3];
     if (SCALAR) {
-      gather<NN>(cn, a.u, false, V, lane);
-      S::eval(sN, sD, V, A, B, lane, GU);
+      T vu[3][N1];
+#pragma unroll
+      for (int k = 0; k < N1; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) vu[i][k] = __ldg(a.u + 3 * (size_t)(ck[k] & NODE_MASK) + i);
+      S::eval(tab, vu, slab, lp, GU);
     }
     T mu = 0, lambda = 0, kappa = 0;
     if (SCALAR || VAR == VAR_SCALAR_REF) material<T>(a.mu[cell], a.nu, mu, lambda, kappa);
+    T out[3][N1];
 #pragma unroll
-    for (int l = 0; l < QPL; ++l) {
-      const int q = lane + 32 * l;
-      if (q >= NQ) continue;
-      const T *r = rec + q;
-      const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * NQ]);
-      T Ji[3][3];
+    for (int c = 0; c < 3; ++c) {
+      T M[Q][6];
 #pragma unroll
-      for (int i = 0; i < 9; ++i) {
-        Jq[q * 9 + i] = r[(C_JINV + i) * NQ];
-        Ji[i / 3][i % 3] = r[(C_JINV + i) * NQ];
-      }
-      ScalarState<T> st;
-      if (SCALAR) {
-        T Jr[3][3];
+      for (int s = 0; s < Q; ++s) {
+        const T *r = cr + s * a.slice_elems + lp.t * RL::TS;
+        T Ji[3][3];
 #pragma unroll
-        for (int i = 0; i < 9; ++i)
-          Jr[i / 3][i % 3] = a.ref_per_cell ? rec[(C_VAR + 1) * NQ + i] : r[(C_VAR + 1 + i) * NQ];
+        for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * CS];
+        const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * CS]);
+        ScalarState<T> st;
+        if (SCALAR) {
+          T Jr[3][3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            st.F[c][d] = GU[l][c][0] * Jr[0][d] + GU[l][c][1] * Jr[1][d] + GU[l][c][2] * Jr[2][d] + (c == d ? T(1) : T(0));
-        st.det = det3(st.F);
-      }
-      if (VAR == VAR_SCALAR_REF) {
-        collocation_F<Q>(rec, q, tab.Dc, Ji, st.F);
-        st.det = det3(st.F);
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int ll = 0; ll < 3; ++ll) {
-          T g[3][3];
+          for (int i = 0; i < 9; ++i) Jr[i / 3][i % 3] = a.ref_per_cell ? ref[i * RL::RS] : r[(C_VAR + 1 + i) * CS];
 #pragma unroll
           for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int j = 0; j < 3; ++j) g[i][j] = (i == c && j == ll) ? T(1) : T(0);
-          T Qm[3][3];
-          physics<T, VAR, NQ>(g, r, mu, lambda, kappa, st, Qm);
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            Bq[q * 27 + (c * 3 + d) * 3 + ll] = variant_folds_jxw(VAR) ? Qm[c][d] : T(Qm[c][d] * jxw);
+            for (int d = 0; d < 3; ++d)
+              st.F[i][d] = GU[s][i][0] * Jr[0][d] + GU[s][i][1] * Jr[1][d] + GU[s][i][2] * Jr[2][d] + (i == d ? T(1) : T(0));
+          st.det = det3(st.F);
         }
-    }
-    __syncwarp();
-    for (int an = lane; an < NN; an += 32) {
-      const int ix = an % N1, iy = (an / N1) % N1, iz = an / (N1 * N1);
-      T o[3] = {T(0), T(0), T(0)};
-      for (int q = 0; q < NQ; ++q) {
-        const int qx = q % Q, qy = (q / Q) % Q, qz = q / (Q * Q);
-        const T nx = sN[qx * N1 + ix], ny = sN[qy * N1 + iy], nz = sN[qz * N1 + iz];
-        const T gx = sD[qx * N1 + ix] * ny * nz, gy = nx * sD[qy * N1 + iy] * nz, gz = nx * ny * sD[qz * N1 + iz];
-        const T *J = Jq + q * 9;
-        T n[3];
+        if (VAR == VAR_SCALAR_REF) {
+          T ux[3][Q];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) n[d] = gx * J[d] + gy * J[3 + d] + gz * J[6 + d];
-        const T *Bc = Bq + q * 27;
+          for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          T s = 0;
+            for (int m = 0; m < Q; ++m) ux[i][m] = cr[m * a.slice_elems + (C_VAR + 1 + i) * CS + lp.t * RL::TS];
+          collocation_F<Q, CS, RL::TS>(ux, cr + s * a.slice_elems, s, lp.b, lp.a, tab.Dc, Ji, st.F);
+          st.det = det3(st.F);
+        }
+        T D[6];
+        diag_block<T, VAR, CS>(c, r, mu, lambda, kappa, st, D);
+        if (VAR == VAR_SCALAR_REF) {
+          // the block is W in the spatial frame: pull back with J^-1 F^-1
+          T Fi[3][3], K[3][3];
+          inv3(st.F, Fi);
 #pragma unroll
-          for (int d = 0; d < 3; ++d)
-            s += n[d] * (Bc[(c * 3 + d) * 3 + 0] * n[0] + Bc[(c * 3 + d) * 3 + 1] * n[1] + Bc[(c * 3 + d) * 3 + 2] * n[2]);
-          o[c] += s;
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) K[i][d] = Ji[i][0] * Fi[0][d] + Ji[i][1] * Fi[1][d] + Ji[i][2] * Fi[2][d];
+#pragma unroll
+          for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = K[i / 3][i % 3];
+        }
+        const T Df[3][3] = {{D[0], D[3], D[4]}, {D[3], D[1], D[5]}, {D[4], D[5], D[2]}};
+        T DJ[3][3];  // D J^-T
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+          for (int f = 0; f < 3; ++f) DJ[d][f] = Df[d][0] * Ji[f][0] + Df[d][1] * Ji[f][1] + Df[d][2] * Ji[f][2];
+#pragma unroll
+        for (int I = 0; I < 6; ++I) {
+          const int i = sym_i(I), f = sym_j(I);
+          const T m = (Ji[i][0] * DJ[0][f] + Ji[i][1] * DJ[1][f] + Ji[i][2] * DJ[2][f]) * (I < 3 ? T(1) : T(2));
+          M[s][I] = variant_folds_jxw(VAR) ? m : T(m * jxw);
         }
       }
-      const int packed = __ldg(cn + an);
-      const int node = packed & NODE_MASK, cm = packed >> NODE_BITS;
-      T *d = a.dst + 3 * (size_t)node;
-      if (!(cm & 1)) scatter_add(d, o[0], a.plain);
-      if (!(cm & 2)) scatter_add(d + 1, o[1], a.plain);
-      if (!(cm & 4)) scatter_add(d + 2, o[2], a.plain);
+      // x: fields xx, yy, zz, xy, xz, yz in lanes (qz, qy)
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < N1; ++i) {
+        T f[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
+#pragma unroll
+        for (int s = 0; s < Q; ++s) {
+          f[0] += sq.DD[s][i] * M[s][0];
+          f[1] += sq.NN[s][i] * M[s][1];
+          f[2] += sq.NN[s][i] * M[s][2];
+          f[3] += sq.ND[s][i] * M[s][3];
+          f[4] += sq.ND[s][i] * M[s][4];
+          f[5] += sq.NN[s][i] * M[s][5];
+        }
+#pragma unroll
+        for (int I = 0; I < 6; ++I) slab[I * BB + i * RB + lp.ln] = f[I];
+      }
+      __syncwarp();
+      // y, lanes (qz, i): the fields that take N N, N D and D D along z
+      T o[3][N1];
+      {
+        const T *Z = slab + lp.r * L + lp.a * Q + lp.b * RB;
+        T z[6][Q];
+#pragma unroll
+        for (int I = 0; I < 6; ++I)
+#pragma unroll
+          for (int qy = 0; qy < Q; ++qy) z[I][qy] = Z[I * BB + qy];
+#pragma unroll
+        for (int j = 0; j < N1; ++j) {
+          T s0 = 0, s1 = 0, s2 = 0;
+#pragma unroll
+          for (int qy = 0; qy < Q; ++qy) {
+            s0 += sq.NN[qy][j] * z[0][qy];
+            s0 += sq.DD[qy][j] * z[1][qy];
+            s0 += sq.ND[qy][j] * z[3][qy];
+            s1 += sq.NN[qy][j] * z[4][qy];
+            s1 += sq.ND[qy][j] * z[5][qy];
+            s2 += sq.NN[qy][j] * z[2][qy];
+          }
+          o[0][j] = s0;
+          o[1][j] = s1;
+          o[2][j] = s2;
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < N1; ++j)
+#pragma unroll
+        for (int m = 0; m < 3; ++m) slab[m * BA + j * RA + lp.ln] = o[m][j];
+      __syncwarp();
+      // z, lanes (j, i)
+      const T *Y = slab + lp.r * L + lp.b + lp.a * RA;
+      T y[3][Q];
+#pragma unroll
+      for (int m = 0; m < 3; ++m)
+#pragma unroll
+        for (int qz = 0; qz < Q; ++qz) y[m][qz] = Y[m * BA + qz * Q];
+#pragma unroll
+      for (int k = 0; k < N1; ++k) {
+        T s = 0;
+#pragma unroll
+        for (int qz = 0; qz < Q; ++qz) {
+          s += sq.NN[qz][k] * y[0][qz];
+          s += sq.ND[qz][k] * y[1][qz];
+          s += sq.DD[qz][k] * y[2][qz];
+        }
+        out[c][k] = s;
+      }
     }
-    __syncwarp();
+    if (valid) {
+#pragma unroll
+      for (int k = 0; k < N1; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+          if (!((ck[k] >> (NODE_BITS + i)) & 1)) scatter_add(a.dst + 3 * (size_t)(ck[k] & NODE_MASK) + i, out[i][k], a.plain);
+    }
   }
 }
 
@@ -1058,8 +1117,9 @@ KArgs<T> make_args(const lsmf_op *op) {
   KArgs<T> a;
   a.cell_nodes = L.d_cell_nodes.ptr;
   a.n_cells = L.n_cells;
-  a.ncomp = op->ncomp;
-  a.rec_elems = op->rec_elems;
+  a.slice_elems = op->slice_elems;
+  a.batch_elems = op->batch_elems;
+  a.ring = 0;
   a.ref_per_cell = op->ref_per_cell ? 1 : 0;
   a.table = (T *)op->d_table.ptr;
   a.src = nullptr;
@@ -1106,15 +1166,48 @@ template <int P, int Q, typename T, int VAR>
 lsmf_status run_cache(lsmf_op *op) {
   auto a = make_args<T>(op);
   const Tab<P, Q> tab = make_tab<P, Q>(op->mesh->basis);
-  using S = SF<P, Q, double>;
-  const int w = warps_for(sizeof(double) * S::SZ, 8);
-  const size_t smem = sizeof(double) * (S::TAB + w * S::SZ);
+  const TabT<P, Q, double> tabt = make_tabt<P, Q, double>(op->mesh->basis);
+  using S = SFC<P, Q, double>;
+  const int w = 4;
+  const size_t smem = sizeof(double) * w * S::SZ;
   auto k = cache_kernel<P, Q, T, VAR>;
   LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int g = grid_for(k, 32 * w, smem, (a.n_cells + w - 1) / w);
-  k<<<g, 32 * w, smem, op->stream>>>(a, tab);
+  const int units = (a.n_cells + S::CPW - 1) / S::CPW;
+  const int g = grid_for(k, 32 * w, smem, (units + w - 1) / w);
+  k<<<g, 32 * w, smem, op->stream>>>(a, tabt, tab);
   LSMF_CUDA(cudaGetLastError());
   return LSMF_OK;
+}
+
+// launch the production cell loop
+template <int P, int Q, typename T, int VAR>
+lsmf_status launch_line(const lsmf_op *op, KArgs<typename Num<T>::S> a, bool peer, int ring, int max_warps,
+                        cudaStream_t stream) {
+  using E = typename Num<T>::S;
+  const TabT<P, Q, T> tab = make_tabt<P, Q, T>(op->mesh->basis);
+  const bool col = a.cells != nullptr, cellbuf = a.cellbuf != nullptr;
+  if (col) ring = 0;
+  const size_t slice_bytes = a.slice_elems * sizeof(E);
+  auto wbytes = [&](int d) { return line_warp_bytes<P, Q, T, VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1>(d, slice_bytes); };
+  // a smaller ring when it would leave fewer than 4 warps per SM
+  while (ring > 0 && warps_for_budget(wbytes(ring), 8, 220 * 1024) < 4) --ring;
+  a.ring = ring;
+  // at most 4 warps per block (the kernel's launch bound is 128 threads);
+  // smaller blocks let several blocks share an SM
+  const int w = warps_for_budget(wbytes(ring), max_warps < 4 ? max_warps : 4, 220 * 1024);
+  const size_t smem = w * wbytes(ring);
+  const int units = col ? UnitMap<P, Q, T, true>::units(a.n_cells) : UnitMap<P, Q, T, false>::units(a.n_cells);
+  auto go = [&](auto k) -> lsmf_status {
+    LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int g = grid_for(k, 32 * w, smem, (units + w - 1) / w);
+    k<<<g, 32 * w, smem, stream>>>(a, tab);
+    return LSMF_OK;
+  };
+  if (col) return go(apply_line_kernel<P, Q, T, VAR, false, SC_COLOUR>);
+  if (cellbuf) return ring ? go(apply_line_kernel<P, Q, T, VAR, true, SC_CELLBUF>) : go(apply_line_kernel<P, Q, T, VAR, false, SC_CELLBUF>);
+  if constexpr (sizeof(E) == 8)
+    if (peer) return ring ? go(apply_line_kernel<P, Q, T, VAR, true, SC_PEER>) : go(apply_line_kernel<P, Q, T, VAR, false, SC_PEER>);
+  return ring ? go(apply_line_kernel<P, Q, T, VAR, true, SC_ATOMIC>) : go(apply_line_kernel<P, Q, T, VAR, false, SC_ATOMIC>);
 }
 
 template <int P, int Q, typename T, int VAR>
@@ -1126,138 +1219,56 @@ lsmf_status run_apply(const lsmf_op *op, T *dst, const T *src, unsigned mask, Ce
   a.mask = mask;
   set_range(a, range);
   if (a.n_cells == 0) return LSMF_OK;
-  // L1 prefetch of each cell's record before its sweeps (plain-load
-  // kernels): measured on B200 at 64^3 Q2 and 48^3 Q4 it shortens every
-  // plain-load kernel (Q4 tensor4 FP64 1.37 -> 1.19 ms, Q2 tensor2 FP32
-  // -6 %) except the FP64 scalar variant (+1 %), which keeps it off
-  if (op->prefetch < 0) a.prefetch = ((VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1) && sizeof(T) == 8) ? 0 : 1;
-  const Tab<P, Q> tab = make_tab<P, Q>(op->mesh->basis);
-  using S = SF<P, Q, T>;
-  const int w = warps_for(sizeof(T) * S::SZ, 8);
-  const size_t smem = sizeof(T) * (S::TAB + w * S::SZ);
   const bool full = (mask & (LSMF_MASK_RW | LSMF_MASK_SF | LSMF_MASK_QD)) ==
                         (LSMF_MASK_RW | LSMF_MASK_SF | LSMF_MASK_QD) &&
                     !(mask & MASK_INHOM);
-  using SR = SFR<P, Q, T>;
-  const size_t rec_bytes = (size_t)op->rec_elems * sizeof(T);
-  const TabT<P, Q, T> tabt = make_tabt<P, Q, T>(op->mesh->basis);
-  auto wbytes = [&](int st) { return ((st * rec_bytes + 8 * (st > 0 ? st : 1) + SR::SZ * sizeof(T) + 127) / 128) * 128; };
-  // defaults measured on B200 (ring depth x record prefetch x warps per
-  // block swept for Q2 / Q3 / Q4 at 64^3 / 48^3 / 48^3 cells): at Q1 / Q2
-  // the variants that stream a large record per point (tensor4, tensor4_ns)
-  // and scalar_referential (whose collocation gradient reads the record out
-  // of order) want the one-stage bulk-copy ring while a record fits in
-  // 24 KB; from Q3 on, plain loads with the L1 record prefetch are faster
-  // (Q3 FP32 tensor4 0.409 -> 0.337 ms, tensor4_ns 0.661 -> 0.449 ms,
-  // scalar_referential FP32 -6 % / FP64 -15 %), as they are for the larger
-  // records (Q3 FP64 tensor4, Q4) and for tensor2 and scalar (latency / FP64
-  // bound)
-  const bool ring_variant = VAR == VAR_TENSOR4 || VAR == VAR_TENSOR4_NS || VAR == VAR_SCALAR_REF;
-  int stages = op->stages >= 0 ? op->stages : ((ring_variant && P <= 2 && rec_bytes <= 24 * 1024) ? 1 : 0);
-  // a level small enough that every warp gets at most one cell (a coarse
-  // multigrid level) gains nothing from the ring, which can only prefetch
-  // a warp's next cell: plain loads (15^3-cell FP64 coarse Chebyshev solve
-  // 10.9 -> 9.9 ms per V-cycle, FP32 unchanged)
-  if (op->stages < 0 && a.n_cells <= 32 * num_sms()) stages = 0;
-  // warps per block, swept 2 / 4 / 8 for every variant and precision at
-  // 64^3 Q2: 8 for the FP64 tensor2 and scalar kernels (scalar 0.478 ->
-  // 0.466 ms, formulation 0 0.497 -> 0.482 ms), 2 for FP64
-  // scalar_referential (0.467 -> 0.452 ms), 4 otherwise (the others within
-  // 1 % of each other)
-  constexpr bool fp64 = sizeof(T) == 8;
-  const int max_warps =
-      op->max_warps > 0 ? op->max_warps
-      : (fp64 && (VAR == VAR_TENSOR2 || VAR == VAR_SCALAR_F1 || VAR == VAR_SCALAR_F0)) ? 8
-      : (fp64 && VAR == VAR_SCALAR_REF) ? 2
-                                        : 4;
-  if (rec_bytes % 16 != 0) stages = 0;
-  // fewer stages when the ring would leave fewer than 4 warps per block
-  while (stages > 0 && warps_for_budget(wbytes(stages), 8, 220 * 1024) < 4) --stages;
-  const bool col = a.cells != nullptr;
-  const bool cellbuf = a.cellbuf != nullptr;
+  const bool col = a.cells != nullptr, cellbuf = a.cellbuf != nullptr, peer = range.peer_nodes != nullptr;
   if (cellbuf && !(full && !op->basic)) {
     set_error("the node-sum scatter serves the full vmult cell loop only");
     return LSMF_ERR_INVALID_ARG;
   }
-  const bool peer = range.peer_nodes != nullptr;
   if (peer && (!full || op->basic || col || cellbuf || sizeof(T) != 8)) {
     set_error("the fused interface exchange serves the full FP64 vmult cell loop with atomic scatter only");
     return LSMF_ERR_INVALID_ARG;
   }
-  // the colour, cell-buffer and peer launches are built with at most one stage
-  if ((col || cellbuf || peer) && stages > 1) stages = 1;
-  if constexpr (std::is_same<T, float>::value) {
-    // automatic choice, measured on B200 (FP32 vmult at 96^3 Q1, 64^3 Q2,
-    // 48^3 Q3 / Q4 and the 15^3 -> 30^3 / 60^3 Q2 V-cycles), pairs where
-    // they were faster: Q1 tensor2 (-2 %) and scalar (-8 %); Q2 tensor2
-    // (-9 %, V-cycle -5 %), scalar (-8 %, V-cycle -7 %) and
-    // scalar_referential (-11 %); Q4 scalar_referential (-10 %).  Every Q3
-    // variant (+5-13 %), the record-heavy tensor4 (Q2 +27 %) and tensor4_ns
-    // (+8 %), whose loops are bound by load latency and lose half their warps
-    // to the pair kernel's registers, and formulation 0 (+12 %, 159
-    // registers) stay one cell per warp.
-    constexpr bool pair_variant = (P == 1 && (VAR == VAR_TENSOR2 || VAR == VAR_SCALAR_F1)) ||
-                                  (P == 2 && (VAR == VAR_TENSOR2 || VAR == VAR_SCALAR_F1 || VAR == VAR_SCALAR_REF)) ||
-                                  (P == 4 && VAR == VAR_SCALAR_REF);
-    if (full && !op->basic && (op->pairs > 0 || (op->pairs < 0 && pair_variant))) {
-      // FP32 cell pairs (plain loads; the ring is not used)
-      const size_t wb = pair_warp_bytes<P, Q>();
-      const int w = warps_for_budget(wb, max_warps < 8 ? max_warps : 8, 220 * 1024);
-      const size_t smem_p = w * wb;
-      const TabT<P, Q, f2> tabp = make_tabt<P, Q, f2>(op->mesh->basis);
-      const int n_pairs = (a.n_cells + 1) / 2;
-      auto go = [&](auto k) -> lsmf_status {
-        LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p));
-        const int g = grid_for(k, 32 * w, smem_p, (n_pairs + w - 1) / w);
-        k<<<g, 32 * w, smem_p, stream>>>(a, tabp);
-        return LSMF_OK;
-      };
-      if (col) return go(apply_pair_kernel<P, Q, VAR, SC_COLOUR>);
-      if (cellbuf) return go(apply_pair_kernel<P, Q, VAR, SC_CELLBUF>);
-      return go(apply_pair_kernel<P, Q, VAR, SC_ATOMIC>);
-    }
-  }
   if (full && !op->basic) {
-    // at most 8 warps per block (the kernel's launch bound is 256 threads);
-    // smaller blocks let several blocks share an SM
-    const int w = warps_for_budget(wbytes(stages), max_warps < 8 ? max_warps : 8, 220 * 1024);
-    const size_t smem_t = w * wbytes(stages);
-    lsmf_status st = LSMF_OK;
+    if (a.cell0 % RecLayout<P, Q, table_halves<T>()>::B != 0) {
+      set_error("a chunk of the cell loop must start at a whole batch of cells");
+      return LSMF_ERR_INVALID_ARG;
+    }
+    // plain loads: L1 prefetch of the unit's records before its sweeps
+    if (op->prefetch < 0) a.prefetch = 1;
+    // Defaults measured on B200 over ring depth x warps per block x chunks at
+    // 96^3 Q1, 60^3 Q2, 40^3 Q3 and 36^3 Q4, FP64 and FP32: a ring of two
+    // slices almost everywhere (60^3 Q2 tensor4 FP64 303 us against 314 with
+    // plain loads and 370 with three slices, which cost resident warps);
+    // three slices for the small records of degree 4 (tensor2 308 against 318
+    // us); plain loads for the scalar variants from degree 2 on (60^3 Q2 348
+    // against 355 us: 11 values per point, and their parked gradients already
+    // fill the shared memory).  2 warps per block; 1 for tensor4_ns up to
+    // degree 2 (406 against 415 us) and 4 at degree 4 (tensor4 376 against
+    // 381 us with 1).
+    constexpr bool scalar = VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1;
+    constexpr int ring_auto = scalar && P >= 2 ? 0 : P == 4 && (VAR == VAR_TENSOR2 || VAR == VAR_SCALAR_REF) ? 3 : 2;
+    constexpr int warps_auto = P == 4 ? 4 : VAR == VAR_TENSOR4_NS && P <= 2 ? 1 : 2;
+    const int ring = op->stages >= 0 ? (op->stages ? op->stages + 1 : 0) : ring_auto;
+    const int max_warps = op->max_warps > 0 ? op->max_warps : warps_auto;
+    // FP32: two cells per lane, in packed registers
+    using N = typename std::conditional<sizeof(T) == 8, double, f2>::type;
+    LSMF_TRY((launch_line<P, Q, N, VAR>(op, a, peer, ring, max_warps, stream)));
+  } else {
+    const Tab<P, Q> tab = make_tab<P, Q>(op->mesh->basis);
+    using S = SF<P, Q, T>;
+    const int w = warps_for(sizeof(T) * S::SZ, 8);
+    const size_t smem = sizeof(T) * (S::TAB + w * S::SZ);
     auto go = [&](auto k) -> lsmf_status {
-      LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t));
-      const int g = grid_for(k, 32 * w, smem_t, (a.n_cells + w - 1) / w);
-      k<<<g, 32 * w, smem_t, stream>>>(a, tabt);
+      LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const int g = grid_for(k, 32 * w, smem, (a.n_cells + w - 1) / w);
+      k<<<g, 32 * w, smem, stream>>>(a, tab);
       return LSMF_OK;
     };
-    if (col) {
-      st = stages == 0 ? go(apply_fast_kernel<P, Q, T, VAR, 0, SC_COLOUR>)
-                       : go(apply_fast_kernel<P, Q, T, VAR, 1, SC_COLOUR>);
-    } else if (cellbuf) {
-      st = stages == 0 ? go(apply_fast_kernel<P, Q, T, VAR, 0, SC_CELLBUF>)
-                       : go(apply_fast_kernel<P, Q, T, VAR, 1, SC_CELLBUF>);
-    } else if (peer) {
-      if constexpr (sizeof(T) == 8)
-        st = stages == 0 ? go(apply_fast_kernel<P, Q, T, VAR, 0, SC_PEER>)
-                         : go(apply_fast_kernel<P, Q, T, VAR, 1, SC_PEER>);
-    } else {
-      switch (stages) {
-        case 0: st = go(apply_fast_kernel<P, Q, T, VAR, 0, SC_ATOMIC>); break;
-        case 1: st = go(apply_fast_kernel<P, Q, T, VAR, 1, SC_ATOMIC>); break;
-        case 2: st = go(apply_fast_kernel<P, Q, T, VAR, 2, SC_ATOMIC>); break;
-        default: st = go(apply_fast_kernel<P, Q, T, VAR, 3, SC_ATOMIC>); break;
-      }
-    }
-    if (st != LSMF_OK) return st;
-  } else if (full) {
-    auto k = apply_kernel<P, Q, T, VAR, true>;
-    LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int g = grid_for(k, 32 * w, smem, (a.n_cells + w - 1) / w);
-    k<<<g, 32 * w, smem, stream>>>(a, tab);
-  } else {
-    auto k = apply_kernel<P, Q, T, VAR, false>;
-    LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int g = grid_for(k, 32 * w, smem, (a.n_cells + w - 1) / w);
-    k<<<g, 32 * w, smem, stream>>>(a, tab);
+    if (full) LSMF_TRY(go(apply_kernel<P, Q, T, VAR, true>));
+    else LSMF_TRY(go(apply_kernel<P, Q, T, VAR, false>));
   }
   LSMF_CUDA(cudaGetLastError());
   return LSMF_OK;
@@ -1269,14 +1280,24 @@ lsmf_status run_diag(lsmf_op *op, T *diag, CellRange range) {
   a.dst = diag;
   set_range(a, range);
   if (a.n_cells == 0) return LSMF_OK;
-  const Tab<P, Q> tab = make_tab<P, Q>(op->mesh->basis);
-  using S = SF<P, Q, T>;
-  const int w = warps_for(sizeof(T) * (S::SZ + 36 * S::NQ), 4);
-  const size_t smem = sizeof(T) * (S::TAB + w * (S::SZ + 36 * S::NQ));
+  const TabT<P, Q, T> tab = make_tabt<P, Q, T>(op->mesh->basis);
+  TabSq<P, Q, T> sq;
+  const Basis &b = op->mesh->basis;
+  for (int k = 0; k < Q; ++k)
+    for (int i = 0; i <= P; ++i) {
+      const double n = b.N[k * (P + 1) + i], d = b.D[k * (P + 1) + i];
+      sq.NN[k][i] = T(n * n);
+      sq.ND[k][i] = T(n * d);
+      sq.DD[k][i] = T(d * d);
+    }
+  using S = SFC<P, Q, T>;
+  const int w = 4;
+  const size_t smem = sizeof(T) * w * S::SZ;
   auto k = diagonal_kernel<P, Q, T, VAR>;
   LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int g = grid_for(k, 32 * w, smem, (a.n_cells + w - 1) / w);
-  k<<<g, 32 * w, smem, op->stream>>>(a, tab);
+  const int units = (a.n_cells + S::CPW - 1) / S::CPW + 1;
+  const int g = grid_for(k, 32 * w, smem, (units + w - 1) / w);
+  k<<<g, 32 * w, smem, op->stream>>>(a, tab, sq);
   LSMF_CUDA(cudaGetLastError());
   return LSMF_OK;
 }

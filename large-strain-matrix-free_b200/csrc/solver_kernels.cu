@@ -609,6 +609,8 @@ __global__ void interpolate_kernel(int n_coarse_nodes, int ncn, const int *__res
 // rhs part), evaluated in the reference configuration:
 //   H[c][f] = -sum_d tau[c][d] (J_ref^-1 F^-1)[f][d] JxW_ref
 // MODE 0: scatter into R; MODE 1: grad[cell] = lambda . (cell vector)
+// Q^2 lanes per cell, 32 / Q^2 cells per warp (SFC): cells of the list, or
+// all n_cells cells.
 template <int P, int Q, int MODE>
 __global__ void __launch_bounds__(128) internal_force_kernel(const int *__restrict__ cell_nodes, int n_cells,
                                                               const int *__restrict__ cells, int plain,
@@ -616,59 +618,47 @@ __global__ void __launch_bounds__(128) internal_force_kernel(const int *__restri
                                                               const double *__restrict__ mu_cell, double nu, int formulation,
                                                               double *R, const double *__restrict__ lam, double *grad,
                                                               TabT<P, Q, double> tab, Tab<P, Q> wtab) {
-  using S = SFR<P, Q, double>;
-  constexpr int N1 = P + 1, NN = S::NN, NQ = S::NQ, QPL = S::QPL, RPL = S::RPL, XR = S::XR;
+  using S = SFC<P, Q, double>;
+  constexpr int N1 = P + 1, NN = S::NN, L = S::L, CPW = S::CPW;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   double *slab = (double *)smem_raw + warp * S::SZ;
-  for (int ic = blockIdx.x * wpb + warp; ic < n_cells; ic += gridDim.x * wpb) {
-    const int cell = cells ? __ldg(cells + ic) : ic;
-    const int *cn = cell_nodes + (size_t)cell * NN;
-    int ck[RPL][N1];
-    double vx[RPL][N1], vu[RPL][N1];
+  const LanePos<Q> lp;
+  const int n_units = (n_cells + CPW - 1) / CPW;
+  for (int w = blockIdx.x * wpb + warp; w < n_units; w += gridDim.x * wpb) {
+    const int e = w * CPW + lp.r, ec = e < n_cells ? e : n_cells - 1;
+    const bool valid = lp.act && e < n_cells;
+    const int cell = cells ? __ldg(cells + ec) : ec;
+    const int *cn = cell_nodes + (size_t)cell * NN + lp.t;
+    int ck[N1];
+    double GX[Q][3][3], G[Q][3][3];
+    {
+      double vx[3][N1], vu[3][N1];
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      const int comp = row < XR ? row / (N1 * N1) : 0, kj = row % (N1 * N1);
+      for (int k = 0; k < N1; ++k) ck[k] = __ldg(cn + k * L) & NODE_MASK;
 #pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        if (row < XR) {
-          const int packed = cn[kj * N1 + i];
-          ck[r][i] = packed;
-          const size_t dof = 3 * (size_t)(packed & NODE_MASK) + comp;
-          vx[r][i] = X[dof];
-          vu[r][i] = u[dof];
-        } else {
-          ck[r][i] = 0; vx[r][i] = 0; vu[r][i] = 0;
+      for (int k = 0; k < N1; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          vx[i][k] = __ldg(X + 3 * (size_t)ck[k] + i);
+          vu[i][k] = __ldg(u + 3 * (size_t)ck[k] + i);
         }
-      }
+      S::eval(tab, vx, slab, lp, GX);
+      S::eval(tab, vu, slab, lp, G);
     }
-    double GX[QPL][3][3], GU[QPL][3][3], H[QPL][3][3];
-    S::eval(tab, vx, slab, lane, GX);
-    S::eval(tab, vu, slab, lane, GU);
     const double mu = mu_cell[cell];
     const double lambda = (2.0 * mu * nu) / (1.0 - 2.0 * nu);
     const double kappa = (2.0 * mu * (1.0 + nu)) / (3.0 * (1.0 - 2.0 * nu));
 #pragma unroll
-    for (int l = 0; l < QPL; ++l) {
-      const int q = lane + 32 * l;
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) H[l][c][e] = 0;
-      if (q >= NQ) continue;
-      const double w = wtab.w[q % Q] * wtab.w[(q / Q) % Q] * wtab.w[q / (Q * Q)];
-      double Jr[3][3], Jri[3][3], F[3][3], Fi[3][3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) Jr[d][e] = GX[l][d][e];
-      const double jxw = inv3(Jr, Jri) * w;
+    for (int s = 0; s < Q; ++s) {
+      const double w3 = wtab.w[s] * wtab.w[lp.b] * wtab.w[lp.a];
+      double Jri[3][3], F[3][3], Fi[3][3];
+      const double jxw = inv3(GX[s], Jri) * w3;
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-          F[c][d] = GU[l][c][0] * Jri[0][d] + GU[l][c][1] * Jri[1][d] + GU[l][c][2] * Jri[2][d] + (c == d ? 1.0 : 0.0);
+          F[c][d] = G[s][c][0] * Jri[0][d] + G[s][c][1] * Jri[1][d] + G[s][c][2] * Jri[2][d] + (c == d ? 1.0 : 0.0);
       const double det = inv3(F, Fi);
       double b[3][3];
 #pragma unroll
@@ -678,15 +668,15 @@ __global__ void __launch_bounds__(128) internal_force_kernel(const int *__restri
       double tau[3][3];
       if (formulation == 0) {
         // material.h:119-150: tau = (J dPsi_vol/dJ - tr(tau_bar)/3) I + tau_bar
-        const double s = pow(det, -2.0 / 3.0);
+        const double sc = pow(det, -2.0 / 3.0);
         const double dPsi = (kappa / 2.0) * (det - 1.0 / det);
         double tr = 0;
 #pragma unroll
-        for (int i = 0; i < 3; ++i) tr += b[i][i] * s * mu;
+        for (int i = 0; i < 3; ++i) tr += b[i][i] * sc * mu;
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int j = 0; j < 3; ++j) tau[i][j] = b[i][j] * s * mu + (i == j ? dPsi * det - tr / 3.0 : 0.0);
+          for (int j = 0; j < 3; ++j) tau[i][j] = b[i][j] * sc * mu + (i == j ? dPsi * det - tr / 3.0 : 0.0);
       } else {
         // material.h:151-158: tau = mu b - (mu - 2 lambda ln J) I
         const double tmp = mu - 2.0 * lambda * log(det);
@@ -704,29 +694,32 @@ __global__ void __launch_bounds__(128) internal_force_kernel(const int *__restri
       for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int f = 0; f < 3; ++f)
-          H[l][c][f] = -(tau[c][0] * JF[f][0] + tau[c][1] * JF[f][1] + tau[c][2] * JF[f][2]) * jxw;
+          G[s][c][f] = -(tau[c][0] * JF[f][0] + tau[c][1] * JF[f][1] + tau[c][2] * JF[f][2]) * jxw;
     }
-    double out[RPL][N1];
-    S::integrate(tab, H, slab, lane, out);
+    double out[3][N1];
+    S::integrate(tab, G, slab, lp, out);
     double acc = 0;
 #pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int row = lane + 32 * r;
-      if (row >= XR) continue;
-      const int comp = row / (N1 * N1);
+    for (int k = 0; k < N1; ++k)
 #pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        const size_t dof = 3 * (size_t)(ck[r][i] & NODE_MASK) + comp;
-        if (MODE == 0) {
-          if (plain) R[dof] += out[r][i];
-          else atomicAdd(R + dof, out[r][i]);
+      for (int i = 0; i < 3; ++i) {
+        const size_t dof = 3 * (size_t)ck[k] + i;
+        if (MODE == 1) acc += lam[dof] * out[i][k];
+        else if (valid) {
+          if (plain) R[dof] += out[i][k];
+          else atomicAdd(R + dof, out[i][k]);
         }
-        else acc += lam[dof] * out[r][i];
       }
-    }
     if (MODE == 1) {
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-      if (lane == 0) grad[cell] = acc;
+      // the cell's lanes in order
+      __syncwarp();
+      slab[lp.ln] = acc;
+      __syncwarp();
+      if (valid && lp.t == 0) {
+        double sum = 0;
+        for (int t = 0; t < L; ++t) sum += slab[lp.ln + t];
+        grad[cell] = sum;
+      }
     }
   }
 }
@@ -1047,7 +1040,7 @@ template <int P, int Q, int MODE>
 static lsmf_status internal_force_impl(const Level &L, const Basis &B, const double *u, const double *mu, double nu,
                                        int formulation, double *R, const double *lam, double *grad, int scatter,
                                        cudaStream_t st) {
-  using S = SFR<P, Q, double>;
+  using S = SFC<P, Q, double>;
   TabT<P, Q, double> t;
   Tab<P, Q> w;
   for (int k = 0; k < Q; ++k) {
@@ -1066,7 +1059,7 @@ static lsmf_status internal_force_impl(const Level &L, const Basis &B, const dou
   // the cell gradient (MODE 1) writes one value per cell and needs no colours
   LSMF_TRY(over_colours(L, MODE == 0 ? scatter : LSMF_SCATTER_ATOMIC,
                         [&](const int *cells, int n, int plain) -> lsmf_status {
-                          int g = (n + wpb - 1) / wpb;
+                          int g = ((n + S::CPW - 1) / S::CPW + wpb - 1) / wpb;
                           if (g > 16 * sms()) g = 16 * sms();
                           k<<<g, 32 * wpb, smem, st>>>(L.d_cell_nodes.ptr, n, cells, plain, L.d_X.ptr, u, mu, nu,
                                                         formulation, R, lam, grad, t, w);

@@ -323,10 +323,7 @@ class NeoHookOperator:
 
     def set_pipeline(self, stages):
         """Ring depth (0..3) of the bulk-copy record pipeline in vmult; 0 =
-        plain loads, -1 = the measured default (one stage for the large-record
-        variants of degree 1 or 2 while a record fits in 24 KB, else plain
-        loads).  True/False
-        select 2/0."""
+        plain loads, -1 = the measured default.  True/False select 2/0."""
         if stages is True:
             stages = 2
         check(lib().lsmf_operator_set_option(self.h, 1, int(stages)))
@@ -355,10 +352,8 @@ class NeoHookOperator:
         check(lib().lsmf_operator_set_option(self.h, 6, int(mode)))
 
     def set_cell_pairs(self, mode):
-        """FP32 operators: 1 = two cells per warp in packed f32x2 arithmetic,
-        0 = one cell per warp, -1 = the measured default (pairs for Q1
-        tensor2 / scalar, Q2 tensor2 / scalar / scalar_referential, Q4
-        scalar_referential; formulation 1)."""
+        """-1, 0 or 1; kept for callers that set it.  The FP32 cell loop always
+        runs two cells per lane in packed f32x2 arithmetic."""
         check(lib().lsmf_operator_set_option(self.h, 7, int(mode)))
 
     def set_chunks(self, k):
