@@ -159,92 +159,98 @@ struct LanePos {
 // traffic.  The slab rows are 32 + Q (z / y transposes) and 33 (y / x)
 // entries apart: = Q and = 1 modulo 16 and 32, which makes every access of
 // both sides of a transpose conflict-free for 8- and 4-byte entries.
-template <int P, int Q, typename T>
+// NCG components go through the slab at a time (3, or 1 where shared memory
+// is short: a third of the slab for three times the barriers).
+template <int P, int Q, typename T, int NCG = 3>
 struct SFC {
   static constexpr int N1 = P + 1, NN = N1 * N1 * N1, NQ = Q * Q * Q;
   static_assert(N1 == Q, "q = p + 1");
   static constexpr int L = Q * Q, CPW = 32 / L, LW = CPW * L;
   static constexpr int RA = 32 + Q, RB = 33;
-  static constexpr int BA = Q * RA, BB = Q * RB;              // one component of one field
-  static constexpr int SZ = 6 * BA > 9 * BB ? 6 * BA : 9 * BB;  // per-warp slab (elements of T)
+  static constexpr int BA = Q * RA, BB = Q * RB;  // one component of one field
+  static constexpr int SZ = NCG * (2 * BA > 3 * BB ? 2 * BA : 3 * BB);  // per-warp slab (elements of T)
 
   // v[c][k]: value of component c at node k of the lane's z line ->
   // G[s][c][e]: reference gradient at point s of the lane's x line, and with
   // Vq the values Vq[s][c] there
   static __device__ __forceinline__ void eval(const TabT<P, Q, T> &tb, const T v[3][N1], T *slab, const LanePos<Q> &lp,
                                               T G[Q][3][3], T (*Vq)[3] = nullptr) {
-    __syncwarp();  // the slab's previous readers are done
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+    for (int c0 = 0; c0 < 3; c0 += NCG) {
+      __syncwarp();  // the slab's previous readers are done
 #pragma unroll
-      for (int qz = 0; qz < Q; ++qz) {
-        T s0 = 0, s1 = 0;
+      for (int g = 0; g < NCG; ++g)
 #pragma unroll
-        for (int k = 0; k < N1; ++k) {
-          s0 += tb.N[qz][k] * v[c][k];
-          s1 += tb.D[qz][k] * v[c][k];
+        for (int qz = 0; qz < Q; ++qz) {
+          T s0 = 0, s1 = 0;
+#pragma unroll
+          for (int k = 0; k < N1; ++k) {
+            s0 += tb.N[qz][k] * v[c0 + g][k];
+            s1 += tb.D[qz][k] * v[c0 + g][k];
+          }
+          slab[g * BA + qz * RA + lp.ln] = s0;
+          slab[(NCG + g) * BA + qz * RA + lp.ln] = s1;
         }
-        slab[c * BA + qz * RA + lp.ln] = s0;
-        slab[(3 + c) * BA + qz * RA + lp.ln] = s1;
+      __syncwarp();
+      // lane (qz, i) = (a, b)
+      T a0[NCG][N1], a1[NCG][N1];
+      {
+        const T *A = slab + lp.r * L + lp.b + lp.a * RA;
+#pragma unroll
+        for (int g = 0; g < NCG; ++g)
+#pragma unroll
+          for (int j = 0; j < N1; ++j) {
+            a0[g][j] = A[g * BA + j * Q];
+            a1[g][j] = A[(NCG + g) * BA + j * Q];
+          }
       }
-    __syncwarp();
-    // lane (qz, i) = (a, b)
-    T a0[3][N1], a1[3][N1];
-    {
-      const T *A = slab + lp.r * L + lp.b + lp.a * RA;
+      __syncwarp();
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
+      for (int g = 0; g < NCG; ++g)
 #pragma unroll
-        for (int j = 0; j < N1; ++j) {
-          a0[c][j] = A[c * BA + j * Q];
-          a1[c][j] = A[(3 + c) * BA + j * Q];
+        for (int qy = 0; qy < Q; ++qy) {
+          T s00 = 0, s01 = 0, s10 = 0;
+#pragma unroll
+          for (int j = 0; j < N1; ++j) {
+            s00 += tb.N[qy][j] * a0[g][j];
+            s01 += tb.D[qy][j] * a0[g][j];
+            s10 += tb.N[qy][j] * a1[g][j];
+          }
+          slab[g * BB + qy * RB + lp.ln] = s00;
+          slab[(NCG + g) * BB + qy * RB + lp.ln] = s01;
+          slab[(2 * NCG + g) * BB + qy * RB + lp.ln] = s10;
         }
-    }
-    __syncwarp();
+      __syncwarp();
+      // lane (qz, qy) = (a, b)
+      const T *B = slab + lp.r * L + lp.a * Q + lp.b * RB;
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-#pragma unroll
-      for (int qy = 0; qy < Q; ++qy) {
-        T s00 = 0, s01 = 0, s10 = 0;
-#pragma unroll
-        for (int j = 0; j < N1; ++j) {
-          s00 += tb.N[qy][j] * a0[c][j];
-          s01 += tb.D[qy][j] * a0[c][j];
-          s10 += tb.N[qy][j] * a1[c][j];
-        }
-        slab[c * BB + qy * RB + lp.ln] = s00;
-        slab[(3 + c) * BB + qy * RB + lp.ln] = s01;
-        slab[(6 + c) * BB + qy * RB + lp.ln] = s10;
-      }
-    __syncwarp();
-    // lane (qz, qy) = (a, b)
-    const T *B = slab + lp.r * L + lp.a * Q + lp.b * RB;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      T b0[N1], by[N1], bz[N1];
-#pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        b0[i] = B[c * BB + i];
-        by[i] = B[(3 + c) * BB + i];
-        bz[i] = B[(6 + c) * BB + i];
-      }
-#pragma unroll
-      for (int s = 0; s < Q; ++s) {
-        T gx = 0, gy = 0, gz = 0;
+      for (int g = 0; g < NCG; ++g) {
+        const int c = c0 + g;
+        T b0[N1], by[N1], bz[N1];
 #pragma unroll
         for (int i = 0; i < N1; ++i) {
-          gx += tb.D[s][i] * b0[i];
-          gy += tb.N[s][i] * by[i];
-          gz += tb.N[s][i] * bz[i];
+          b0[i] = B[g * BB + i];
+          by[i] = B[(NCG + g) * BB + i];
+          bz[i] = B[(2 * NCG + g) * BB + i];
         }
-        G[s][c][0] = gx;
-        G[s][c][1] = gy;
-        G[s][c][2] = gz;
-        if (Vq) {
-          T x = 0;
 #pragma unroll
-          for (int i = 0; i < N1; ++i) x += tb.N[s][i] * b0[i];
-          Vq[s][c] = x;
+        for (int s = 0; s < Q; ++s) {
+          T gx = 0, gy = 0, gz = 0;
+#pragma unroll
+          for (int i = 0; i < N1; ++i) {
+            gx += tb.D[s][i] * b0[i];
+            gy += tb.N[s][i] * by[i];
+            gz += tb.N[s][i] * bz[i];
+          }
+          G[s][c][0] = gx;
+          G[s][c][1] = gy;
+          G[s][c][2] = gz;
+          if (Vq) {
+            T x = 0;
+#pragma unroll
+            for (int i = 0; i < N1; ++i) x += tb.N[s][i] * b0[i];
+            Vq[s][c] = x;
+          }
         }
       }
     }
@@ -254,78 +260,81 @@ struct SFC {
   // of component c at node k of the lane's z line
   static __device__ __forceinline__ void integrate(const TabT<P, Q, T> &tb, const T H[Q][3][3], T *slab,
                                                    const LanePos<Q> &lp, T out[3][N1]) {
-    __syncwarp();
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+    for (int c0 = 0; c0 < 3; c0 += NCG) {
+      __syncwarp();
 #pragma unroll
-      for (int i = 0; i < N1; ++i) {
-        T zx = 0, zy = 0, zz = 0;
+      for (int g = 0; g < NCG; ++g)
 #pragma unroll
-        for (int s = 0; s < Q; ++s) {
-          zx += tb.D[s][i] * H[s][c][0];
-          zy += tb.N[s][i] * H[s][c][1];
-          zz += tb.N[s][i] * H[s][c][2];
+        for (int i = 0; i < N1; ++i) {
+          T zx = 0, zy = 0, zz = 0;
+#pragma unroll
+          for (int s = 0; s < Q; ++s) {
+            zx += tb.D[s][i] * H[s][c0 + g][0];
+            zy += tb.N[s][i] * H[s][c0 + g][1];
+            zz += tb.N[s][i] * H[s][c0 + g][2];
+          }
+          slab[g * BB + i * RB + lp.ln] = zx;
+          slab[(NCG + g) * BB + i * RB + lp.ln] = zy;
+          slab[(2 * NCG + g) * BB + i * RB + lp.ln] = zz;
         }
-        slab[c * BB + i * RB + lp.ln] = zx;
-        slab[(3 + c) * BB + i * RB + lp.ln] = zy;
-        slab[(6 + c) * BB + i * RB + lp.ln] = zz;
-      }
-    __syncwarp();
-    // lane (qz, i) = (a, b)
-    T o1[3][N1], o2[3][N1];
-    {
-      const T *Z = slab + lp.r * L + lp.a * Q + lp.b * RB;
+      __syncwarp();
+      // lane (qz, i) = (a, b)
+      T o1[NCG][N1], o2[NCG][N1];
+      {
+        const T *Z = slab + lp.r * L + lp.a * Q + lp.b * RB;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        T zx[Q], zy[Q], zz[Q];
-#pragma unroll
-        for (int qy = 0; qy < Q; ++qy) {
-          zx[qy] = Z[c * BB + qy];
-          zy[qy] = Z[(3 + c) * BB + qy];
-          zz[qy] = Z[(6 + c) * BB + qy];
-        }
-#pragma unroll
-        for (int j = 0; j < N1; ++j) {
-          T s1 = 0, s2 = 0;
+        for (int g = 0; g < NCG; ++g) {
+          T zx[Q], zy[Q], zz[Q];
 #pragma unroll
           for (int qy = 0; qy < Q; ++qy) {
-            s1 += tb.N[qy][j] * zx[qy];
-            s1 += tb.D[qy][j] * zy[qy];
-            s2 += tb.N[qy][j] * zz[qy];
+            zx[qy] = Z[g * BB + qy];
+            zy[qy] = Z[(NCG + g) * BB + qy];
+            zz[qy] = Z[(2 * NCG + g) * BB + qy];
           }
-          o1[c][j] = s1;
-          o2[c][j] = s2;
+#pragma unroll
+          for (int j = 0; j < N1; ++j) {
+            T s1 = 0, s2 = 0;
+#pragma unroll
+            for (int qy = 0; qy < Q; ++qy) {
+              s1 += tb.N[qy][j] * zx[qy];
+              s1 += tb.D[qy][j] * zy[qy];
+              s2 += tb.N[qy][j] * zz[qy];
+            }
+            o1[g][j] = s1;
+            o2[g][j] = s2;
+          }
         }
       }
-    }
-    __syncwarp();
+      __syncwarp();
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+      for (int g = 0; g < NCG; ++g)
 #pragma unroll
-      for (int j = 0; j < N1; ++j) {
-        slab[c * BA + j * RA + lp.ln] = o1[c][j];
-        slab[(3 + c) * BA + j * RA + lp.ln] = o2[c][j];
-      }
-    __syncwarp();
-    // lane (j, i) = (a, b)
-    const T *Y = slab + lp.r * L + lp.b + lp.a * RA;
+        for (int j = 0; j < N1; ++j) {
+          slab[g * BA + j * RA + lp.ln] = o1[g][j];
+          slab[(NCG + g) * BA + j * RA + lp.ln] = o2[g][j];
+        }
+      __syncwarp();
+      // lane (j, i) = (a, b)
+      const T *Y = slab + lp.r * L + lp.b + lp.a * RA;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      T y1[Q], y2[Q];
-#pragma unroll
-      for (int qz = 0; qz < Q; ++qz) {
-        y1[qz] = Y[c * BA + qz * Q];
-        y2[qz] = Y[(3 + c) * BA + qz * Q];
-      }
-#pragma unroll
-      for (int k = 0; k < N1; ++k) {
-        T s = 0;
+      for (int g = 0; g < NCG; ++g) {
+        T y1[Q], y2[Q];
 #pragma unroll
         for (int qz = 0; qz < Q; ++qz) {
-          s += tb.N[qz][k] * y1[qz];
-          s += tb.D[qz][k] * y2[qz];
+          y1[qz] = Y[g * BA + qz * Q];
+          y2[qz] = Y[(NCG + g) * BA + qz * Q];
         }
-        out[c][k] = s;
+#pragma unroll
+        for (int k = 0; k < N1; ++k) {
+          T s = 0;
+#pragma unroll
+          for (int qz = 0; qz < Q; ++qz) {
+            s += tb.N[qz][k] * y1[qz];
+            s += tb.D[qz][k] * y2[qz];
+          }
+          out[c0 + g][k] = s;
+        }
       }
     }
   }

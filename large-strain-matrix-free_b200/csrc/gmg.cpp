@@ -273,6 +273,11 @@ lsmf_status chebyshev_run(lsmf_gmg *g, int l, T *x, const T *b, bool zero_start)
   const T *invd = (const T *)op->d_inv_diag.ptr;
   const lsmf_cheb &c = GL.cheb;
   const uint8_t *cm = op->L().d_cmask.ptr;
+  // a small level with many steps: all of them in one cooperative kernel
+  // (its start, ~8 us, is worth it from about four steps on: a step takes
+  // ~2-4 us there and 8-10 us as two launches)
+  if (l == 0 && zero_start && g->coarse.usable && !op->basic && c.degree >= 4 && std::fabs(c.delta) >= 1e-40)
+    return launch_coarse_cheb(op, g->coarse, x, b, c.theta, c.delta, c.degree);
   // r is kept at zero between the steps by the update kernels
   if (zero_start) {
     LSMF_TRY(cheb_zero_async<T>(x, b, invd, c.theta, n, st));
@@ -455,6 +460,14 @@ lsmf_status lsmf_gmg_create(lsmf_mesh *m, const lsmf_gmg_desc *desc, lsmf_gmg **
     if ((s = GL.x.alloc(n)) != LSMF_OK || (s = GL.b.alloc(n)) != LSMF_OK || (s = GL.r.alloc(n)) != LSMF_OK ||
         (s = GL.xold.alloc(n)) != LSMF_OK || (s = GL.u.alloc(n)) != LSMF_OK)
       break;
+  }
+  if (s == LSMF_OK && desc->coarse_chebyshev) {
+    int dev = 0, sms = 0, smem = 0, coop = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop)
+      s = build_coarse_plan(g->levels[0].op, sms, (size_t)smem - 1024, g->coarse);
   }
   if (s == LSMF_OK) s = g->sc.alloc(SC_N);
   if (s == LSMF_OK) s = g->partial.alloc(2 * (size_t)reduce_blocks());  // two partial-sum arrays
@@ -646,15 +659,22 @@ lsmf_status lsmf_cg_solve(lsmf_op *A, int precond, double omega, lsmf_gmg *gmg, 
       ++k;
     }
   }
-  int flag = 0;
+  int flag = 0, coarse_flag = 0;
   LSMF_CUDA(cudaMemcpyAsync(&flag, A->d_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+  // the coarse-level kernel of the preconditioner has bounded waits too
+  int *d_coarse_flag = precond == 2 && gmg->coarse.usable ? gmg->levels[0].op->d_flag.ptr : nullptr;
+  if (d_coarse_flag) LSMF_CUDA(cudaMemcpyAsync(&coarse_flag, d_coarse_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   LSMF_CUDA(cudaStreamSynchronize(st));
+  if (coarse_flag & 2) {
+    LSMF_CUDA(cudaMemsetAsync(d_coarse_flag, 0, sizeof(int), st));
+    flag |= 2;
+  }
   if (info) { info->iterations = it; info->residual = res; info->converged = conv ? 1 : 0; }
   if (flag & 2) {
     // reported once: the word is cleared for the calls that follow
     LSMF_CUDA(cudaMemsetAsync(A->d_flag.ptr, 0, sizeof(int), st));
     LSMF_CUDA(cudaStreamSynchronize(st));
-    set_error("a bounded device wait timed out in the vmult kernel");
+    set_error("a bounded device wait timed out in the vmult or the coarse-level kernel");
     return LSMF_ERR_TIMEOUT;
   }
   if (flag & 4) {

@@ -416,6 +416,12 @@ lsmf_status launch_apply_cells(const lsmf_op *op, void *dst, const void *src) {
   return for_cell_ranges(op->L(), op->scatter, [&](CellRange r) { return t->apply(op, dst, src, mask, r); });
 }
 
+lsmf_status launch_coarse_cheb(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta,
+                               double delta, int degree) {
+  const OpsTable *t = table_of(op);
+  return t ? t->coarse_cheb(op, plan, x, b, theta, delta, degree) : LSMF_ERR_UNSUPPORTED;
+}
+
 // K g over the constrained columns: gather without zeroing, scatter skipping
 // constrained rows (dst zeroed first, no identity rows)
 lsmf_status launch_apply_inhomogeneous(const lsmf_op *op, void *dst, const void *g) {

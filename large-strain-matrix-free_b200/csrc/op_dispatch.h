@@ -2,6 +2,7 @@
 // (P, Number) pair is compiled in its own unit (op_p<P>_<f64|f32>.cu) so
 // that the instantiations build in parallel; kernels.cu dispatches here.
 #pragma once
+#include "coarse_plan.h"
 #include "lsmf_internal.h"
 
 namespace lsmf {
@@ -38,6 +39,11 @@ struct OpsTable {
   // `mask`, internal bit MASK_INHOM_BIT: gather constrained entries)
   lsmf_status (*apply)(const lsmf_op *op, void *dst, const void *src, unsigned mask, CellRange range);
   lsmf_status (*diag)(lsmf_op *op, void *diag, CellRange range);
+  // coarse-level solver (coarse_plan.h): sizes of a CTA with W working warps,
+  // and x = the degree-step Chebyshev solution of A x = b from zero
+  CoarseShape (*coarse_shape)(const lsmf_op *op, int W);
+  lsmf_status (*coarse_cheb)(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta, double delta,
+                             int degree);
 };
 
 // gather constrained entries instead of zeroing them (the inhomogeneity

@@ -17,6 +17,7 @@
 
 #include "cell_kernels.cuh"
 #include "lsmf_internal.h"
+#include "coarse_plan.h"
 #include "op_dispatch.h"
 #include "pair.cuh"
 
@@ -497,6 +498,55 @@ __device__ __forceinline__ T join_of(const typename Num<T>::S *h, int stride) {
   else return h[0];
 }
 
+// One quadrature point of a lane's x line: G (reference gradient of the
+// source) becomes H, what the transposed sweeps take.  slice: the cell's
+// record at the point's slice and lane 0 (component stride CS, lane stride
+// TS); ref: the cell's reference metric (entry stride RS) when ref_per_cell;
+// park: the point's displacement gradient (scalar variants), entry stride
+// LW; ux: displacement along the x line (scalar_referential).
+template <int Q, typename T, int VAR, int CS, int TS, int LW, typename R, typename RF, typename DC>
+__device__ __forceinline__ void line_point(T G[3][3], int s, const R &slice, const RF &ref, int RS, bool ref_per_cell,
+                                           const T *park, const T ux[3][Q], const LanePos<Q> &lp, const DC &Dc, T mu,
+                                           T lambda, T kappa) {
+  constexpr bool SCALAR = (VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1);
+  const auto r = slice + lp.t * TS;
+  T Ji[3][3];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * CS];
+  const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * CS]);
+  T g[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) g[i][d] = G[i][0] * Ji[0][d] + G[i][1] * Ji[1][d] + G[i][2] * Ji[2][d];
+  ScalarState<T> st;
+  if (SCALAR) {
+    T Jr[3][3];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) Jr[i / 3][i % 3] = ref_per_cell ? T(ref[i * RS]) : T(r[(C_VAR + 1 + i) * CS]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const T u0 = park[(3 * i) * LW], u1 = park[(3 * i + 1) * LW], u2 = park[(3 * i + 2) * LW];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) st.F[i][d] = u0 * Jr[0][d] + u1 * Jr[1][d] + u2 * Jr[2][d] + (i == d ? T(1) : T(0));
+    }
+    st.det = det3(st.F);
+  }
+  if (VAR == VAR_SCALAR_REF) {
+    collocation_F<Q, CS, TS>(ux, slice, s, lp.b, lp.a, Dc, Ji, st.F);
+    st.det = det3(st.F);
+  }
+  T Qm[3][3];
+  physics<T, VAR, CS>(g, r, mu, lambda, kappa, st, Qm);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const T h0 = Qm[i][0] * Ji[e][0] + Qm[i][1] * Ji[e][1] + Qm[i][2] * Ji[e][2];
+      G[i][e] = variant_folds_jxw(VAR) ? h0 : T(h0 * jxw);
+    }
+}
+
 // Blocks of 128 threads the register allocation leaves room for: three (168
 // registers, 12 warps per SM) up to degree 2, where the working set fits
 // (60^3 Q2 FP64: tensor4 311 -> 303 us, scalar 367 -> 348, scalar_referential
@@ -685,46 +735,8 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
       kappa = join_of<T>(m[2], H - 1);
     }
     const auto ref = rec_at([](int cell, int be, int se) { return RL::ref(cell, be, se); });
-    // one point: G[s] becomes H[s]; slice: the record at the point's slice
-    // and lane 0 of the cell
     auto point = [&](int s, auto slice) {
-      const auto r = slice + lp.t * TS;
-      T Ji[3][3];
-#pragma unroll
-      for (int i = 0; i < 9; ++i) Ji[i / 3][i % 3] = r[(C_JINV + i) * CS];
-      const T jxw = variant_folds_jxw(VAR) ? T(1) : T(r[C_JXW * CS]);
-      T g[3][3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) g[i][d] = G[s][i][0] * Ji[0][d] + G[s][i][1] * Ji[1][d] + G[s][i][2] * Ji[2][d];
-      ScalarState<T> st;
-      if (SCALAR) {
-        T Jr[3][3];
-#pragma unroll
-        for (int i = 0; i < 9; ++i) Jr[i / 3][i % 3] = a.ref_per_cell ? T(ref[i * RS]) : T(r[(C_VAR + 1 + i) * CS]);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const T u0 = park[(s * 9 + 3 * i) * LW], u1 = park[(s * 9 + 3 * i + 1) * LW], u2 = park[(s * 9 + 3 * i + 2) * LW];
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            st.F[i][d] = u0 * Jr[0][d] + u1 * Jr[1][d] + u2 * Jr[2][d] + (i == d ? T(1) : T(0));
-        }
-        st.det = det3(st.F);
-      }
-      if (VAR == VAR_SCALAR_REF) {
-        collocation_F<Q, CS, TS>(ux, slice, s, lp.b, lp.a, tab.Dc, Ji, st.F);
-        st.det = det3(st.F);
-      }
-      T Qm[3][3];
-      physics<T, VAR, CS>(g, r, mu, lambda, kappa, st, Qm);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-          const T h0 = Qm[i][0] * Ji[e][0] + Qm[i][1] * Ji[e][1] + Qm[i][2] * Ji[e][2];
-          G[s][i][e] = variant_folds_jxw(VAR) ? h0 : T(h0 * jxw);
-        }
+      line_point<Q, T, VAR, CS, TS, LW>(G[s], s, slice, ref, RS, a.ref_per_cell != 0, park + s * 9 * LW, ux, lp, tab.Dc, mu, lambda, kappa);
     };
 #pragma unroll
     for (int s = 0; s < Q; ++s) {
@@ -1041,6 +1053,9 @@ __global__ void __launch_bounds__(128) diagonal_kernel(KArgs<T> a, TabT<P, Q, T>
   }
 }
 
+// ------------------------------------------------ coarse-level solver
+#include "coarse_kernels.cuh"
+
 int g_num_sms = 0;
 int num_sms() {
   if (!g_num_sms) {
@@ -1302,6 +1317,39 @@ lsmf_status run_diag(lsmf_op *op, T *diag, CellRange range) {
   return LSMF_OK;
 }
 
+// Sizes of a CTA of the coarse-level solver with W working warps
+template <int P, int Q, typename T, int VAR>
+CoarseShape coarse_shape(const lsmf_op *op, int W) {
+  CoarseShape s;
+  s.batch = 32 / (Q * Q);
+  s.cells = W * s.batch;
+  s.unit_bytes = coarse_unit_bytes<P, Q, T, VAR>(op->slice_elems);
+  s.out_offset = coarse_out_offset<P, Q, T, VAR>(op->slice_elems);
+  return s;
+}
+
+template <int P, int Q, typename T, int VAR>
+lsmf_status run_coarse_cheb(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta, double delta,
+                            int degree) {
+  auto a = make_args<T>(op);
+  const TabT<P, Q, T> tab = make_tabt<P, Q, T>(op->mesh->basis);
+  CoarseArgs<T> ca = coarse_args<T>(plan);
+  ca.b = (const T *)b;
+  ca.x = (T *)x;
+  ca.invd = (const T *)op->d_inv_diag.ptr;
+  ca.cmask = op->L().d_cmask.ptr;
+  ca.theta = theta;
+  ca.delta = delta;
+  ca.degree = degree;
+  // every packet of the exchange starts without a tag
+  if (plan.xbuf.n) LSMF_CUDA(cudaMemsetAsync(plan.xbuf.ptr, 0, plan.xbuf.n * sizeof(ulonglong2), op->stream));
+  auto k = plan.max_nodes <= 2 * COARSE_THREADS ? coarse_cheb_kernel<P, Q, T, VAR, 2> : coarse_cheb_kernel<P, Q, T, VAR, 4>;
+  LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+  void *args[] = {(void *)&a, (void *)&tab, (void *)&ca};
+  LSMF_CUDA(cudaLaunchCooperativeKernel((const void *)k, dim3(plan.n_cta), dim3(COARSE_THREADS), args, plan.smem, op->stream));
+  return LSMF_OK;
+}
+
 #define LSMF_DISPATCH_VAR(v, ...)                                                     \
   [&]() -> lsmf_status {                                                              \
     switch (v) {                                                                      \
@@ -1327,8 +1375,17 @@ struct DegreeOps {
   static lsmf_status diag(lsmf_op *op, void *d, CellRange range) {
     return LSMF_DISPATCH_VAR(variant_of(op), (run_diag<P, Q, T, V_>(op, (T *)d, range)));
   }
+  static CoarseShape shape(const lsmf_op *op, int W) {
+    CoarseShape s;
+    (void)LSMF_DISPATCH_VAR(variant_of(op), (s = coarse_shape<P, Q, T, V_>(op, W), LSMF_OK));
+    return s;
+  }
+  static lsmf_status cheb(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta, double delta,
+                          int degree) {
+    return LSMF_DISPATCH_VAR(variant_of(op), (run_coarse_cheb<P, Q, T, V_>(op, plan, x, b, theta, delta, degree)));
+  }
   static const OpsTable &table() {
-    static const OpsTable t = {&cache, &apply, &diag};
+    static const OpsTable t = {&cache, &apply, &diag, &shape, &cheb};
     return t;
   }
 };

@@ -2,8 +2,10 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <vector>
 
+#include "coarse_plan.h"
 #include "lsmf_internal.h"
 
 namespace lsmf {
@@ -79,6 +81,11 @@ lsmf_status adjoint_cell_grad_async(const Level &L, const Basis &B, const double
 // constrained columns, the inhomogeneity term of the rhs)
 lsmf_status launch_apply_inhomogeneous(const lsmf_op *op, void *dst, const void *g);
 
+// x = the degree-step Chebyshev solution of A x = b from zero on the level of
+// a usable plan (one cooperative kernel)
+lsmf_status launch_coarse_cheb(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta,
+                               double delta, int degree);
+
 // Eigenvalues of a symmetric tridiagonal matrix (Sturm bisection).
 double tridiag_eig(const std::vector<double> &d, const std::vector<double> &e, bool want_max);
 
@@ -114,6 +121,8 @@ struct lsmf_gmg {
   // pinned host copies of two batches of alpha / beta / residual history
   // (2 slots x 3 x 8 doubles), read while the next batch runs
   double *eig_pinned = nullptr;
+  // level-0 Chebyshev iteration as one cooperative kernel, where it fits
+  lsmf::CoarsePlan coarse;
   cudaStream_t stream = 0;
   bool ready = false;
   // the V-cycle replayed as one CUDA graph: captured again after each
