@@ -88,7 +88,7 @@ struct CoarseArgs {
   const uint16_t *lid, *contrib, *item_place, *first;
   const unsigned *nodes;
   const uint8_t *sums;
-  ulonglong2 *xbuf;
+  ulonglong2 *xbuf, *rbuf;
   const E *b, *invd;
   const uint8_t *cmask;
   E *x;
@@ -117,6 +117,7 @@ CoarseArgs<E> coarse_args(const CoarsePlan &p) {
   c.nodes = p.nodes;
   c.sums = p.sums;
   c.xbuf = p.xbuf.ptr;
+  c.rbuf = p.xbuf.ptr + (size_t)2 * p.n_slots * p.packets;
   return c;
 }
 
@@ -134,6 +135,22 @@ __device__ __forceinline__ ulonglong2 ld_packet(const ulonglong2 *p) {
                : "memory");
   return v;
 }
+// A load that comes before its packet is not only in vain: it leaves the old
+// line in the reader's half of the L2, which the store has to invalidate
+// first.  So a reader waits about as long as a store takes before it looks.
+__device__ __forceinline__ void coarse_pause(int cycles) {
+  const long long t0 = clock64();
+  while (clock64() - t0 < cycles) {
+  }
+}
+// measured at 15^3 / 8^3 Q2 cells (FP32, FP64): the reduction's lines have a
+// reader in every CTA, an estimate's iteration takes 10.4 / 7.8 / 12.0 / 9.6
+// us without a pause and 8.0 / 6.2 / 9.8 / 7.5 us with this one
+constexpr int PAUSE_ALL_SUM = 800;
+// exchange of shared nodes (one reader a line): FP32 15^3 Chebyshev step 3.75
+// -> 3.63 us, estimate 7.67 -> 7.35 us; FP64 estimate 9.46 -> 9.4 us
+template <typename E>
+__host__ __device__ constexpr int pause_exchange() { return sizeof(E) == 4 ? 300 : 100; }
 __device__ __forceinline__ unsigned packet_tag(const ulonglong2 &v) { return (unsigned)(v.y >> 32); }
 template <typename E>
 struct Packet;
@@ -388,6 +405,7 @@ struct CoarseNodes {
   // the other CTAs' sums into recv.  false: a wait ran out
   __device__ __forceinline__ bool receive(unsigned step, int tries) {
     const ulonglong2 *buf = xbuf + (size_t)(step & 1) * n_slots * PK;
+    coarse_pause(pause_exchange<E>());
     ulonglong2 v[IB][PK];
 #pragma unroll
     for (int j = 0; j < IB; ++j)
@@ -477,8 +495,7 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
     cells.apply(nodes.xg);
     __syncthreads();
     nodes.sum_and_send((unsigned)k);
-    // the step's coefficients, while the sums are on their way (a load issued
-    // at once would come back too early and cost a second trip)
+    // the step's coefficients, while the sums are on their way
     const double rhokp = 1. / (2. * sigma - rhok), f1 = rhokp * rhok, f2 = 2. * rhokp / ca.delta;
     rhok = rhokp;
     if (!nodes.receive((unsigned)k, a.wait_tries)) dead = 1;
@@ -508,5 +525,192 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
     if (!nodes.has(q) || !(nodes.node[q] & 1)) continue;
 #pragma unroll
     for (int i = 0; i < 3; ++i) ca.x[3 * (size_t)(nodes.node[q] >> 1) + i] = T(x[q][i]);
+  }
+}
+
+// Sums of v[0..NV) over all CTAs, the same bits in every thread of every CTA:
+// each CTA's sums go out as tagged packets and every CTA adds all of them in
+// CTA order.  Two buffers alternate (a CTA stores reduction r + 2 after it
+// has seen every CTA's r + 1, which they store after reading r).
+template <int NV>
+__device__ __forceinline__ bool coarse_all_sum(double v[NV], ulonglong2 *rbuf, int n_cta, unsigned tag, int tries,
+                                               double (*sh)[COARSE_MAX_WARPS][2]) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto warp_sum = [&](double x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const double s = warp_sum(v[j]);
+    if (lane == 0) sh[0][warp][j] = s;
+  }
+  __syncthreads();
+  // a line of its own for every writer
+  constexpr int STRIDE = 8;
+  ulonglong2 *buf = rbuf + (size_t)(tag & 1) * n_cta * STRIDE;
+  if (threadIdx.x < NV) {
+    double s = 0;
+#pragma unroll
+    for (int w = 0; w < COARSE_MAX_WARPS; ++w) s += sh[0][w][threadIdx.x];
+    st_packet(buf + STRIDE * blockIdx.x + threadIdx.x, __double_as_longlong(s), (unsigned long long)tag << 32);
+  }
+  bool ok = true;
+  double r[NV];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) r[j] = 0;
+  if (threadIdx.x < n_cta) {
+    coarse_pause(PAUSE_ALL_SUM);
+    const ulonglong2 *p = buf + STRIDE * threadIdx.x;
+    for (int t = 0;; ++t) {
+      bool all = true;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const ulonglong2 q = ld_packet(p + j);
+        r[j] = __longlong_as_double(q.x);
+        all = all && packet_tag(q) == tag;
+      }
+      if (all) break;
+      if (t >= tries) {
+        ok = false;
+        break;
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const double s = warp_sum(r[j]);
+    if (lane == 0) sh[1][warp][j] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    double s = 0;
+#pragma unroll
+    for (int w = 0; w < COARSE_MAX_WARPS; ++w) s += sh[1][w][j];
+    v[j] = s;
+  }
+  return ok;
+}
+
+struct CoarseEigArgs {
+  double mean;                          // of i mod 11 over the dofs
+  double tol_abs, tol_rel;
+  int max_it;
+  double *alpha, *beta, *res2;          // history
+  int *its;
+};
+
+// The eigenvalue estimate's CG (Jacobi, start vector (i mod 11) - mean) with
+// its three dot products reduced over the CTAs: the arithmetic of eig_start /
+// eig_dh / eig_update_precond / eig_dir_clear, stopped at the tolerance.  An
+// iteration at 15^3 Q2 cells takes 7.4 us (FP32) / 9.4 us (FP64), of which the
+// two reductions are about 3 us, where a cell loop and five vector and
+// reduction launches took 18 / 20 us.
+template <int P, int Q, typename T, int VAR, int NPT>
+__global__ void __launch_bounds__(COARSE_THREADS, 1)
+    coarse_eig_kernel(KArgs<T> a, TabT<P, Q, T> tab, CoarseArgs<T> ca, CoarseEigArgs ea) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ double sh[2][COARSE_MAX_WARPS][2];
+  __shared__ int dead;
+  if (threadIdx.x == 0) dead = 0;
+  CoarseCells<P, Q, T, VAR> cells(a, tab, ca, smem);
+  CoarseNodes<T, NPT> nodes(ca, smem);
+  T g[NPT][3], d[NPT][3], iv[NPT][3];
+  double s[2] = {0, 0};
+#pragma unroll
+  for (int q = 0; q < NPT; ++q) {
+    if (!nodes.has(q)) continue;
+    const bool own = nodes.node[q] & 1;
+    double dd[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const size_t dof = 3 * (size_t)(nodes.node[q] >> 1) + i;
+      iv[q][i] = ca.invd[dof];
+      g[q][i] = T(ea.mean - (double)(dof % 11));
+      const T h = T(1) * iv[q][i] * g[q][i];
+      d[q][i] = -h;
+      dd[i] = (double)d[q][i];
+      if (own) {
+        s[0] += (double)g[q][i] * (double)g[q][i];
+        s[1] += (double)g[q][i] * (double)h;
+      }
+    }
+    nodes.put_x(q, dd);
+  }
+  __syncthreads();
+  unsigned tag = 1;
+  auto all_sum = [&](auto &v, auto nv) {
+    if (!coarse_all_sum<decltype(nv)::value>(v, ca.rbuf, ca.n_cta, tag++, a.wait_tries, sh)) dead = 1;
+  };
+  all_sum(s, std::integral_constant<int, 2>{});
+  double gh = s[1];
+  const double res0 = sqrt(s[0]);
+  const double tol = fmax(ea.tol_abs, ea.tol_rel * res0);
+  int its = 0;
+  bool done = !(res0 > tol) || ea.max_it < 1;
+  while (!done) {
+    const int k = its++;
+    cells.apply(nodes.xg);
+    __syncthreads();
+    nodes.sum_and_send((unsigned)(k + 1));
+    if (!nodes.receive((unsigned)(k + 1), a.wait_tries)) dead = 1;
+    __syncthreads();
+    if (dead) break;
+    nodes.finish();
+    double dh[1] = {0};
+#pragma unroll
+    for (int q = 0; q < NPT; ++q) {
+      if (!nodes.has(q)) continue;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        if (nodes.constrained(q, i)) nodes.sum[q][i] = d[q][i];  // identity rows
+        if (nodes.node[q] & 1) dh[0] += (double)d[q][i] * (double)nodes.sum[q][i];
+      }
+    }
+    all_sum(dh, std::integral_constant<int, 1>{});
+    const double alpha = gh / dh[0];
+    s[0] = s[1] = 0;
+    T h[NPT][3];
+#pragma unroll
+    for (int q = 0; q < NPT; ++q) {
+      if (!nodes.has(q)) continue;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        g[q][i] = T((double)g[q][i] + alpha * (double)nodes.sum[q][i]);
+        h[q][i] = T(1) * iv[q][i] * g[q][i];
+        if (nodes.node[q] & 1) {
+          s[0] += (double)g[q][i] * (double)g[q][i];
+          s[1] += (double)g[q][i] * (double)h[q][i];
+        }
+      }
+    }
+    all_sum(s, std::integral_constant<int, 2>{});
+    const double beta = s[1] / gh;
+    gh = s[1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      ea.alpha[k] = alpha;
+      ea.beta[k] = beta;
+      ea.res2[k] = s[0];
+    }
+    done = sqrt(s[0]) <= tol || its >= ea.max_it;
+#pragma unroll
+    for (int q = 0; q < NPT; ++q) {
+      if (!nodes.has(q)) continue;
+      double dd[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        d[q][i] = T(beta * (double)d[q][i] - (double)h[q][i]);
+        dd[i] = (double)d[q][i];
+      }
+      nodes.put_x(q, dd);
+    }
+    __syncthreads();
+    if (dead) break;
+  }
+  if (threadIdx.x == 0) {
+    if (dead) atomicOr(a.flag, FLAG_TIMEOUT);
+    if (blockIdx.x == 0) *ea.its = its;
   }
 }

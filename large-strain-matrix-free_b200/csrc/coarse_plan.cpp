@@ -249,7 +249,7 @@ lsmf_status build_coarse_plan(const lsmf_op *op, int sms, size_t smem_limit, Coa
   plan.item_place = (const uint16_t *)(d + o_place);
   plan.first = (const uint16_t *)(d + o_first);
   plan.sums = d + o_sums;
-  LSMF_TRY(plan.xbuf.alloc((size_t)2 * n_slots * plan.packets + (size_t)4 * P));
+  LSMF_TRY(plan.xbuf.alloc((size_t)2 * n_slots * plan.packets + (size_t)16 * P));
   plan.usable = true;
   return LSMF_OK;
 }

@@ -47,7 +47,17 @@ struct CoarsePlan {
   const uint16_t *first = nullptr;       // [cta][max_nodes]: first sum of a shared node in the receive array
   const uint8_t *sums = nullptr;         // [cta][max_nodes]: number of its sums | place of the own one << 4 (0: not shared)
   DevBuf<uint8_t> lists;
-  mutable DevBuf<ulonglong2> xbuf;  // two exchange buffers of n_slots * packets
+  mutable DevBuf<ulonglong2> xbuf;  // two exchange buffers of n_slots * packets, two of 8 * n_cta (reductions)
+};
+
+// The CG of an eigenvalue estimate: mean of the start vector's integers i mod
+// 11, tolerance max(tol_abs, tol_rel * initial residual), and where its
+// history (alpha, beta, squared residual per iteration) and iteration count go
+struct CoarseEig {
+  double mean = 0, tol_abs = 0, tol_rel = 0;
+  int max_it = 0;
+  double *alpha = nullptr, *beta = nullptr, *res2 = nullptr;
+  int *its = nullptr;
 };
 
 // shared memory of a CTA beside its units

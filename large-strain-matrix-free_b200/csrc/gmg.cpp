@@ -79,15 +79,79 @@ lsmf_status estimate_eigenvalues(lsmf_gmg *g, int l, int max_it, double &emin, d
   lsmf_op *op = GL.op;
   const size_t n = (size_t)op->L().n_dofs();
   cudaStream_t st = g->stream;
+  // start vector (i mod 11) - mean, made on the device; the mean of the
+  // integers i mod 11 is exact in closed form (the sum is below 2^53)
+  const size_t q11 = n / 11, r11 = n % 11;
+  const double mean = (double)(55 * q11 + r11 * (r11 - 1) / 2) / (double)n;
+  const double tol_abs = std::sqrt((double)std::numeric_limits<T>::epsilon()), tol_rel = 1e-10;
+  std::vector<double> dT, oT;
+  its = 0;
+  // Lanczos matrix from the CG coefficients, one iteration at a time
+  double prev_beta = 0, prev_alpha = 0;
+  auto lanczos = [&](double alpha, double beta) {
+    ++its;
+    if (its > 1) {
+      dT.push_back(1.0 / alpha + prev_beta / prev_alpha);
+      oT.push_back(std::sqrt(prev_beta) / prev_alpha);
+    } else {
+      dT.push_back(1.0 / alpha);
+    }
+    prev_beta = beta;
+    prev_alpha = alpha;
+  };
+  auto finish = [&]() {
+    emin = emax = 1.0;
+    if (!dT.empty()) {
+      emin = tridiag_eig(dT, oT, false);
+      emax = tridiag_eig(dT, oT, true);
+    }
+    return LSMF_OK;
+  };
+  // one history buffer for every level (sized for the largest iteration
+  // budget, so no level re-allocates it)
+  size_t need = 0;
+  for (const auto &L : g->levels) need = std::max(need, (size_t)L.op->L().n_dofs());
+  need = 3 * (std::max(need, (size_t)g->desc.eig_cg_iterations) + 8);
+  if (g->eig_hist.n < need) LSMF_TRY(g->eig_hist.alloc(need));
+  const size_t stride = need / 3;
+  double *ha = g->eig_hist.ptr, *hb = ha + stride, *hr = hb + stride;
+  if (l == 0 && g->coarse.usable && !op->basic) {
+    // the whole CG in one cooperative kernel
+    if (g->eig_kbase.n < 1) LSMF_TRY(g->eig_kbase.alloc(1));
+    CoarseEig e;
+    e.mean = mean;
+    e.tol_abs = tol_abs;
+    e.tol_rel = tol_rel;
+    e.max_it = max_it;
+    e.alpha = ha;
+    e.beta = hb;
+    e.res2 = hr;
+    e.its = g->eig_kbase.ptr;
+    LSMF_TRY(launch_coarse_eig(op, g->coarse, e));
+    int m = 0, flag = 0;
+    LSMF_CUDA(cudaMemcpyAsync(&m, g->eig_kbase.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    LSMF_CUDA(cudaMemcpyAsync(&flag, op->d_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    LSMF_CUDA(cudaStreamSynchronize(st));
+    if (flag & 2) {
+      // reported once: the word is cleared for the calls that follow
+      LSMF_CUDA(cudaMemsetAsync(op->d_flag.ptr, 0, sizeof(int), st));
+      set_error("a bounded device wait timed out in the coarse-level eigenvalue estimate");
+      return LSMF_ERR_TIMEOUT;
+    }
+    std::vector<double> h((size_t)2 * m);
+    if (m) {
+      LSMF_CUDA(cudaMemcpyAsync(h.data(), ha, m * sizeof(double), cudaMemcpyDeviceToHost, st));
+      LSMF_CUDA(cudaMemcpyAsync(h.data() + m, hb, m * sizeof(double), cudaMemcpyDeviceToHost, st));
+      LSMF_CUDA(cudaStreamSynchronize(st));
+    }
+    for (int k = 0; k < m; ++k) lanczos(h[k], h[m + k]);
+    return finish();
+  }
   // work vectors at 16-byte-aligned offsets (whole multiples of 4 values)
   const size_t ns = (n + 3) / 4 * 4;
   T *x = (T *)g->eig_vecs.ptr, *gg = x + ns, *h = gg + ns, *d = h + ns;
   const T *invd = (const T *)op->d_inv_diag.ptr;
   const uint8_t *cm = op->L().d_cmask.ptr;
-  // start vector (i mod 11) - mean, made on the device; the mean of the
-  // integers i mod 11 is exact in closed form (the sum is below 2^53)
-  const size_t q11 = n / 11, r11 = n % 11;
-  const double mean = (double)(55 * q11 + r11 * (r11 - 1) / 2) / (double)n;
   LSMF_TRY(eig_start_async<T>(gg, n, mean, st));  // g = A 0 - b
   LSMF_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), st));
   double *sc = g->sc.ptr, *part = g->partial.ptr;
@@ -101,9 +165,7 @@ lsmf_status estimate_eigenvalues(lsmf_gmg *g, int l, int max_it, double &emin, d
   double res2;
   LSMF_TRY(dot(gg, gg, res2));
   const double res0 = std::sqrt(res2);
-  const double tol = std::max(std::sqrt((double)std::numeric_limits<T>::epsilon()), 1e-10 * res0);
-  std::vector<double> dT, oT;
-  its = 0;
+  const double tol = std::max(tol_abs, tol_rel * res0);
   if (res0 > tol) {
     LSMF_TRY(jacobi_async<T>(h, invd, gg, 1.0, n, st));
     LSMF_CUDA(cudaMemsetAsync(d, 0, n * sizeof(T), st));
@@ -114,14 +176,6 @@ lsmf_status estimate_eigenvalues(lsmf_gmg *g, int l, int max_it, double &emin, d
     // alpha / beta / residual history is read once per batch and the Lanczos
     // matrix is cut at the first iteration that meets the tolerance, so the
     // estimate equals the one of an iteration checked every step
-    // one history buffer for every level (sized for the largest iteration
-    // budget, so no level re-allocates it)
-    size_t need = 0;
-    for (const auto &L : g->levels) need = std::max(need, (size_t)L.op->L().n_dofs());
-    need = 3 * (std::max(need, (size_t)g->desc.eig_cg_iterations) + 8);
-    if (g->eig_hist.n < need) LSMF_TRY(g->eig_hist.alloc(need));
-    const size_t stride = need / 3;
-    double *ha = g->eig_hist.ptr, *hb = ha + stride, *hr = hb + stride;
     // one batch of iterations k0 + j, j < batch; with kbase the history
     // index is *kbase + j and the batch is the same launch sequence every
     // time (parity of k0 even), so it can be captured once and replayed
@@ -204,7 +258,6 @@ lsmf_status estimate_eigenvalues(lsmf_gmg *g, int l, int max_it, double &emin, d
       return LSMF_OK;
     };
     bool done = false;
-    double prev_beta = 0, prev_alpha = 0;
     int cur = 0;
     if (status == LSMF_OK && max_it > 0) status = issue(cur);
     while (status == LSMF_OK && !done && slot_busy[cur]) {
@@ -214,17 +267,8 @@ lsmf_status estimate_eigenvalues(lsmf_gmg *g, int l, int max_it, double &emin, d
       if (e != cudaSuccess) { set_error(std::string("eigenvalue CG history: ") + cudaGetErrorString(e)); status = LSMF_ERR_CUDA; break; }
       const double *P = g->eig_pinned + cur * 24;
       for (int j = 0; j < slot_n[cur] && !done; ++j) {
-        ++its;
-        const double alpha = P[j];
-        if (its > 1) {
-          dT.push_back(1.0 / alpha + prev_beta / prev_alpha);
-          oT.push_back(std::sqrt(prev_beta) / prev_alpha);
-        } else {
-          dT.push_back(1.0 / alpha);
-        }
+        lanczos(P[j], P[8 + j]);
         if (std::sqrt(P[16 + j]) <= tol || its >= max_it) done = true;
-        prev_beta = P[8 + j];
-        prev_alpha = alpha;
       }
       cur ^= 1;
     }
@@ -237,12 +281,7 @@ lsmf_status estimate_eigenvalues(lsmf_gmg *g, int l, int max_it, double &emin, d
     if (bexec) cudaGraphExecDestroy(bexec);
     if (status != LSMF_OK) return status;
   }
-  emin = emax = 1.0;
-  if (!dT.empty()) {
-    emin = tridiag_eig(dT, oT, false);
-    emax = tridiag_eig(dT, oT, true);
-  }
-  return LSMF_OK;
+  return finish();
 }
 
 // Chebyshev data from the eigenvalue estimates (degree <= 0: "solver" mode

@@ -422,6 +422,11 @@ lsmf_status launch_coarse_cheb(const lsmf_op *op, const CoarsePlan &plan, void *
   return t ? t->coarse_cheb(op, plan, x, b, theta, delta, degree) : LSMF_ERR_UNSUPPORTED;
 }
 
+lsmf_status launch_coarse_eig(const lsmf_op *op, const CoarsePlan &plan, const CoarseEig &e) {
+  const OpsTable *t = table_of(op);
+  return t ? t->coarse_eig(op, plan, e) : LSMF_ERR_UNSUPPORTED;
+}
+
 // K g over the constrained columns: gather without zeroing, scatter skipping
 // constrained rows (dst zeroed first, no identity rows)
 lsmf_status launch_apply_inhomogeneous(const lsmf_op *op, void *dst, const void *g) {

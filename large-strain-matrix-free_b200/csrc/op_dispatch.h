@@ -44,6 +44,8 @@ struct OpsTable {
   CoarseShape (*coarse_shape)(const lsmf_op *op, int W);
   lsmf_status (*coarse_cheb)(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta, double delta,
                              int degree);
+  // ... and the CG of its eigenvalue estimate
+  lsmf_status (*coarse_eig)(const lsmf_op *op, const CoarsePlan &plan, const CoarseEig &e);
 };
 
 // gather constrained entries instead of zeroing them (the inhomogeneity

@@ -1328,26 +1328,55 @@ CoarseShape coarse_shape(const lsmf_op *op, int W) {
   return s;
 }
 
+// launch a coarse-level kernel: cooperative, one CTA per part of the plan
+template <typename K, typename... A>
+lsmf_status launch_coarse(const lsmf_op *op, const CoarsePlan &plan, K k, A &...args) {
+  // every packet starts without a tag
+  LSMF_CUDA(cudaMemsetAsync(plan.xbuf.ptr, 0, plan.xbuf.n * sizeof(ulonglong2), op->stream));
+  LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+  void *ptrs[] = {(void *)&args...};
+  LSMF_CUDA(cudaLaunchCooperativeKernel((const void *)k, dim3(plan.n_cta), dim3(COARSE_THREADS), ptrs, plan.smem, op->stream));
+  return LSMF_OK;
+}
+template <typename T>
+CoarseArgs<T> coarse_level_args(const lsmf_op *op, const CoarsePlan &plan) {
+  CoarseArgs<T> ca = coarse_args<T>(plan);
+  ca.invd = (const T *)op->d_inv_diag.ptr;
+  ca.cmask = op->L().d_cmask.ptr;
+  return ca;
+}
+
 template <int P, int Q, typename T, int VAR>
 lsmf_status run_coarse_cheb(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta, double delta,
                             int degree) {
   auto a = make_args<T>(op);
   const TabT<P, Q, T> tab = make_tabt<P, Q, T>(op->mesh->basis);
-  CoarseArgs<T> ca = coarse_args<T>(plan);
+  CoarseArgs<T> ca = coarse_level_args<T>(op, plan);
   ca.b = (const T *)b;
   ca.x = (T *)x;
-  ca.invd = (const T *)op->d_inv_diag.ptr;
-  ca.cmask = op->L().d_cmask.ptr;
   ca.theta = theta;
   ca.delta = delta;
   ca.degree = degree;
-  // every packet of the exchange starts without a tag
-  if (plan.xbuf.n) LSMF_CUDA(cudaMemsetAsync(plan.xbuf.ptr, 0, plan.xbuf.n * sizeof(ulonglong2), op->stream));
   auto k = plan.max_nodes <= 2 * COARSE_THREADS ? coarse_cheb_kernel<P, Q, T, VAR, 2> : coarse_cheb_kernel<P, Q, T, VAR, 4>;
-  LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
-  void *args[] = {(void *)&a, (void *)&tab, (void *)&ca};
-  LSMF_CUDA(cudaLaunchCooperativeKernel((const void *)k, dim3(plan.n_cta), dim3(COARSE_THREADS), args, plan.smem, op->stream));
-  return LSMF_OK;
+  return launch_coarse(op, plan, k, a, tab, ca);
+}
+
+template <int P, int Q, typename T, int VAR>
+lsmf_status run_coarse_eig(const lsmf_op *op, const CoarsePlan &plan, const CoarseEig &e) {
+  auto a = make_args<T>(op);
+  const TabT<P, Q, T> tab = make_tabt<P, Q, T>(op->mesh->basis);
+  CoarseArgs<T> ca = coarse_level_args<T>(op, plan);
+  CoarseEigArgs ea;
+  ea.mean = e.mean;
+  ea.tol_abs = e.tol_abs;
+  ea.tol_rel = e.tol_rel;
+  ea.max_it = e.max_it;
+  ea.alpha = e.alpha;
+  ea.beta = e.beta;
+  ea.res2 = e.res2;
+  ea.its = e.its;
+  auto k = plan.max_nodes <= 2 * COARSE_THREADS ? coarse_eig_kernel<P, Q, T, VAR, 2> : coarse_eig_kernel<P, Q, T, VAR, 4>;
+  return launch_coarse(op, plan, k, a, tab, ca, ea);
 }
 
 #define LSMF_DISPATCH_VAR(v, ...)                                                     \
@@ -1384,8 +1413,11 @@ struct DegreeOps {
                           int degree) {
     return LSMF_DISPATCH_VAR(variant_of(op), (run_coarse_cheb<P, Q, T, V_>(op, plan, x, b, theta, delta, degree)));
   }
+  static lsmf_status eig(const lsmf_op *op, const CoarsePlan &plan, const CoarseEig &e) {
+    return LSMF_DISPATCH_VAR(variant_of(op), (run_coarse_eig<P, Q, T, V_>(op, plan, e)));
+  }
   static const OpsTable &table() {
-    static const OpsTable t = {&cache, &apply, &diag, &shape, &cheb};
+    static const OpsTable t = {&cache, &apply, &diag, &shape, &cheb, &eig};
     return t;
   }
 };

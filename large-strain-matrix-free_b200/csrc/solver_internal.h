@@ -85,6 +85,7 @@ lsmf_status launch_apply_inhomogeneous(const lsmf_op *op, void *dst, const void 
 // a usable plan (one cooperative kernel)
 lsmf_status launch_coarse_cheb(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta,
                                double delta, int degree);
+lsmf_status launch_coarse_eig(const lsmf_op *op, const CoarsePlan &plan, const CoarseEig &e);
 
 // Eigenvalues of a symmetric tridiagonal matrix (Sturm bisection).
 double tridiag_eig(const std::vector<double> &d, const std::vector<double> &e, bool want_max);

@@ -90,3 +90,20 @@ def test_run_out_wait_is_reported_and_recovers():
     g.level_option(0, WAIT_TRIES, -1)
     x.zero_()
     assert lsmf.cg_solve(op, x, b, 1e-8 * float(b.norm()), 100, "gmg", g)["converged"]
+
+
+@pytest.mark.parametrize("caching,formulation", VARIANTS)
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_eigenvalue_estimate(caching, formulation, precision):
+    # the estimate's CG as one kernel against the launch-per-iteration form:
+    # the tolerances of the estimates' parity tests (1e-9 / 2e-3), equal degrees
+    gm, g, mu, u, b = _setup(2, (5, 4, 3), 0, caching, formulation, precision)
+    g.setup(u)
+    one = g.level_info(0)
+    g.level_option(0, BASIC, 1)
+    g.setup(u)
+    steps = g.level_info(0)
+    tol = 1e-9 if precision == "fp64" else 2e-3
+    assert np.allclose(one[:2], steps[:2], rtol=tol, atol=0), (one, steps)
+    assert one[2] == steps[2]
+    assert abs(one[5] - steps[5]) <= 0.05 * steps[5]
