@@ -125,7 +125,8 @@ lsmf_status build_coarse_plan(const lsmf_op *op, int sms, size_t smem_limit, Coa
   // exchange slots, consecutive in a part's local order, so that a line of
   // packets has one writer and mostly one reader (slots numbered by node, the
   // writers of a node side by side, cost 1.5 us a step)
-  std::vector<int> count(L.n_nodes, 0), by(part_nodes.size()), node_slot((size_t)L.n_nodes * 8, -1), key(L.n_nodes);
+  std::vector<int> count(L.n_nodes, 0), by(part_nodes.size()), node_slot((size_t)L.n_nodes * 8, -1);
+  std::vector<uint64_t> keys;
   int n_slots = 0;
   for (int p = 0; p < P; ++p) {
     const int n0 = node_off[p], n1 = node_off[p + 1];
@@ -135,14 +136,15 @@ lsmf_status build_coarse_plan(const lsmf_op *op, int sms, size_t smem_limit, Coa
         int &c = count[L.cell_nodes[(size_t)order[s] * nn + a]];
         if (++c > 8) return LSMF_OK;
       }
+    keys.resize(n1 - n0);
     for (int k = n0; k < n1; ++k) {
       const int n = part_nodes[k], m = n_parts[n];
       const int *np = &node_parts[8 * (size_t)n];
       const int other = m == 2 ? (np[0] == p ? np[1] : np[0]) : 0;
-      key[n] = ((8 - m) * 4096 + other) * 16 + (8 - count[n]);
+      keys[k - n0] = (uint64_t)(((8 - m) * 4096 + other) * 16 + (8 - count[n])) << 32 | (uint32_t)n;
     }
-    std::copy(&part_nodes[n0], &part_nodes[n0] + (n1 - n0), &by[n0]);
-    std::sort(&by[n0], &by[n0] + (n1 - n0), [&](int a, int b) { return key[a] != key[b] ? key[a] < key[b] : a < b; });
+    std::sort(keys.begin(), keys.end());
+    for (int k = n0; k < n1; ++k) by[k] = (int)(uint32_t)keys[k - n0];
     for (int k = n0; k < n1; ++k) {
       const int n = by[k];
       if (n_parts[n] < 2) break;
