@@ -34,7 +34,6 @@ std::vector<std::string> split(const std::string &s, char sep) {
 
 // ------------------------------------------------------------ expressions
 // Recursive-descent parser producing a postfix program over a value stack.
-enum Op { PUSH, VAR_X, VAR_Y, VAR_Z, VAR_T, ADD, SUB, MUL, DIV, POW, NEG, FN };
 
 struct Parser {
   const std::string &s;

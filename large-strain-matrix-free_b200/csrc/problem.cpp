@@ -72,58 +72,52 @@ void face_local_nodes(int p, int f, std::vector<int> &out) {
       }
 }
 
-// external (dead) load: sum over Neumann faces of N_a T(x, t) JxW with the
-// face quadrature QGauss<2>(q) (mf_elasticity.h:2859-2892)
-void neumann_load(const lsmf_problem &pb, double t, std::vector<double> &f) {
+// lists of the external (dead) load: sum over Neumann faces of N_a T(x, t) JxW
+// with the face quadrature QGauss<2>(q) (mf_elasticity.h:2859-2892), formed on
+// the device (NeumannLoad)
+lsmf_status build_neumann(lsmf_problem &pb) {
+  NeumannLoad &N = pb.neumann;
   const Level &L = *pb.mesh->levels.back();
-  const Basis &B = pb.mesh->basis;
-  const int p = L.p, q = L.q, n1 = p + 1, ncn = L.ncn();
-  f.assign(L.n_dofs(), 0.0);
-  std::vector<double> v[3], dv[3];
-  for (int d = 0; d < 3; ++d) { v[d].resize(n1); dv[d].resize(n1); }
-  for (size_t k = 0; k < L.bfaces.size(); k += 3) {
-    const int cell = L.bfaces[k], face = L.bfaces[k + 1], id = L.bfaces[k + 2];
-    for (const BCExpr &nm : pb.prm.neumann) {
-      if (nm.id != id) continue;
-      const int nd = face / 2, ta = nd == 0 ? 1 : 0, tb = nd == 2 ? 1 : 2;
-      const int *nodes = &L.cell_nodes[(size_t)cell * ncn];
-      for (int qb = 0; qb < q; ++qb)
-        for (int qa = 0; qa < q; ++qa) {
-          double xi[3];
-          xi[nd] = (face & 1) ? 1.0 : 0.0;
-          xi[ta] = B.qpts[qa];
-          xi[tb] = B.qpts[qb];
-          for (int d = 0; d < 3; ++d) B.eval(xi[d], v[d].data(), dv[d].data());
-          double x[3] = {0, 0, 0}, tA[3] = {0, 0, 0}, tB[3] = {0, 0, 0};
-          std::vector<double> Nv(ncn);
-          for (int c = 0; c <= p; ++c)
-            for (int b = 0; b <= p; ++b)
-              for (int a = 0; a <= p; ++a) {
-                const int ln = (c * n1 + b) * n1 + a;
-                const int li[3] = {a, b, c};
-                const double *X = &L.X[3 * (size_t)nodes[ln]];
-                Nv[ln] = v[0][a] * v[1][b] * v[2][c];
-                double ga = 1, gb = 1;
-                for (int d = 0; d < 3; ++d) {
-                  ga *= d == ta ? dv[d][li[d]] : v[d][li[d]];
-                  gb *= d == tb ? dv[d][li[d]] : v[d][li[d]];
-                }
-                for (int d = 0; d < 3; ++d) {
-                  x[d] += Nv[ln] * X[d];
-                  tA[d] += ga * X[d];
-                  tB[d] += gb * X[d];
-                }
-              }
-          const double cr[3] = {tA[1] * tB[2] - tA[2] * tB[1], tA[2] * tB[0] - tA[0] * tB[2],
-                                tA[0] * tB[1] - tA[1] * tB[0]};
-          const double jxw = std::sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]) * B.qw[qa] * B.qw[qb];
-          double T[3];
-          for (int c = 0; c < 3; ++c) T[c] = nm.expr[c].eval(x[0], x[1], x[2], t);
-          for (int ln = 0; ln < ncn; ++ln)
-            for (int c = 0; c < 3; ++c) f[3 * (size_t)nodes[ln] + c] += Nv[ln] * T[c] * jxw;
-        }
+  const int n1 = L.p + 1, nf = n1 * n1;
+  std::vector<ExprIns> prog;
+  std::vector<int> off(1, 0), faces;
+  for (const BCExpr &nm : pb.prm.neumann)
+    for (int c = 0; c < 3; ++c) {
+      for (const Expr::Ins &i : nm.expr[c].prog) prog.push_back({i.op, i.f, i.v});
+      off.push_back((int)prog.size());
     }
+  for (size_t k = 0; k < L.bfaces.size(); k += 3)
+    for (size_t b = 0; b < pb.prm.neumann.size(); ++b)
+      if (pb.prm.neumann[b].id == L.bfaces[k + 2]) faces.insert(faces.end(), {L.bfaces[k], L.bfaces[k + 1], (int)b});
+  N.n_faces = (int)faces.size() / 3;
+  if (!N.n_faces) return LSMF_OK;
+  // loaded nodes in increasing order, their contributions in face order
+  std::vector<std::pair<int, int>> at;
+  at.reserve((size_t)N.n_faces * nf);
+  for (int f = 0; f < N.n_faces; ++f) {
+    const int cell = faces[3 * f], face = faces[3 * f + 1], nd = face / 2;
+    const int stride[3] = {1, n1, nf}, ta = nd == 0 ? 1 : 0, tb = nd == 2 ? 1 : 2;
+    const int *cn = &L.cell_nodes[(size_t)cell * L.ncn() + ((face & 1) ? L.p : 0) * stride[nd]];
+    for (int l = 0; l < nf; ++l) at.push_back({cn[(l % n1) * stride[ta] + (l / n1) * stride[tb]], f * nf + l});
   }
+  std::sort(at.begin(), at.end());
+  std::vector<int> nodes, node_off, places;
+  for (const auto &e : at) {
+    if (nodes.empty() || nodes.back() != e.first) {
+      nodes.push_back(e.first);
+      node_off.push_back((int)places.size());
+    }
+    places.push_back(e.second);
+  }
+  node_off.push_back((int)places.size());
+  N.n_nodes = (int)nodes.size();
+  LSMF_TRY(N.faces.upload(faces.data(), faces.size()));
+  LSMF_TRY(N.off.upload(off.data(), off.size()));
+  LSMF_TRY(N.prog.upload(prog.data(), prog.size()));
+  LSMF_TRY(N.nodes.upload(nodes.data(), nodes.size()));
+  LSMF_TRY(N.node_off.upload(node_off.data(), node_off.size()));
+  LSMF_TRY(N.places.upload(places.data(), places.size()));
+  return N.results.alloc((size_t)N.n_faces * nf * 3);
 }
 
 // constrained values of the load step (applied as the step increment at the
@@ -255,14 +249,14 @@ struct Timer {
   }
 };
 
-// R = fext - f_int(u) with the constrained entries zeroed: the right-hand
-// side of assemble_system (mf_elasticity.h:2736-2921); fext is the device
-// Neumann load of the step
-lsmf_status residual_async(lsmf_problem *pb, const double *u, const double *fext, double *R) {
+// R = fext(t) - f_int(u) with the constrained entries zeroed: the right-hand
+// side of assemble_system (mf_elasticity.h:2736-2921)
+lsmf_status residual_async(lsmf_problem *pb, const double *u, double t, double *R) {
   const Level &L = *pb->mesh->levels.back();
   const size_t n = (size_t)L.n_dofs();
   cudaStream_t st = pb->stream;
-  LSMF_CUDA(cudaMemcpyAsync(R, fext, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  LSMF_CUDA(cudaMemsetAsync(R, 0, n * sizeof(double), st));
+  LSMF_TRY(neumann_load_async(L, pb->mesh->basis, pb->neumann, t, R, st));
   LSMF_TRY(internal_force_async(L, pb->mesh->basis, u, pb->mu_dev.ptr, pb->prm.nu, pb->prm.formulation, R,
                                 pb->op->scatter, st));
   return set_indexed_async<double>(R, L.d_constrained.ptr, (int)L.constrained.size(), 0.0, st);
@@ -294,14 +288,12 @@ lsmf_status problem_run(lsmf_problem *pb, lsmf_newton_info *info) {
   double *u_n = pb->u_n.ptr, *du = pb->du.ptr, *u_tot = pb->u_tot.ptr, *R = pb->R.ptr, *dx = pb->dx.ptr;
   LSMF_CUDA(cudaMemsetAsync(u_n, 0, n * sizeof(double), st));
   if (info) std::memset(info, 0, sizeof(*info));
-  std::vector<double> fext, g;
+  std::vector<double> g;
   double time = 0.0;
   time += P.dt;  // Time::increment
   int step = 0;
   lsmf_status result = LSMF_OK;
   while (time <= P.end_time) {
-    neumann_load(*pb, time, fext);
-    LSMF_TRY(pb->fext.upload(fext.data(), n));
     const bool inhom = dirichlet_values(*pb, time, g);
     if (inhom) LSMF_TRY(pb->gvals.upload(g.data(), n));
     LSMF_CUDA(cudaMemsetAsync(du, 0, n * sizeof(double), st));
@@ -313,7 +305,7 @@ lsmf_status problem_run(lsmf_problem *pb, lsmf_newton_info *info) {
       Timer tr(st);
       LSMF_CUDA(cudaMemcpyAsync(u_tot, u_n, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
       LSMF_TRY(axpy_async<double>(u_tot, 1.0, du, n, st));
-      LSMF_TRY(residual_async(pb, u_tot, pb->fext.ptr, R));
+      LSMF_TRY(residual_async(pb, u_tot, time, R));
       bool cached = false;
       if (it == 0 && inhom) {
         // rhs -= K g over the constrained columns (the inhomogeneity that
@@ -521,12 +513,13 @@ lsmf_status lsmf_problem_create(const char *text, lsmf_problem **out) {
   }
   const Level &L = *pb->mesh->levels.back();
   const size_t n = (size_t)L.n_dofs();
-  for (auto *b : {&pb->u_n, &pb->du, &pb->u_tot, &pb->R, &pb->dx, &pb->fext, &pb->gvals, &pb->tmp, &pb->lam})
+  for (auto *b : {&pb->u_n, &pb->du, &pb->u_tot, &pb->R, &pb->dx, &pb->gvals, &pb->tmp, &pb->lam})
     if ((s = b->alloc(n)) != LSMF_OK) { delete pb; return s; }
   if ((s = pb->op->sc.alloc(SC_N)) != LSMF_OK || (s = pb->op->partial.alloc(reduce_blocks())) != LSMF_OK) {
     delete pb;
     return s;
   }
+  if ((s = build_neumann(*pb)) != LSMF_OK) { delete pb; return s; }
   if (!P.output_points.empty()) {
     double pt[3] = {P.output_points[0][0], P.output_points[0][1], P.output_points[0][2]};
     pb->have_point = locate_point(L, pb->mesh->basis, pt, pb->point_nodes, pb->point_w);
@@ -601,11 +594,7 @@ lsmf_status lsmf_problem_run(lsmf_problem *pb, lsmf_newton_info *info) {
 
 lsmf_status lsmf_residual(lsmf_problem *pb, const double *d_u, double t, double *d_R, double *norm) {
   if (!pb || !d_u || !d_R) { set_error("null argument"); return LSMF_ERR_INVALID_ARG; }
-  const size_t n = (size_t)pb->mesh->levels.back()->n_dofs();
-  std::vector<double> fext;
-  neumann_load(*pb, t, fext);
-  LSMF_TRY(pb->fext.upload(fext.data(), n));
-  LSMF_TRY(residual_async(pb, d_u, pb->fext.ptr, d_R));
+  LSMF_TRY(residual_async(pb, d_u, t, d_R));
   const double r = norm_of(pb, d_R);
   if (!(r == r)) { set_error("residual norm is not a number"); return LSMF_ERR_CUDA; }
   if (norm) *norm = r;

@@ -10,6 +10,9 @@
 
 namespace lsmf {
 
+// Instructions of a parsed expression: a postfix program over a value stack.
+enum ExprOp { PUSH, VAR_X, VAR_Y, VAR_Z, VAR_T, ADD, SUB, MUL, DIV, POW, NEG, FN };
+
 // A parsed function of (x, y, z, t) (the FunctionParser expressions of the
 // "Boundary conditions" subsection, mf_elasticity.h:215-248).
 struct Expr {
@@ -75,11 +78,12 @@ lsmf_status parse_prm(const std::string &text, ProblemParams &P);
 
 struct lsmf_problem {
   lsmf::ProblemParams prm;
+  lsmf::NeumannLoad neumann;
   lsmf_mesh *mesh = nullptr;
   lsmf_op *op = nullptr;       // FP64 fine operator
   lsmf_gmg *gmg = nullptr;     // level hierarchy (gmg preconditioner)
   std::vector<double> mu_fine;
-  lsmf::DevBuf<double> u_n, du, u_tot, R, dx, fext, gvals, tmp, lam, grad, target, mu_dev;
+  lsmf::DevBuf<double> u_n, du, u_tot, R, dx, gvals, tmp, lam, grad, target, mu_dev;
   std::vector<uint8_t> obj_mask_dofs;
   bool inhom = false;
   // output point: fine cell node ids + shape weights

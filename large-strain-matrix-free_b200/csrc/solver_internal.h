@@ -77,6 +77,23 @@ lsmf_status internal_force_async(const Level &L, const Basis &B, const double *u
                                  int formulation, double *R, int scatter, cudaStream_t st);
 lsmf_status adjoint_cell_grad_async(const Level &L, const Basis &B, const double *u, const double *mu, double nu,
                                     int formulation, const double *lam, double *grad, cudaStream_t st);
+// Surface load on the device: sum over Neumann faces of N_a T(x, t) JxW.
+// Faces are (cell, face, condition); the traction of condition k is the three
+// programs prog[off[3k + c] .. off[3k + c + 1]); the loaded nodes and, per
+// node, the places of its contributions in the faces' results, in face order
+// (a fixed order of summation).
+struct ExprIns {
+  int op, f;
+  double v;
+};
+struct NeumannLoad {
+  int n_faces = 0, n_nodes = 0;
+  DevBuf<int> faces, off, nodes, node_off, places;
+  DevBuf<ExprIns> prog;
+  DevBuf<double> results;  // [face][(p+1)^2][3]
+};
+// R (zeroed by the caller) = the load at time t on the loaded nodes
+lsmf_status neumann_load_async(const Level &L, const Basis &B, const NeumannLoad &N, double t, double *R, cudaStream_t st);
 // apply with an un-zeroed gather of constrained entries (K g over the
 // constrained columns, the inhomogeneity term of the rhs)
 lsmf_status launch_apply_inhomogeneous(const lsmf_op *op, void *dst, const void *g);
