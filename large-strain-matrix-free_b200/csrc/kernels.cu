@@ -27,6 +27,30 @@ __global__ void constrained_add_kernel(T *dst, const T *src, const int *idx, int
     dst[k] += src[k];
   }
 }
+// dst = src on the constrained dofs and zero elsewhere, for the dofs first ..
+// last - 1: the zeroing and the identity rows of a vmult in one launch (the
+// cell loop adds nothing to constrained dofs).  Every thread writes aligned
+// 16-byte groups of dst; the ends of the range are written value by value.
+// It lets a cell loop launched as its programmatic dependent start at once.
+template <typename T>
+__global__ void identity_rows_kernel(T *__restrict__ dst, const T *__restrict__ src, const uint8_t *__restrict__ cmask,
+                                     size_t first, size_t last) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  constexpr int W = 16 / sizeof(T);
+  const size_t shift = ((size_t)dst / sizeof(T)) % W;  // dst + i is aligned where (i + shift) % W == 0
+  const size_t g0 = (first + shift) / W, g1 = (last + shift + W - 1) / W;
+  for (size_t g = g0 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; g < g1; g += (size_t)gridDim.x * blockDim.x) {
+    const size_t a = g * W < shift ? 0 : g * W - shift, b = g * W + W - shift;
+    if (g * W >= first + shift && b <= last) {
+      alignas(16) T v[W];
+#pragma unroll
+      for (int k = 0; k < W; ++k) v[k] = __ldg(cmask + a + k) ? src[a + k] : T(0);
+      *(float4 *)(dst + a) = *(const float4 *)v;
+    } else {
+      for (size_t i = a > first ? a : first; i < (b < last ? b : last); ++i) dst[i] = cmask[i] ? src[i] : T(0);
+    }
+  }
+}
 template <typename T>
 __global__ void constrained_set_kernel(T *dst, const int *idx, int n, T val) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[idx[i]] = val;
@@ -58,6 +82,19 @@ const OpsTable *table_of(const lsmf_op *op) {
   const OpsTable *t = L.q == L.p + 1 ? ops_for(L.p, op->precision == LSMF_FP32) : nullptr;
   if (!t) set_error("unsupported (degree, n_q_points_1d): only q = p + 1, p = 1..4");
   return t;
+}
+
+lsmf_status identity_rows(const lsmf_op *op, void *dst, const void *src, size_t first, size_t last, cudaStream_t st) {
+  if (last <= first) return LSMF_OK;
+  const size_t per = 16 / op->elem(), groups = (last - first + per - 1) / per + 1;
+  const int g = (int)std::min<size_t>((groups + 255) / 256, (size_t)8 * num_sms());
+  const uint8_t *cm = op->L().d_cmask.ptr;
+  if (op->precision == LSMF_FP64)
+    identity_rows_kernel<double><<<g, 256, 0, st>>>((double *)dst, (const double *)src, cm, first, last);
+  else
+    identity_rows_kernel<float><<<g, 256, 0, st>>>((float *)dst, (const float *)src, cm, first, last);
+  LSMF_CUDA(cudaGetLastError());
+  return LSMF_OK;
 }
 
 // node-sum scatter: dst (+)= the sum over the node's cells, in increasing
@@ -292,23 +329,23 @@ lsmf_status effective_chunks(const lsmf_op *op, int *k) {
 
 
 // The vmult over the plan's chunks, forked from and joined back into the
-// operator's stream: chunk c zeroes its node range of dst (zero) and adds
-// the identity rows of the constrained dofs in it (rows), then runs its
+// operator's stream: chunk c zeroes its node range of dst (zero) and sets, or
+// without it adds, the identity rows of the constrained dofs there, then runs its
 // cells once chunk c + 1 has zeroed its range (its cells add into that
 // range's first node layer).  The scatter skips constrained components, so
 // the identity rows are never touched by another chunk.
 static lsmf_status apply_chunked(const lsmf_op *op, const OpsTable *t, const ChunkPlan &cp, void *dst,
-                                 const void *src, unsigned mask, bool zero, bool rows) {
+                                 const void *src, unsigned mask, bool zero) {
   const Level &L = op->L();
-  const size_t e = op->elem();
   const int g_max = 4 * num_sms();
   LSMF_CUDA(cudaEventRecord(cp.fork, op->stream));
   for (int c = 0; c < cp.k; ++c) {
     cudaStream_t st = cp.stream[c];
     LSMF_CUDA(cudaStreamWaitEvent(st, cp.fork, 0));
     const size_t d0 = 3 * (size_t)cp.node0[c], d1 = 3 * (size_t)cp.node0[c + 1];
-    if (zero && d1 > d0) LSMF_CUDA(cudaMemsetAsync((char *)dst + d0 * e, 0, (d1 - d0) * e, st));
-    if (rows) {
+    if (zero) {
+      LSMF_TRY(identity_rows(op, dst, src, d0, d1, st));
+    } else {
       // L.constrained is in increasing dof order
       const int a0 = (int)(std::lower_bound(L.constrained.begin(), L.constrained.end(), (int)d0) - L.constrained.begin());
       const int a1 = (int)(std::lower_bound(L.constrained.begin(), L.constrained.end(), (int)d1) - L.constrained.begin());
@@ -348,10 +385,17 @@ lsmf_status launch_apply(const lsmf_op *op, void *dst, const void *src, unsigned
     if (chunkable(op, mask)) {
       const ChunkPlan *cp = nullptr;
       LSMF_TRY(chunk_plan(op, chunk_count(op), &cp));
-      if (cp) return apply_chunked(op, t, *cp, dst, src, mask, !add && (mask & LSMF_MASK_ZERO), true);
+      if (cp) return apply_chunked(op, t, *cp, dst, src, mask, !add && (mask & LSMF_MASK_ZERO));
     }
-    if (!add && (mask & LSMF_MASK_ZERO)) LSMF_CUDA(cudaMemsetAsync(dst, 0, n * op->elem(), op->stream));
-    LSMF_TRY(for_cell_ranges(L, op->scatter, [&](CellRange r) { return t->apply(op, dst, src, mask, r); }));
+    const bool zero = !add && (mask & LSMF_MASK_ZERO), rows = mask & LSMF_MASK_RW;
+    if (zero && rows) LSMF_TRY(identity_rows(op, dst, src, 0, n, op->stream));
+    else if (zero) LSMF_CUDA(cudaMemsetAsync(dst, 0, n * op->elem(), op->stream));
+    LSMF_TRY(for_cell_ranges(L, op->scatter, [&](CellRange r) {
+      // only the scatter of the first launch has to wait for the rows
+      r.dependent = zero && rows && !r.cells;
+      return t->apply(op, dst, src, mask, r);
+    }));
+    if (zero && rows) return LSMF_OK;
   }
   // constrained rows: dst += src (mf_nh_operator.h:702-705)
   const int nc = (int)L.constrained.size();

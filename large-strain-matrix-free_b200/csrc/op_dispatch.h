@@ -31,6 +31,10 @@ struct CellRange {
   // one chunk of a cell loop split over concurrent streams
   int first = 0, count = -1;
   cudaStream_t stream = nullptr;
+  // launched right after the kernel that writes dst's identity rows, as its
+  // programmatic dependent: the production kernel waits for it only before
+  // its first scatter
+  bool dependent = false;
 };
 
 struct OpsTable {

@@ -767,6 +767,9 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
     }
     T out[3][N1];
     S::integrate(tab, G, slab, lp, out);
+    // dst's rows are written by the kernel before (no effect in a launch that
+    // is not its programmatic dependent)
+    if (w == gw) asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       if (!ok[h]) continue;
@@ -1196,7 +1199,7 @@ lsmf_status run_cache(lsmf_op *op) {
 
 // launch the production cell loop
 template <int P, int Q, typename T, int VAR>
-lsmf_status launch_line(const lsmf_op *op, KArgs<typename Num<T>::S> a, bool peer, int ring, int max_warps,
+lsmf_status launch_line(const lsmf_op *op, KArgs<typename Num<T>::S> a, bool peer, bool dependent, int ring, int max_warps,
                         cudaStream_t stream) {
   using E = typename Num<T>::S;
   const TabT<P, Q, T> tab = make_tabt<P, Q, T>(op->mesh->basis);
@@ -1213,9 +1216,22 @@ lsmf_status launch_line(const lsmf_op *op, KArgs<typename Num<T>::S> a, bool pee
   const size_t smem = w * wbytes(ring);
   const int units = col ? UnitMap<P, Q, T, true>::units(a.n_cells) : UnitMap<P, Q, T, false>::units(a.n_cells);
   auto go = [&](auto k) -> lsmf_status {
-    LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int g = grid_for(k, 32 * w, smem, (units + w - 1) / w);
-    k<<<g, 32 * w, smem, stream>>>(a, tab);
+    // small launches are bound by the host: shared memory up to 48 KB needs
+    // no attribute, and a grid within the SMs no occupancy query
+    if (smem > 48 * 1024) LSMF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = (units + w - 1) / w;
+    const int g = blocks <= num_sms() ? blocks : grid_for(k, 32 * w, smem, blocks);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(g);
+    cfg.blockDim = dim3(32 * w);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = dependent ? 1 : 0;
+    LSMF_CUDA(cudaLaunchKernelEx(&cfg, k, a, tab));
     return LSMF_OK;
   };
   if (col) return go(apply_line_kernel<P, Q, T, VAR, false, SC_COLOUR>);
@@ -1270,7 +1286,7 @@ lsmf_status run_apply(const lsmf_op *op, T *dst, const T *src, unsigned mask, Ce
     const int max_warps = op->max_warps > 0 ? op->max_warps : warps_auto;
     // FP32: two cells per lane, in packed registers
     using N = typename std::conditional<sizeof(T) == 8, double, f2>::type;
-    LSMF_TRY((launch_line<P, Q, N, VAR>(op, a, peer, ring, max_warps, stream)));
+    LSMF_TRY((launch_line<P, Q, N, VAR>(op, a, peer, range.dependent, ring, max_warps, stream)));
   } else {
     const Tab<P, Q> tab = make_tab<P, Q>(op->mesh->basis);
     using S = SF<P, Q, T>;
