@@ -145,6 +145,20 @@ struct LanePos {
   }
 };
 
+// Jacobian of an affine cell from four of its corners (cn: the cell's nodes)
+template <int P>
+__device__ __forceinline__ void affine_jacobian(const int *__restrict__ cn, const double *__restrict__ X, double J[3][3]) {
+  constexpr int N1 = P + 1;
+  const double *x0 = X + 3 * (size_t)(__ldg(cn) & NODE_MASK);
+  const int corner[3] = {P, P * N1, P * N1 * N1};
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const double *xe = X + 3 * (size_t)(__ldg(cn + corner[e]) & NODE_MASK);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) J[d][e] = __ldg(xe + d) - __ldg(x0 + d);
+  }
+}
+
 // Sum factorisation with whole lines per lane, Q^2 lanes per cell.
 //   eval:      lane (j, i) holds the nodes k = 0..P of its z line; the z
 //              sweep runs in registers, its two fields (value, derivative)
