@@ -199,8 +199,8 @@ struct UnitMap {
 // access of the warp.  FP32 tables hold two cells per lane slot; their two
 // halves are worked on one after the other.  AFFINE (box meshes): the
 // reference Jacobian is one per cell, from four corners, instead of an
-// evaluation of X at every point, which takes a third of the gathers and
-// sweeps and 26-45 registers off.  tensor4 FP64 at 60^3 Q2: 414 -> 329 us, with the
+// evaluation of X at every point, which takes half of the gathers and
+// sweeps and 12-42 registers off.  tensor4 FP64 at 60^3 Q2: 414 -> 329 us, with the
 // 1.68 GB of the table alone 257 us at copy bandwidth.
 template <int P, int Q, typename T, int VAR, bool AFFINE>
 __global__ void __launch_bounds__(128) cache_kernel(KArgs<T> a, TabT<P, Q, double> tabt, Tab<P, Q> tab) {
@@ -756,6 +756,8 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
             if (w + ((s + k) / Q) * nw < n_units) mbar_wait_bounded(&bar[place], parity);
             if (++place == D) { place = 0; parity ^= 1; }
           }
+          // the launch is not to end before the one whose dependent it is
+          asm volatile("griddepcontrol.wait;" ::: "memory");
           return;
         }
         point(s, (const T *)(wbase + place * slice_bytes) + lp.r * L);
