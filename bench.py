@@ -4,7 +4,7 @@ Workload (one "step"): one tangent vmult, tensor4 caching, FP64, on the
 64^3-cell Q2 unit cube (6,440,067 DoFs): per-cell mu drawn from {1, 10} by
 seed, nu = 0.3, bottom face clamped, a seeded smooth displacement field
 bounded by 0.01 (det F > 0.5 checked) and a seeded source vector
-uniform in [-1, 1].  The cache tables (2.9 GB) are larger than L2, so no
+uniform in [-1, 1].  The cache tables (2.0 GB) are larger than L2, so no
 L2 flush is needed between timed steps.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl lsmf|reference]
@@ -37,19 +37,20 @@ METRIC = "Tangent vmult GDoF/s & Newton-step time, FP32-GMG vs FP64, same 1e-8 r
 
 def alg_bytes(variant, S, n_nodes, n_qp, n_cells):
     """Algorithmic bytes per vmult (values counted once, index maps excluded):
-    scalar S(9N + 11Q + 10C), tensor2 S(6N + 17Q), tensor4 S(6N + 51Q);
+    scalar S(9N + 11Q + 10C), tensor2 S(6N + 17Q), tensor4 S(6N + 36Q);
     the referential variants: scalar_referential S(6N + 14Q) (c, the point
-    displacement, metric), tensor4_ns S(6N + 90Q) (dP/dF, inverse Jacobian).
+    displacement, metric), tensor4_ns S(6N + 54Q) (dP/dF, inverse Jacobian).
     tensor4, tensor2 and tensor4_ns cache their coefficients times JxW, so
-    their records carry no JxW value."""
+    their records carry no JxW value; C and dP/dF are symmetric matrices, of
+    which the records hold the upper triangle (21 of 36, 45 of 81 values)."""
     if variant == "tensor4":
-        return S * (6 * n_nodes + 51 * n_qp)
+        return S * (6 * n_nodes + 36 * n_qp)
     if variant == "tensor2":
         return S * (6 * n_nodes + 17 * n_qp)
     if variant == "scalar_referential":
         return S * (6 * n_nodes + 14 * n_qp)
     if variant == "tensor4_ns":
-        return S * (6 * n_nodes + 90 * n_qp)
+        return S * (6 * n_nodes + 54 * n_qp)
     return S * (9 * n_nodes + 11 * n_qp + 10 * n_cells)
 
 
@@ -691,9 +692,9 @@ def profile_setup(cells=15, refinements=2, precision="fp32"):
 
 
 def profile_pairs(sizes=(48, 15)):
-    """One FP32 vmult per (cells^3 Q2 cube, tensor4 / tensor2, one cell per
-    warp / cell pairs), plain record loads, no warm-up: the launches that an
-    ncu capture of apply_fast_kernel and apply_pair_kernel compares."""
+    """One FP32 vmult per (cells^3 Q2 cube, tensor4 / tensor2), plain record
+    loads, no warm-up: the launches of an ncu capture of apply_line_kernel,
+    whose FP32 form works two cells per lane in packed registers."""
     import torch
     import lsmf
     for n in sizes:
@@ -709,10 +710,8 @@ def profile_pairs(sizes=(48, 15)):
             op.set_material(mu, NU)
             op.cache(u)
             op.set_pipeline(0)
-            for pairs in (0, 1):
-                op.set_cell_pairs(pairs)
-                dst = torch.empty_like(src)
-                op.vmult(dst, src)
+            dst = torch.empty_like(src)
+            op.vmult(dst, src)
             torch.cuda.synchronize()
             del op
     print(json.dumps({"profile_pairs": "done", "sizes": list(sizes)}), flush=True)
@@ -930,7 +929,7 @@ def run_lsmf(args):
     roofline = {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": traffic,
                 "peak_kind": peak_kind, "alg_bytes_per_launch": alg,
-                "kernel": "apply_fast_kernel<2,3,double,tensor4,1 stage>",
+                "kernel": "apply_line_kernel<2,3,double,tensor4>",
                 "chunks": chunks,
                 "timed": "the cell loop of one vmult_add (its %d concurrent chunks forked from and joined back into "
                          "the timing stream) plus the identity rows, CUDA events on that stream" % chunks}
@@ -942,7 +941,7 @@ def run_lsmf(args):
             stages[variant] = stage_split(mesh, mu, u64, src64, variant)
 
     # the large single-GPU configurations: tensor4 vmults at 48^3 Q4 and
-    # 128^3 Q2 (24.4 GB of FP64 records)
+    # 128^3 Q2 (16.3 GB of FP64 records)
     large = {}
     dist_parts = None
     if not args.no_variants and not args.no_large:
@@ -983,11 +982,11 @@ def run_lsmf(args):
                 "config": {"workload": "tangent vmult, tensor4 caching, FP64, %d^3-cell Q2 unit cube" % args.cells,
                            "n_dofs": n_dofs, "n_cells": n_cells, "degree": DEGREE,
                            "parallelism": "replicas" if world > 1 else "single GPU",
-                           "l2": "inputs larger than L2 (2.9 GB cache tables), no flush"},
+                           "l2": "inputs larger than L2 (2.0 GB cache tables), no flush"},
                 "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
-                # per vmult: one apply launch per chunk and one identity-row
-                # launch (the clamped bottom face lies in the first chunk)
-                "gpu_launches": (chunks + 1) * args.steps, "clocks": clocks, "variants": variants,
+                # per vmult and chunk: the zeroing with the identity rows, and
+                # the cell loop
+                "gpu_launches": 2 * chunks * args.steps, "clocks": clocks, "variants": variants,
                 "stage_split_fp64": stages, "large_vmults": large, "dist_vmult_one_gpu": dist_parts,
                 "newton_step": newton, "newton_load_steps": load_steps, "adjoint": adjoint}
         print(json.dumps(line), flush=True)
@@ -1019,7 +1018,7 @@ def main():
     ap.add_argument("--profile-setup", action="store_true",
                     help="only one FP32 multigrid set-up of the 15^3 -> 60^3 hierarchy between cudaProfilerStart / Stop")
     ap.add_argument("--profile-pairs", action="store_true",
-                    help="only one FP32 vmult per (48^3 / 15^3, tensor4 / tensor2, one cell / cell pairs) for ncu")
+                    help="only one FP32 vmult per (48^3 / 15^3, tensor4 / tensor2) for ncu")
     ap.add_argument("--c5", action="store_true",
                     help="only the large configurations (128^3 Q2, 48^3 Q4 vmults; 128^3 inclusion Newton step)")
     args = ap.parse_args()

@@ -143,7 +143,9 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   variants of degree 2 and more.  The depth is reduced when the ring would
  *   not fit in shared memory; cell lists (colour8) use plain loads.
  * LSMF_OPT_BASIC_KERNEL: 1 = the basic vmult kernel (per-warp shared-memory
- *   sweeps, plain loads); the stage mask of vmult always uses it.
+ *   sweeps, plain loads); the stage mask of vmult always uses it.  On the
+ *   coarsest level of a GMG object it also selects the coarse solver that
+ *   launches every Chebyshev step by itself.
  * LSMF_OPT_MAX_WARPS: cap on warps per block of the vmult kernel (1..8, the
  *   kernel uses at most 4; 0 = default: 4 at degree 4, 1 for tensor4_ns of
  *   degree 1 and 2, 2 otherwise).
@@ -151,7 +153,9 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   record (mbarrier try_wait calls; -1 = default 2^22, seconds).  A wait
  *   that runs out sets the operator's device error word, lets every copy
  *   the warp still has in flight land (default bound) and ends the warp;
- *   0 makes every wait run out at once (for tests of that path).
+ *   0 makes every wait run out at once (for tests of that path).  On the
+ *   coarsest level of a GMG object it also bounds the waits of the coarse
+ *   solver's kernels for the other blocks' node sums (polls).
  * LSMF_OPT_SCATTER: 0 (default) = the cell loop adds its contributions
  *   with atomics (summation order varies run to run); 1 = colour8: the
  *   cells are processed in the 8 parity colours of the structured lattice,
@@ -184,8 +188,8 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   creates start at 1 (measured faster inside the Newton solve).  The
  *   chunks' streams and events are created by lsmf_operator_cache (and by
  *   this option on a cached operator), not by the vmult.
- * A bounded device wait that runs out in the pipelined kernel is reported
- * as LSMF_ERR_TIMEOUT by lsmf_operator_sync, lsmf_cg_solve and the GMG
+ * A bounded device wait that runs out in the pipelined or the coarse-level
+ * kernels is reported as LSMF_ERR_TIMEOUT by lsmf_operator_sync, lsmf_cg_solve and the GMG
  * set-up (the next synchronising call on the operator). */
 enum { LSMF_OPT_BULK_PIPELINE = 1, LSMF_OPT_BASIC_KERNEL = 2, LSMF_OPT_MAX_WARPS = 3, LSMF_OPT_WAIT_TRIES = 4,
        LSMF_OPT_SCATTER = 5, LSMF_OPT_RECORD_PREFETCH = 6, LSMF_OPT_CELL_PAIRS = 7, LSMF_OPT_CHUNKS = 8 };
