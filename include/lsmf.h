@@ -141,7 +141,7 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   plain coalesced loads; -1 (default) = measured choice: 2 slices, 3 for
  *   tensor2 and scalar_referential of degree 4, plain loads for the scalar
  *   variants of degree 2 and more.  The depth is reduced when the ring would
- *   not fit in shared memory; cell lists (colour8) use plain loads.
+ *   not fit in shared memory.
  * LSMF_OPT_BASIC_KERNEL: 1 = the basic vmult kernel (per-warp shared-memory
  *   sweeps, plain loads); the stage mask of vmult always uses it.  On the
  *   coarsest level of a GMG object it also selects the coarse solver that
@@ -160,8 +160,10 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   with atomics (summation order varies run to run); 1 = colour8: the
  *   cells are processed in the 8 parity colours of the structured lattice,
  *   one launch per colour, so that no two cells of a launch share a node
- *   and the sums are formed in a fixed order without atomics
- *   (bit-reproducible vmult, for parity and debugging); 2 = nodesum: one
+ *   and the sums are formed in a fixed order without atomics; the
+ *   production vmult kernel takes whole batches of cells in groups that
+ *   share no node, one launch per group, and adds the cells of a batch one
+ *   after the other (bit-reproducible vmult, for parity and debugging); 2 = nodesum: one
  *   full cell loop stores every cell's results to a per-cell buffer
  *   (n_cells x 3 (p+1)^3 values, allocated when the mode is selected) and
  *   a node kernel adds each node's cell contributions in increasing cell

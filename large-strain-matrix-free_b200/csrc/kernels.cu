@@ -185,6 +185,59 @@ lsmf_status for_cell_ranges(const Level &L, int scatter, F &&f) {
   return f(CellRange{});
 }
 
+// The cell ranges of a vmult cell loop.  The production kernel of a
+// deterministic scatter takes whole batches of cells, in groups that share no
+// node, so that its records are read as contiguous slices; the basic kernel
+// takes the cells of the lattice colours.
+template <typename F>
+static lsmf_status for_apply_ranges(const lsmf_op *op, unsigned mask, F &&f) {
+  const unsigned all = LSMF_MASK_RW | LSMF_MASK_SF | LSMF_MASK_QD;
+  const bool production = !op->basic && (mask & all) == all && !(mask & MASK_INHOM_BIT);
+  if (op->scatter == LSMF_SCATTER_ATOMIC || !production) return for_cell_ranges(op->L(), op->scatter, f);
+  const Level::BatchGroups &g = op->L().batch_groups[op->precision == LSMF_FP32];
+  for (size_t c = 0; c + 1 < g.off.size(); ++c) {
+    CellRange r;
+    r.cells = g.list.ptr + g.off[c];
+    r.n_list = g.off[c + 1] - g.off[c];
+    r.plain = r.batches = true;
+    r.dependent = c > 0;
+    LSMF_TRY(f(r));
+  }
+  return LSMF_OK;
+}
+
+// Groups of the level's batches: each batch, in order, joins the first group
+// none of whose batches has one of its nodes (a bit per group and node, 64
+// groups at a time; 8 to 12 groups on the meshes in use).
+static lsmf_status build_batch_groups(Level &L, int B, Level::BatchGroups &g) {
+  const int nb = (L.n_cells + B - 1) / B, ncn = L.ncn();
+  std::vector<std::vector<uint64_t>> used;
+  std::vector<int> group(nb);
+  int n_groups = 0;
+  for (int b = 0; b < nb; ++b) {
+    const int *n0 = &L.cell_nodes[(size_t)b * B * ncn], *n1 = n0 + (size_t)std::min(B, L.n_cells - b * B) * ncn;
+    for (size_t l = 0;; ++l) {
+      if (l == used.size()) used.emplace_back(L.n_nodes, 0);
+      uint64_t taken = 0;
+      for (const int *n = n0; n < n1; ++n) taken |= used[l][*n];
+      if (taken == ~0ull) continue;
+      const int bit = __builtin_ctzll(~taken);
+      for (const int *n = n0; n < n1; ++n) used[l][*n] |= 1ull << bit;
+      group[b] = 64 * (int)l + bit;
+      break;
+    }
+    n_groups = std::max(n_groups, group[b] + 1);
+  }
+  std::vector<int> off(n_groups + 1, 0), list(nb);
+  for (int b = 0; b < nb; ++b) ++off[group[b] + 1];
+  for (int c = 0; c < n_groups; ++c) off[c + 1] += off[c];
+  std::vector<int> pos(off.begin(), off.end() - 1);
+  for (int b = 0; b < nb; ++b) list[pos[group[b]]++] = b;
+  LSMF_TRY(g.list.upload(list.data(), list.size()));
+  g.off = off;
+  return LSMF_OK;
+}
+
 // the node-sum path applies: the operator asks for it and the launch is the
 // full production cell loop
 static bool node_sum_path(const lsmf_op *op, unsigned mask) {
@@ -218,6 +271,10 @@ lsmf_status set_scatter_mode(lsmf_op *op, int mode) {
   if (mode != LSMF_SCATTER_ATOMIC && mode != LSMF_SCATTER_COLOUR8 && mode != LSMF_SCATTER_NODESUM) {
     set_error("scatter must be 0 (atomic), 1 (colour8) or 2 (nodesum)");
     return LSMF_ERR_INVALID_ARG;
+  }
+  if (mode != LSMF_SCATTER_ATOMIC) {
+    Level::BatchGroups &g = op->L().batch_groups[op->precision == LSMF_FP32];
+    if (g.off.empty()) LSMF_TRY(build_batch_groups(op->L(), cells_per_batch(op->L().p, op->precision), g));
   }
   if (mode == LSMF_SCATTER_NODESUM) {
     Level &L = op->L();
@@ -390,9 +447,11 @@ lsmf_status launch_apply(const lsmf_op *op, void *dst, const void *src, unsigned
     const bool zero = !add && (mask & LSMF_MASK_ZERO), rows = mask & LSMF_MASK_RW;
     if (zero && rows) LSMF_TRY(identity_rows(op, dst, src, 0, n, op->stream));
     else if (zero) LSMF_CUDA(cudaMemsetAsync(dst, 0, n * op->elem(), op->stream));
-    LSMF_TRY(for_cell_ranges(L, op->scatter, [&](CellRange r) {
-      // only the scatter of the first launch has to wait for the rows
-      r.dependent = zero && rows && !r.cells;
+    LSMF_TRY(for_apply_ranges(op, mask, [&](CellRange r) {
+      // the scatter of the first launch has to wait for the rows, that of
+      // every further group of batches for the group before (small levels
+      // are bound by the launches: 16^3 Q2 has 12 groups)
+      r.dependent = r.cells ? r.dependent : zero && rows;
       return t->apply(op, dst, src, mask, r);
     }));
     if (zero && rows) return LSMF_OK;
@@ -457,7 +516,7 @@ lsmf_status launch_apply_cells(const lsmf_op *op, void *dst, const void *src) {
       return LSMF_OK;
     }
   }
-  return for_cell_ranges(op->L(), op->scatter, [&](CellRange r) { return t->apply(op, dst, src, mask, r); });
+  return for_apply_ranges(op, mask, [&](CellRange r) { return t->apply(op, dst, src, mask, r); });
 }
 
 lsmf_status launch_coarse_cheb(const lsmf_op *op, const CoarsePlan &plan, void *x, const void *b, double theta,

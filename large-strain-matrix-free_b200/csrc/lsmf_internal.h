@@ -123,6 +123,14 @@ struct Level {
   std::vector<int> colour_cells;
   int colour_off[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   DevBuf<int> d_colour_cells;
+  // for the production vmult kernel of a deterministic scatter (built when
+  // one is selected): batches of consecutive cells, the cells a warp works on
+  // at a time, in groups whose batches share no node; [0] FP64, [1] FP32
+  // batches.  Group c is list[off[c] .. off[c+1])
+  struct BatchGroups {
+    std::vector<int> off;
+    DevBuf<int> list;
+  } batch_groups[2];
   // node -> its cells, for the node-sum scatter (built on first use): the
   // entries of node n are node_cell_off[n] .. node_cell_off[n+1], each the
   // offset (cell * ncn + local node) * 3 of the node's slot in a per-cell

@@ -9,14 +9,15 @@ namespace lsmf {
 
 // A cell loop runs over `cells[0 .. n_list)` when `cells` is given (one
 // colour of the lattice: no two listed cells share a node, so the scatter
-// is a plain read-modify-write), else over all cells of the level with
+// is a plain read-modify-write; batches: the list names whole batches of
+// cells, for the production vmult kernel), else over all cells of the level with
 // atomic scatter, or, with `cellbuf` (full vmult cell loop only), storing
 // every cell's results to cellbuf[cell][local node][component] for a node
 // sum that follows.
 struct CellRange {
   const int *cells = nullptr;
   int n_list = 0;
-  bool plain = false;
+  bool plain = false, batches = false;
   void *cellbuf = nullptr;
   // fused interface exchange of a partitioned FP64 vmult (full cell loop,
   // atomic scatter): `peer_nodes` replaces the level's index map; its nodes
@@ -31,9 +32,9 @@ struct CellRange {
   // one chunk of a cell loop split over concurrent streams
   int first = 0, count = -1;
   cudaStream_t stream = nullptr;
-  // launched right after the kernel that writes dst's identity rows, as its
-  // programmatic dependent: the production kernel waits for it only before
-  // its first scatter
+  // launched right after the kernel that writes dst's identity rows, or the
+  // group of batches before, as its programmatic dependent: the production
+  // kernel waits for it only before its first scatter
   bool dependent = false;
 };
 

@@ -44,6 +44,7 @@ struct KArgs {
   int wait_tries;        // try_wait calls before a bulk-copy wait gives up
   int prefetch;          // plain loads: L1 prefetch of the records (0 off, 1 this unit, 2 the next unit)
   const int *cells;      // cell list of one colour (nullptr: all n_cells cells)
+  int n_batches;         // cells lists this many batches of the n_cells cells (production vmult)
   int plain;             // scatter with plain adds (colour launches) instead of atomics
   T *cellbuf;            // node-sum scatter: per-cell results [cell][local node][component]
   // fused interface exchange (SC_PEER): the neighbour part's vectors, read
@@ -470,8 +471,9 @@ __global__ void __launch_bounds__(256) apply_kernel(KArgs<T> a, Tab<P, Q> tab) {
 // the slice's points are done, so copies stay in flight through the whole
 // unit; without it the records are read with plain coalesced loads.
 // SC (scatter): SC_ATOMIC loops over all cells and adds with atomics;
-// SC_COLOUR over the cell list of one lattice colour (a.cells, a.n_cells
-// entries; no two of them share a node) with plain adds; SC_CELLBUF over all
+// SC_COLOUR over the list of one group of batches (a.cells, a.n_batches
+// entries; no two batches share a node) with plain adds, the cells of a batch
+// one after the other; SC_CELLBUF over all
 // cells, storing every cell's results to
 // a.cellbuf[cell][local node][component] (constrained rows as zero) for the
 // node sum that follows; SC_PEER as SC_ATOMIC, with the neighbour part's
@@ -573,15 +575,13 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   constexpr bool COL = SC == SC_COLOUR;
   constexpr bool SCALAR = (VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1);
   static_assert(H == TH, "one number holds the cells of a table entry");
-  static_assert(!(RING && COL), "the ring streams whole batches");
   using S = SFC<P, Q, T>;
-  using UM = UnitMap<P, Q, T, COL>;
+  using UM = UnitMap<P, Q, T, false>;
   using RL = RecLayout<P, Q, TH>;
   constexpr int N1 = P + 1, NN = S::NN, L = S::L, CPW = S::CPW, LW = S::LW;
-  // record access in numbers of T; the pairs of a cell list are put together
-  // from their two cells, in scalars
-  constexpr int U = COL ? TH : 1, TS = U, CS = LW * U, RS = CPW * U;
-  const int SS = a.slice_elems / (COL ? 1 : H);
+  // record access in numbers of T
+  constexpr int TS = 1, CS = LW, RS = CPW;
+  const int SS = a.slice_elems / H;
   const int WPB = blockDim.x >> 5;
   extern __shared__ __align__(128) unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -593,11 +593,10 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   T *slab = (T *)(wbase + D * slice_bytes + 16 * ((D + 1) / 2));
   T *park = slab + S::SZ + lp.ln;  // entry (s, c, e) at ((s * 3 + c) * 3 + e) * LW
   const int gw = blockIdx.x * WPB + warp, nw = gridDim.x * WPB;
-  const int n_units = UM::units(a.n_cells);
-  // list entry -> cell
-  auto cid = [&](int i) -> int { return COL ? __ldg(a.cells + i) : a.cell0 + i; };
-  // batch of a contiguous unit (a.cell0 is a multiple of the batch size)
-  auto batch_ptr = [&](int w) -> const E * { return a.table + (size_t)(a.cell0 / RL::B + w) * a.batch_elems; };
+  const int n_units = COL ? a.n_batches : UM::units(a.n_cells);
+  // batch of a unit, counted from a.cell0 (a multiple of the batch size)
+  auto batch = [&](int w) -> int { return COL ? __ldg(a.cells + w) : w; };
+  auto batch_ptr = [&](int w) -> const E * { return a.table + (size_t)(a.cell0 / RL::B + batch(w)) * a.batch_elems; };
   uint64_t pol = 0;
   auto copy_slice = [&](int w, int s, int place) {
     mbar_expect_tx(&bar[place], slice_bytes);
@@ -618,13 +617,13 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   uint32_t parity = 0;  // copy completes
   // cells of the lane: c[h]; ok[h]: stored by this lane
   auto cells_of = [&](int w, int c[H], bool ok[H]) {
-    const int e0 = UM::entry(w, lp.r);
+    const int e0 = UM::entry(batch(w), lp.r);
     const int last = a.n_cells - 1;
     const int f = e0 < a.n_cells ? e0 : last - last % H;
-    c[0] = cid(f);
+    c[0] = a.cell0 + f;
     ok[0] = lp.act && e0 < a.n_cells;
     if (H == 2) {
-      c[H - 1] = f + 1 < a.n_cells ? cid(f + 1) : c[0];
+      c[H - 1] = f + 1 < a.n_cells ? c[0] + 1 : c[0];
       ok[H - 1] = lp.act && e0 + 1 < a.n_cells;
     }
   };
@@ -658,7 +657,7 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   };
   // the reference metric of a batch into L1, ahead of its use
   auto prefetch_ref = [&](int w) {
-    if (SCALAR && !COL && a.ref_per_cell && lane * 128 < 9 * RL::B * (int)sizeof(E))
+    if (SCALAR && a.ref_per_cell && lane * 128 < 9 * RL::B * (int)sizeof(E))
       asm volatile("prefetch.global.L1 [%0];" ::"l"((const char *)(batch_ptr(w) + (size_t)Q * a.slice_elems) + lane * 128));
   };
   if (gw < n_units) {
@@ -672,12 +671,7 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
     bool ok[H];
     cells_of(w, c, ok);
     // the cell's record at lane 0 of the cell, and its reference metric
-    auto rec_at = [&](size_t (*at)(int, int, int)) {
-      if constexpr (COL && H == 2)
-        return RecPair{a.table + at(c[0], a.batch_elems, a.slice_elems), a.table + at(c[H - 1], a.batch_elems, a.slice_elems)};
-      else return (const T *)(a.table + at(c[0], a.batch_elems, a.slice_elems));
-    };
-    const auto rec = rec_at([](int cell, int be, int) { return RL::base(cell, be); });
+    const T *rec = (const T *)(a.table + RL::base(c[0], a.batch_elems));
     T ux[3][Q];  // scalar_referential: displacement along the x line
     if (VAR == VAR_SCALAR_REF) {
 #pragma unroll
@@ -711,7 +705,7 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
         prefetch(w + nw);
         prefetch_ref(w + nw);
       }
-      if (!RING && !COL && a.prefetch) {
+      if (!RING && a.prefetch) {
         // one 128-byte line of the records per lane into L1, issued before
         // the sweeps so that the point loop's loads find it there
         const int pw = a.prefetch == 2 ? w + nw : w;
@@ -739,7 +733,7 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
       lambda = join_of<T>(m[1], H - 1);
       kappa = join_of<T>(m[2], H - 1);
     }
-    const auto ref = rec_at([](int cell, int be, int se) { return RL::ref(cell, be, se); });
+    const T *ref = (const T *)(a.table + RL::ref(c[0], a.batch_elems, a.slice_elems));
     auto point = [&](int s, auto slice) {
       line_point<Q, T, VAR, CS, TS, LW>(G[s], s, slice, ref, RS, a.ref_per_cell != 0, park + s * 9 * LW, ux, lp, tab.Dc, mu, lambda, kappa);
     };
@@ -777,9 +771,7 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
     // dst's rows are written by the kernel before (no effect in a launch that
     // is not its programmatic dependent)
     if (w == gw) asm volatile("griddepcontrol.wait;" ::: "memory");
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-      if (!ok[h]) continue;
+    auto scatter = [&](int h) {
 #pragma unroll
       for (int k = 0; k < N1; ++k) {
         const int packed = ck[h][k];
@@ -796,12 +788,45 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
             if (!con)
               atomic_add(((packed & PEER_BIT) ? a.pdst : a.dst) + 3 * (size_t)(packed & PEER_NODE_MASK) + i, o);
           } else if (!con) {
-            E *d = a.dst + 3 * (size_t)(packed & NODE_MASK) + i;
-            if (COL) *d += o;
-            else atomic_add(d, o);
+            atomic_add(a.dst + 3 * (size_t)(packed & NODE_MASK) + i, o);
           }
         }
       }
+    };
+    // plain adds of a line's values: all loads before the first store, as one
+    // round trip (the compiler has to take nine in turn).  From L2: with the
+    // launches of the groups overlapping, L1 may hold an earlier group's line.
+    // 60^3 Q2 tensor4 FP64: 462 us, 707 with nine round trips; 747 us with one
+    // cell per warp and a launch per lattice colour.
+    auto add_line = [&](int h) {
+      E old[N1][3];
+#pragma unroll
+      for (int k = 0; k < N1; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) old[k][i] = __ldcg(a.dst + 3 * (size_t)(ck[h][k] & NODE_MASK) + i);
+#pragma unroll
+      for (int k = 0; k < N1; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          E o;
+          if constexpr (H == 2) o = h ? hi2(out[i][k]) : lo2(out[i][k]);
+          else o = out[i][k];
+          if (!((ck[h][k] >> (NODE_BITS + i)) & 1)) a.dst[3 * (size_t)(ck[h][k] & NODE_MASK) + i] = old[k][i] + o;
+        }
+    };
+    if constexpr (COL) {
+      // neighbours within the batch add to the same nodes: in cell order
+      for (int r = 0; r < CPW; ++r) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          if (lp.r == r && ok[h]) add_line(h);
+          __syncwarp();
+        }
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < H; ++h)
+        if (ok[h]) scatter(h);
     }
   }
 }
@@ -1142,6 +1167,7 @@ KArgs<T> make_args(const lsmf_op *op) {
   KArgs<T> a;
   a.cell_nodes = L.d_cell_nodes.ptr;
   a.n_cells = L.n_cells;
+  a.n_batches = 0;
   a.slice_elems = op->slice_elems;
   a.batch_elems = op->batch_elems;
   a.ring = 0;
@@ -1171,7 +1197,8 @@ template <typename T>
 void set_range(KArgs<T> &a, const CellRange &r) {
   if (r.cells) {
     a.cells = r.cells;
-    a.n_cells = r.n_list;
+    if (r.batches) a.n_batches = r.n_list;
+    else a.n_cells = r.n_list;
   }
   a.plain = r.plain ? 1 : 0;
   a.cellbuf = (T *)r.cellbuf;
@@ -1211,7 +1238,6 @@ lsmf_status launch_line(const lsmf_op *op, KArgs<typename Num<T>::S> a, bool pee
   using E = typename Num<T>::S;
   const TabT<P, Q, T> tab = make_tabt<P, Q, T>(op->mesh->basis);
   const bool col = a.cells != nullptr, cellbuf = a.cellbuf != nullptr;
-  if (col) ring = 0;
   const size_t slice_bytes = a.slice_elems * sizeof(E);
   auto wbytes = [&](int d) { return line_warp_bytes<P, Q, T, VAR == VAR_SCALAR_F0 || VAR == VAR_SCALAR_F1>(d, slice_bytes); };
   // a smaller ring when it would leave fewer than 4 warps per SM
@@ -1221,7 +1247,7 @@ lsmf_status launch_line(const lsmf_op *op, KArgs<typename Num<T>::S> a, bool pee
   // smaller blocks let several blocks share an SM
   const int w = warps_for_budget(wbytes(ring), max_warps < 4 ? max_warps : 4, 220 * 1024);
   const size_t smem = w * wbytes(ring);
-  const int units = col ? UnitMap<P, Q, T, true>::units(a.n_cells) : UnitMap<P, Q, T, false>::units(a.n_cells);
+  const int units = col ? a.n_batches : UnitMap<P, Q, T, false>::units(a.n_cells);
   auto go = [&](auto k) -> lsmf_status {
     // small launches are bound by the host: shared memory up to 48 KB needs
     // no attribute, and a grid within the SMs no occupancy query
@@ -1241,7 +1267,7 @@ lsmf_status launch_line(const lsmf_op *op, KArgs<typename Num<T>::S> a, bool pee
     LSMF_CUDA(cudaLaunchKernelEx(&cfg, k, a, tab));
     return LSMF_OK;
   };
-  if (col) return go(apply_line_kernel<P, Q, T, VAR, false, SC_COLOUR>);
+  if (col) return ring ? go(apply_line_kernel<P, Q, T, VAR, true, SC_COLOUR>) : go(apply_line_kernel<P, Q, T, VAR, false, SC_COLOUR>);
   if (cellbuf) return ring ? go(apply_line_kernel<P, Q, T, VAR, true, SC_CELLBUF>) : go(apply_line_kernel<P, Q, T, VAR, false, SC_CELLBUF>);
   if constexpr (sizeof(E) == 8)
     if (peer) return ring ? go(apply_line_kernel<P, Q, T, VAR, true, SC_PEER>) : go(apply_line_kernel<P, Q, T, VAR, false, SC_PEER>);
@@ -1270,6 +1296,10 @@ lsmf_status run_apply(const lsmf_op *op, T *dst, const T *src, unsigned mask, Ce
     return LSMF_ERR_INVALID_ARG;
   }
   if (full && !op->basic) {
+    if (col && !range.batches) {
+      set_error("the production vmult kernel takes a list of batches");
+      return LSMF_ERR_INVALID_ARG;
+    }
     if (a.cell0 % RecLayout<P, Q, table_halves<T>()>::B != 0) {
       set_error("a chunk of the cell loop must start at a whole batch of cells");
       return LSMF_ERR_INVALID_ARG;

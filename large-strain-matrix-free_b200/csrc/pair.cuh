@@ -105,12 +105,4 @@ __device__ __forceinline__ f2 &operator-=(f2 &c, f2p p) { return c = fma2(neg2(p
 __device__ __forceinline__ f2 &operator-=(f2 &c, f2 a) { return c = sub2(c, a); }
 __device__ __forceinline__ f2 &operator*=(f2 &c, f2 a) { return c = mul2(c, a); }
 
-// The records of two cells read as one: element i is the pair
-// (first[i], second[i]).
-struct RecPair {
-  const float *p0, *p1;
-  __device__ __forceinline__ f2 operator[](int i) const { return pack2(__ldg(p0 + i), __ldg(p1 + i)); }
-  __device__ __forceinline__ RecPair operator+(int i) const { return {p0 + i, p1 + i}; }
-};
-
 }  // namespace lsmf
