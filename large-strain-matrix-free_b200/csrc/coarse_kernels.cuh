@@ -21,8 +21,9 @@
 // one load trip through L2 per step.  Two buffers alternate: a CTA stores
 // step k + 2 only after it has seen step k + 1 of its neighbours, which they
 // store after they have read step k.  Waits are bounded: a CTA that gives up
-// sets the operator's error word and returns, and so do the CTAs that wait
-// for it.
+// stores NaN for its nodes, sets the operator's error word and returns, and
+// so do the CTAs that wait for it (a CTA that owns no node matters only to
+// those).
 // A step at 15^3 Q2 cells (141 CTAs, tensor4) takes 3.7 us in FP32 and 5.4 us
 // in FP64, where the two launches took 7.2 and 10.1 us.  Of the FP32 step the
 // cell operator is 1.75 us (issue: two warps per scheduler), the exchange 1.2
@@ -501,6 +502,12 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
     if (!nodes.receive((unsigned)k, a.wait_tries)) dead = 1;
     __syncthreads();
     if (dead) {
+      // no solution: what x holds from an earlier call is not to be taken for one
+#pragma unroll
+      for (int q = 0; q < NPT; ++q)
+        if (nodes.has(q) && (nodes.node[q] & 1))
+#pragma unroll
+          for (int i = 0; i < 3; ++i) ca.x[3 * (size_t)(nodes.node[q] >> 1) + i] = T(nan(""));
       if (threadIdx.x == 0) atomicOr(a.flag, FLAG_TIMEOUT);
       return;
     }
