@@ -191,8 +191,12 @@ lsmf_status lsmf_operator_el(lsmf_op *op, int row, int col, double *value);
  *   chunks' streams and events are created by lsmf_operator_cache (and by
  *   this option on a cached operator), not by the vmult.
  * A bounded device wait that runs out in the pipelined or the coarse-level
- * kernels is reported as LSMF_ERR_TIMEOUT by lsmf_operator_sync, lsmf_cg_solve and the GMG
- * set-up (the next synchronising call on the operator). */
+ * kernels is reported once, as LSMF_ERR_TIMEOUT, by the next of
+ * lsmf_operator_sync and lsmf_cg_solve on the operator, and for the kernels
+ * of a V-cycle by the next of lsmf_gmg_sync, lsmf_gmg_setup and lsmf_cg_solve
+ * on the GMG object.  A set-up or a solve that reports a V-cycle from before
+ * it (the message says so) has done its own work: the GMG object is set up,
+ * x and info hold the solve's result. */
 enum { LSMF_OPT_BULK_PIPELINE = 1, LSMF_OPT_BASIC_KERNEL = 2, LSMF_OPT_MAX_WARPS = 3, LSMF_OPT_WAIT_TRIES = 4,
        LSMF_OPT_SCATTER = 5, LSMF_OPT_RECORD_PREFETCH = 6, LSMF_OPT_CELL_PAIRS = 7, LSMF_OPT_CHUNKS = 8 };
 enum { LSMF_SCATTER_ATOMIC = 0, LSMF_SCATTER_COLOUR8 = 1, LSMF_SCATTER_NODESUM = 2 };
@@ -239,8 +243,13 @@ lsmf_status lsmf_gmg_set_material(lsmf_gmg *g, const double *mu_per_fine_cell, d
 /* interpolate_to_mg + level cache + diagonal + Chebyshev eigenvalue
  * estimates (mf_elasticity.h:1929-2113); d_u_fine: FP64 device vector */
 lsmf_status lsmf_gmg_setup(lsmf_gmg *g, const double *d_u_fine);
-/* PreconditionMG::vmult: one V-cycle, dst = M^-1 src (FP64 device vectors) */
+/* PreconditionMG::vmult: one V-cycle, dst = M^-1 src (FP64 device vectors);
+ * a coarse solve whose bounded wait ran out gives NaN */
 lsmf_status lsmf_gmg_vmult(lsmf_gmg *g, double *d_dst, const double *d_src);
+/* Waits for the object's stream and reports the device error words of the
+ * level operators (LSMF_ERR_TIMEOUT: a bounded wait ran out in a V-cycle
+ * since the last report).  No reference counterpart. */
+lsmf_status lsmf_gmg_sync(lsmf_gmg *g);
 /* Chebyshev data of a level: out6 = {eig_min, eig_max (Lanczos estimates),
  * degree, theta, delta, eigenvalue-CG iterations} */
 lsmf_status lsmf_gmg_level_info(const lsmf_gmg *g, int level, double *out6);

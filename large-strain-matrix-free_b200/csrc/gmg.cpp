@@ -450,6 +450,37 @@ lsmf_status gmg_vmult_impl(lsmf_gmg *g, double *dst, const double *src) {
   return LSMF_OK;
 }
 
+// the error words of the level operators, read (the stream is waited for)
+// and cleared: an error is reported once
+lsmf_status take_level_words(lsmf_gmg *g, int *bits) {
+  const size_t nl = g->levels.size();
+  std::vector<int> word(nl, 0);
+  for (size_t l = 0; l < nl; ++l)
+    LSMF_CUDA(cudaMemcpyAsync(&word[l], g->levels[l].op->d_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+  LSMF_CUDA(cudaStreamSynchronize(g->stream));
+  *bits = 0;
+  for (size_t l = 0; l < nl; ++l)
+    if (word[l]) {
+      *bits |= word[l];
+      LSMF_CUDA(cudaMemsetAsync(g->levels[l].op->d_flag.ptr, 0, sizeof(int), g->stream));
+    }
+  g->unread = false;
+  return LSMF_OK;
+}
+
+// status of an error word's bits that a vmult or V-cycle left
+lsmf_status word_status(int bits, const char *where) {
+  if (bits & 2) {
+    set_error(std::string("a bounded device wait timed out in ") + where);
+    return LSMF_ERR_TIMEOUT;
+  }
+  if (bits & 4) {
+    set_error(std::string("a kernel was launched with less shared memory than its layout needs and did no work, in ") + where);
+    return LSMF_ERR_CUDA;
+  }
+  return LSMF_OK;
+}
+
 }  // namespace
 }  // namespace lsmf
 
@@ -538,7 +569,18 @@ lsmf_status lsmf_gmg_setup(lsmf_gmg *g, const double *d_u) {
   // the executable V-cycle graph is kept: the next vmult captures the new
   // launch sequence and updates it in place
   g->vstale = true;
-  return g->desc.precision == LSMF_FP64 ? gmg_setup_impl<double>(g, d_u) : gmg_setup_impl<float>(g, d_u);
+  // the set-up clears the words: what V-cycles before it left is reported here
+  int earlier = 0;
+  if (g->unread) LSMF_TRY(take_level_words(g, &earlier));
+  LSMF_TRY(g->desc.precision == LSMF_FP64 ? gmg_setup_impl<double>(g, d_u) : gmg_setup_impl<float>(g, d_u));
+  return word_status(earlier, "a V-cycle before this set-up, which is complete");
+}
+
+lsmf_status lsmf_gmg_sync(lsmf_gmg *g) {
+  if (!g) { set_error("null argument"); return LSMF_ERR_INVALID_ARG; }
+  int bits = 0;
+  LSMF_TRY(take_level_words(g, &bits));
+  return word_status(bits, "a V-cycle");
 }
 
 lsmf_status lsmf_gmg_level_operator(lsmf_gmg *g, int level, lsmf_op **op) {
@@ -572,6 +614,7 @@ lsmf_status lsmf_gmg_set_option(lsmf_gmg *g, int option, int value) {
 lsmf_status lsmf_gmg_vmult(lsmf_gmg *g, double *dst, const double *src) {
   if (!g || !dst || !src) { set_error("null argument"); return LSMF_ERR_INVALID_ARG; }
   if (!g->ready) { set_error("lsmf_gmg_setup has not been called"); return LSMF_ERR_NOT_INITIALIZED; }
+  g->unread = true;
   auto run = [&]() {
     return g->desc.precision == LSMF_FP64 ? gmg_vmult_impl<double>(g, dst, src) : gmg_vmult_impl<float>(g, dst, src);
   };
@@ -650,6 +693,8 @@ lsmf_status lsmf_cg_solve(lsmf_op *A, int precond, double omega, lsmf_gmg *gmg, 
   const size_t n = (size_t)A->L().n_dofs();
   cudaStream_t st = A->stream;
   if (gmg) lsmf_gmg_set_stream(gmg, st);
+  int earlier = 0;  // what V-cycles before this solve left in the levels' error words
+  if (precond == 2 && gmg->unread) LSMF_TRY(take_level_words(gmg, &earlier));
   LSMF_TRY(A->cg_g.alloc(n));
   LSMF_TRY(A->cg_h.alloc(n));
   LSMF_TRY(A->cg_d.alloc(n));
@@ -698,30 +743,20 @@ lsmf_status lsmf_cg_solve(lsmf_op *A, int precond, double omega, lsmf_gmg *gmg, 
       ++k;
     }
   }
-  int flag = 0, coarse_flag = 0;
+  int flag = 0;
   LSMF_CUDA(cudaMemcpyAsync(&flag, A->d_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-  // the coarse-level kernel of the preconditioner has bounded waits too
-  int *d_coarse_flag = precond == 2 && gmg->coarse.usable ? gmg->levels[0].op->d_flag.ptr : nullptr;
-  if (d_coarse_flag) LSMF_CUDA(cudaMemcpyAsync(&coarse_flag, d_coarse_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
-  LSMF_CUDA(cudaStreamSynchronize(st));
-  if (coarse_flag & 2) {
-    LSMF_CUDA(cudaMemsetAsync(d_coarse_flag, 0, sizeof(int), st));
-    flag |= 2;
-  }
+  // the kernels of the preconditioner have words of their own
+  int levels = 0;
+  if (precond == 2) LSMF_TRY(take_level_words(gmg, &levels));
+  else LSMF_CUDA(cudaStreamSynchronize(st));
   if (info) { info->iterations = it; info->residual = res; info->converged = conv ? 1 : 0; }
-  if (flag & 2) {
+  if (flag & 6) {
     // reported once: the word is cleared for the calls that follow
     LSMF_CUDA(cudaMemsetAsync(A->d_flag.ptr, 0, sizeof(int), st));
     LSMF_CUDA(cudaStreamSynchronize(st));
-    set_error("a bounded device wait timed out in the vmult or the coarse-level kernel");
-    return LSMF_ERR_TIMEOUT;
   }
-  if (flag & 4) {
-    LSMF_CUDA(cudaMemsetAsync(A->d_flag.ptr, 0, sizeof(int), st));
-    LSMF_CUDA(cudaStreamSynchronize(st));
-    set_error("a vmult kernel was launched with less shared memory than its layout needs and did no work");
-    return LSMF_ERR_CUDA;
-  }
+  LSMF_TRY(word_status(flag | levels, precond == 2 ? "the vmult or the V-cycle" : "the vmult"));
+  LSMF_TRY(word_status(earlier, "a V-cycle before this solve, which ran as reported"));
   if (!conv) {
     // the facts of deal.II's SolverControl::NoConvergence: last step and value
     char msg[160];

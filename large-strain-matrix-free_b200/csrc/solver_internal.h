@@ -143,6 +143,7 @@ struct lsmf_gmg {
   lsmf::CoarsePlan coarse;
   cudaStream_t stream = 0;
   bool ready = false;
+  bool unread = false;  // V-cycles ran since the levels' error words were last read
   // the V-cycle replayed as one CUDA graph: captured again after each
   // set-up (vstale) and applied to the executable graph in place when the
   // launch sequence is unchanged

@@ -93,6 +93,7 @@ SIGNATURES = {
     "lsmf_gmg_set_material": (ctypes.c_int, [vp, dp, ctypes.c_double]),
     "lsmf_gmg_setup": (ctypes.c_int, [vp, vp]),
     "lsmf_gmg_vmult": (ctypes.c_int, [vp, vp, vp]),
+    "lsmf_gmg_sync": (ctypes.c_int, [vp]),
     "lsmf_gmg_level_info": (ctypes.c_int, [vp, ctypes.c_int, dp]),
     "lsmf_gmg_set_stream": (ctypes.c_int, [vp, vp]),
     "lsmf_gmg_set_option": (ctypes.c_int, [vp, ctypes.c_int, ctypes.c_int]),
@@ -427,6 +428,11 @@ class GMG:
 
     def vmult(self, dst, src):
         check(lib().lsmf_gmg_vmult(self.h, _dptr(dst), _dptr(src)))
+
+    def sync(self):
+        """Wait for the object's stream; raises LsmfError (status 8) if a
+        bounded device wait ran out in a V-cycle since the last report."""
+        check(lib().lsmf_gmg_sync(self.h))
 
     def set_graph(self, enable):
         """Replay the V-cycle as one CUDA graph (default) or launch kernel by kernel."""

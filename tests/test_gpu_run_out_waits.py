@@ -46,3 +46,45 @@ def test_solve_ends_with_the_first_run_out_wait(precision):
     g.level_option(0, WAIT_TRIES, -1)
     x.zero_()
     assert lsmf.cg_solve(op, x, b, 1e-8 * float(b.norm()), 100, "gmg", g)["converged"]
+
+
+def test_sync_reports_a_vcycle_once():
+    g, op, u, b = _problem()
+    g.sync()
+    g.level_option(0, WAIT_TRIES, 0)
+    _vcycle(g, b)
+    with pytest.raises(lsmf.LsmfError) as e:
+        g.sync()
+    assert e.value.status == TIMEOUT
+    g.sync()
+
+
+def test_setup_reports_the_vcycle_before_it():
+    g, op, u, b = _problem()
+    good = _vcycle(g, b)
+    g.level_option(0, WAIT_TRIES, 0)
+    _vcycle(g, b)
+    g.level_option(0, WAIT_TRIES, -1)
+    with pytest.raises(lsmf.LsmfError) as e:
+        g.setup(u)
+    assert e.value.status == TIMEOUT and "before this set-up" in str(e.value)
+    again = _vcycle(g, b)  # the set-up was complete
+    assert float((again - good).abs().max() / good.abs().max()) < 1e-10
+    g.setup(u)
+    g.sync()
+
+
+def test_solve_tells_an_earlier_vcycle_from_its_own():
+    g, op, u, b = _problem()
+    g.level_option(0, WAIT_TRIES, 0)
+    _vcycle(g, b)
+    g.level_option(0, WAIT_TRIES, -1)
+    x, info, tol = torch.zeros_like(b), lsmf.SolveInfo(), 1e-8 * float(b.norm())
+    st = lsmf.lib().lsmf_cg_solve(op.h, 2, 1.0, g.h, lsmf._dptr(x), lsmf._dptr(b), tol, 100, ctypes.byref(info))
+    assert st == TIMEOUT and b"before this solve" in lsmf.lib().lsmf_last_error()
+    assert info.converged and info.residual <= tol
+    r = torch.empty_like(b)
+    op.vmult(r, x)
+    assert float((r - b).norm()) <= 1.01 * tol
+    x.zero_()
+    assert lsmf.cg_solve(op, x, b, tol, 100, "gmg", g)["converged"]
