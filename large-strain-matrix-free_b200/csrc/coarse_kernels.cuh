@@ -716,6 +716,7 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
     __syncthreads();
     if (dead) break;
   }
+  __syncthreads();  // the first reduction's outcome, where the loop was not entered
   if (threadIdx.x == 0) {
     if (dead) atomicOr(a.flag, FLAG_TIMEOUT);
     if (blockIdx.x == 0) *ea.its = its;

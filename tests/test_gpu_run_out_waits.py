@@ -88,3 +88,16 @@ def test_solve_tells_an_earlier_vcycle_from_its_own():
     assert float((r - b).norm()) <= 1.01 * tol
     x.zero_()
     assert lsmf.cg_solve(op, x, b, tol, 100, "gmg", g)["converged"]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_estimate_of_a_run_out_wait_fails_the_setup(precision):
+    gm, g, mu, u, b = _setup(2, (8, 8, 8), 0, "tensor4", 1, precision)
+    for _ in range(5):
+        g.level_option(0, WAIT_TRIES, 0)
+        with pytest.raises(lsmf.LsmfError) as e:
+            g.setup(u)
+        assert e.value.status == TIMEOUT
+    g.level_option(0, WAIT_TRIES, -1)
+    g.setup(u)
+    assert torch.isfinite(_vcycle(g, b)).all()
