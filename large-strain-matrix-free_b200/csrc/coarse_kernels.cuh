@@ -83,7 +83,7 @@ __host__ __device__ inline size_t coarse_unit_bytes(int slice_elems) {
 
 template <typename E>
 struct CoarseArgs {
-  int n_cta, warps, cells_per_cta, max_nodes, max_items, n_slots;
+  int n_cta, warps, cells_per_cta, max_nodes, max_items, max_sums, n_slots;
   int unit_bytes;
   const int *counts, *cells, *send, *item_slot;
   const uint16_t *lid, *contrib, *item_place, *first;
@@ -97,6 +97,26 @@ struct CoarseArgs {
   int degree;
 };
 
+// The units of a plan are as long as this kernel's, and the CTA has room for
+// them and for what CoarseNodes keeps behind them
+template <int P, int Q, typename T, int VAR, typename E>
+__device__ __forceinline__ bool coarse_smem_short(const KArgs<E> &a, const CoarseArgs<E> &ca) {
+  constexpr int XS = coarse_stride<E>();
+  const size_t tail = ((size_t)((XS * ca.max_nodes + 3) / 4 * 4) + (size_t)XS * ca.max_sums) * sizeof(E);
+  const bool unit = (size_t)ca.unit_bytes >= coarse_unit_bytes<P, Q, T, VAR>(a.slice_elems);
+  return smem_short(unit ? (size_t)ca.warps * ca.unit_bytes + tail : ~(size_t)0, a.flag);
+}
+
+// NaN at the nodes a CTA stores: what x holds from an earlier call is not to
+// be taken for a solution
+template <typename E>
+__device__ void coarse_no_solution(const CoarseArgs<E> &ca) {
+  const unsigned *nodes = ca.nodes + (size_t)blockIdx.x * ca.max_nodes;
+  for (int n = threadIdx.x; n < ca.counts[4 * blockIdx.x + 1]; n += blockDim.x)
+    if (nodes[n] & 1)
+      for (int i = 0; i < 3; ++i) ca.x[3 * (size_t)(nodes[n] >> 1) + i] = E(nan(""));
+}
+
 template <typename E>
 CoarseArgs<E> coarse_args(const CoarsePlan &p) {
   CoarseArgs<E> c{};
@@ -105,6 +125,7 @@ CoarseArgs<E> coarse_args(const CoarsePlan &p) {
   c.cells_per_cta = p.cells_per_cta;
   c.max_nodes = p.max_nodes;
   c.max_items = p.max_items;
+  c.max_sums = p.max_sums;
   c.n_slots = p.n_slots;
   c.unit_bytes = (int)p.unit_bytes;
   c.counts = p.counts;
@@ -472,6 +493,10 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
     coarse_cheb_kernel(KArgs<T> a, TabT<P, Q, T> tab, CoarseArgs<T> ca) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int dead;
+  if (coarse_smem_short<P, Q, T, VAR>(a, ca)) {
+    coarse_no_solution(ca);
+    return;
+  }
   if (threadIdx.x == 0) dead = 0;
   CoarseCells<P, Q, T, VAR> cells(a, tab, ca, smem);
   CoarseNodes<T, NPT> nodes(ca, smem);
@@ -502,12 +527,7 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
     if (!nodes.receive((unsigned)k, a.wait_tries)) dead = 1;
     __syncthreads();
     if (dead) {
-      // no solution: what x holds from an earlier call is not to be taken for one
-#pragma unroll
-      for (int q = 0; q < NPT; ++q)
-        if (nodes.has(q) && (nodes.node[q] & 1))
-#pragma unroll
-          for (int i = 0; i < 3; ++i) ca.x[3 * (size_t)(nodes.node[q] >> 1) + i] = T(nan(""));
+      coarse_no_solution(ca);
       if (threadIdx.x == 0) atomicOr(a.flag, FLAG_TIMEOUT);
       return;
     }
@@ -621,6 +641,10 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ double sh[2][COARSE_MAX_WARPS][2];
   __shared__ int dead;
+  if (coarse_smem_short<P, Q, T, VAR>(a, ca)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ea.its = 0;
+    return;
+  }
   if (threadIdx.x == 0) dead = 0;
   CoarseCells<P, Q, T, VAR> cells(a, tab, ca, smem);
   CoarseNodes<T, NPT> nodes(ca, smem);

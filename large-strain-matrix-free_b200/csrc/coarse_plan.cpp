@@ -235,6 +235,7 @@ lsmf_status build_coarse_plan(const lsmf_op *op, int sms, size_t smem_limit, Coa
   plan.cells_per_cta = sh.cells;
   plan.max_nodes = max_nodes;
   plan.max_items = max_items;
+  plan.max_sums = max_sums;
   plan.n_slots = n_slots;
   plan.packets = elem == 8 ? 2 : 1;
   plan.unit_bytes = sh.unit_bytes;

@@ -33,7 +33,7 @@ struct CoarseShape {
 // number of CTAs that share them, then of contributions, both falling.
 struct CoarsePlan {
   bool usable = false;
-  int n_cta = 0, warps = 0, cells_per_cta = 0, max_nodes = 0, max_items = 0, n_slots = 0, packets = 0;
+  int n_cta = 0, warps = 0, cells_per_cta = 0, max_nodes = 0, max_items = 0, max_sums = 0, n_slots = 0, packets = 0;
   size_t unit_bytes = 0, smem = 0;
   // device arrays, parts of one buffer
   const int *counts = nullptr;           // [cta][4]: cells, nodes, items, 0

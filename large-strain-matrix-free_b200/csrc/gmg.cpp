@@ -69,6 +69,19 @@ std::vector<double> coarsen_cell_field(const lsmf_mesh &M, int level, const std:
 
 namespace {
 
+// status of an error word's bits that a vmult or V-cycle left
+lsmf_status word_status(int bits, const char *where) {
+  if (bits & 2) {
+    set_error(std::string("a bounded device wait timed out in ") + where);
+    return LSMF_ERR_TIMEOUT;
+  }
+  if (bits & 4) {
+    set_error(std::string("a kernel was launched with less shared memory than its layout needs and did no work, in ") + where);
+    return LSMF_ERR_CUDA;
+  }
+  return LSMF_OK;
+}
+
 // CG with the inverse diagonal on a level operator (PreconditionChebyshev's
 // eigenvalue estimate): start vector (i % 11) - mean, ReductionControl with
 // absolute sqrt(eps) and relative 1e-10, extreme eigenvalues of the Lanczos
@@ -132,12 +145,9 @@ lsmf_status estimate_eigenvalues(lsmf_gmg *g, int l, int max_it, double &emin, d
     LSMF_CUDA(cudaMemcpyAsync(&m, g->eig_kbase.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
     LSMF_CUDA(cudaMemcpyAsync(&flag, op->d_flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
     LSMF_CUDA(cudaStreamSynchronize(st));
-    if (flag & 2) {
-      // reported once: the word is cleared for the calls that follow
-      LSMF_CUDA(cudaMemsetAsync(op->d_flag.ptr, 0, sizeof(int), st));
-      set_error("a bounded device wait timed out in the coarse-level eigenvalue estimate");
-      return LSMF_ERR_TIMEOUT;
-    }
+    // reported once: the word is cleared for the calls that follow
+    if (flag & 6) LSMF_CUDA(cudaMemsetAsync(op->d_flag.ptr, 0, sizeof(int), st));
+    LSMF_TRY(word_status(flag, "the coarse-level eigenvalue estimate"));
     std::vector<double> h((size_t)2 * m);
     if (m) {
       LSMF_CUDA(cudaMemcpyAsync(h.data(), ha, m * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -465,19 +475,6 @@ lsmf_status take_level_words(lsmf_gmg *g, int *bits) {
       LSMF_CUDA(cudaMemsetAsync(g->levels[l].op->d_flag.ptr, 0, sizeof(int), g->stream));
     }
   g->unread = false;
-  return LSMF_OK;
-}
-
-// status of an error word's bits that a vmult or V-cycle left
-lsmf_status word_status(int bits, const char *where) {
-  if (bits & 2) {
-    set_error(std::string("a bounded device wait timed out in ") + where);
-    return LSMF_ERR_TIMEOUT;
-  }
-  if (bits & 4) {
-    set_error(std::string("a kernel was launched with less shared memory than its layout needs and did no work, in ") + where);
-    return LSMF_ERR_CUDA;
-  }
   return LSMF_OK;
 }
 

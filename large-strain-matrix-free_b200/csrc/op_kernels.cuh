@@ -154,6 +154,17 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // ran out, a kernel found less dynamic shared memory than its layout needs
 // (it returned without touching memory)
 constexpr int FLAG_DETF = 1, FLAG_TIMEOUT = 2, FLAG_SMEM = 4;
+// Dynamic shared memory of a launch against what the kernel's layout needs
+// (bytes, uniform over the grid).  The host computes the size of the kernels
+// whose layout depends on run-time values; where it gives them less, they set
+// the error word and touch no shared memory.
+__device__ __forceinline__ bool smem_short(size_t need, int *flag) {
+  uint32_t have;
+  asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(have));
+  if (have >= need) return false;
+  if (threadIdx.x == 0) atomicOr(flag, FLAG_SMEM);
+  return true;
+}
 // internal stage bit: gather constrained entries instead of zeroing them
 constexpr unsigned MASK_INHOM = MASK_INHOM_BIT;
 
@@ -588,7 +599,13 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   const LanePos<Q> lp;
   const int D = RING ? a.ring : 0;
   const uint32_t slice_bytes = (uint32_t)(a.slice_elems * sizeof(E));
-  unsigned char *wbase = smem + warp * line_warp_bytes<P, Q, T, SCALAR>(D, slice_bytes);
+  const size_t warp_bytes = line_warp_bytes<P, Q, T, SCALAR>(D, slice_bytes);
+  if (smem_short(WPB * warp_bytes, a.flag)) {
+    // the launch is not to end before the one whose dependent it is
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
+  unsigned char *wbase = smem + warp * warp_bytes;
   uint64_t *bar = (uint64_t *)(wbase + D * slice_bytes);
   T *slab = (T *)(wbase + D * slice_bytes + 16 * ((D + 1) / 2));
   T *park = slab + S::SZ + lp.ln;  // entry (s, c, e) at ((s * 3 + c) * 3 + e) * LW
