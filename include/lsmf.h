@@ -126,7 +126,10 @@ lsmf_status lsmf_operator_get_diagonal(lsmf_op *op, const void **d_diag, const v
 lsmf_status lsmf_operator_precondition_jacobi(lsmf_op *op, void *d_dst, const void *d_src, double omega);
 /* m(), n(), memory_consumption() (mf_nh_operator.h:300-392): rows and
  * columns (n_dofs); bytes of the cache tables plus the index map and node
- * coordinates (the MatrixFree data), diagonals excluded like the reference */
+ * coordinates (the MatrixFree data), diagonals excluded like the reference.
+ * The tables count with their full tensors, 51 values per point for tensor4
+ * and 90 for tensor4_ns; on the device the symmetric matrices take their
+ * upper triangle, 36 and 54 values. */
 int lsmf_operator_m(const lsmf_op *op);
 int lsmf_operator_n(const lsmf_op *op);
 size_t lsmf_operator_memory_consumption(const lsmf_op *op);

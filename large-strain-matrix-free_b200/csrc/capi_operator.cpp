@@ -185,8 +185,8 @@ lsmf_status lsmf_operator_create(lsmf_mesh *m, int level, lsmf_caching caching, 
   // scalar caching on affine cells: the reference inverse Jacobian is one
   // 3x3 block per cell beside the 11 per-point values (c, Eulerian inverse
   // Jacobian, JxW).  The documented tables of tensor4 and tensor4_ns hold
-  // full tensors; the stored records keep the upper triangles and use the
-  // front of the buffer.
+  // full tensors (memory_consumption counts those); the stored records keep
+  // the upper triangles.
   op->ref_per_cell = caching == LSMF_CACHE_SCALAR && L.affine;
   const int al = 16 / (int)op->elem(), extra = op->ref_per_cell ? 9 : 0;
   auto padded = [&](int n) { return (n + al - 1) / al * al; };
@@ -197,7 +197,7 @@ lsmf_status lsmf_operator_create(lsmf_mesh *m, int level, lsmf_caching caching, 
   op->batch_elems = L.q * op->slice_elems + padded(extra * B);
   op->table_bytes = (size_t)L.n_cells * padded(documented * L.nq() + extra) * op->elem();
   lsmf_status s;
-  if ((s = op->d_table.alloc(std::max(op->table_bytes, (size_t)n_batches * op->batch_elems * op->elem()))) != LSMF_OK ||
+  if ((s = op->d_table.alloc((size_t)n_batches * op->batch_elems * op->elem())) != LSMF_OK ||
       (s = op->d_diag.alloc((size_t)L.n_dofs() * op->elem())) != LSMF_OK ||
       (s = op->d_inv_diag.alloc((size_t)L.n_dofs() * op->elem())) != LSMF_OK ||
       (s = op->d_flag.alloc(1)) != LSMF_OK) {
