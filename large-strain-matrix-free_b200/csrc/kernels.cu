@@ -185,15 +185,16 @@ lsmf_status for_cell_ranges(const Level &L, int scatter, F &&f) {
   return f(CellRange{});
 }
 
-// The cell ranges of a vmult cell loop.  The production kernel of a
-// deterministic scatter takes whole batches of cells, in groups that share no
+// The cell ranges of a vmult cell loop (the node-sum path's production loops
+// go through apply_node_sum).  The production kernel of a colour8 operator
+// takes whole batches of cells, in groups that share no
 // node, so that its records are read as contiguous slices; the basic kernel
 // takes the cells of the lattice colours.
 template <typename F>
 static lsmf_status for_apply_ranges(const lsmf_op *op, unsigned mask, F &&f) {
   const unsigned all = LSMF_MASK_RW | LSMF_MASK_SF | LSMF_MASK_QD;
   const bool production = !op->basic && (mask & all) == all && !(mask & MASK_INHOM_BIT);
-  if (op->scatter == LSMF_SCATTER_ATOMIC || !production) return for_cell_ranges(op->L(), op->scatter, f);
+  if (op->scatter != LSMF_SCATTER_COLOUR8 || !production) return for_cell_ranges(op->L(), op->scatter, f);
   const Level::BatchGroups &g = op->L().batch_groups[op->precision == LSMF_FP32];
   for (size_t c = 0; c + 1 < g.off.size(); ++c) {
     CellRange r;
@@ -272,7 +273,7 @@ lsmf_status set_scatter_mode(lsmf_op *op, int mode) {
     set_error("scatter must be 0 (atomic), 1 (colour8) or 2 (nodesum)");
     return LSMF_ERR_INVALID_ARG;
   }
-  if (mode != LSMF_SCATTER_ATOMIC) {
+  if (mode == LSMF_SCATTER_COLOUR8) {
     Level::BatchGroups &g = op->L().batch_groups[op->precision == LSMF_FP32];
     if (g.off.empty()) LSMF_TRY(build_batch_groups(op->L(), cells_per_batch(op->L().p, op->precision), g));
   }

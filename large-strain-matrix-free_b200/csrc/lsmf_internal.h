@@ -123,8 +123,8 @@ struct Level {
   std::vector<int> colour_cells;
   int colour_off[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   DevBuf<int> d_colour_cells;
-  // for the production vmult kernel of a deterministic scatter (built when
-  // one is selected): batches of consecutive cells, the cells a warp works on
+  // for the production vmult kernel of the colour8 scatter (built when it is
+  // selected): batches of consecutive cells, the cells a warp works on
   // at a time, in groups whose batches share no node; [0] FP64, [1] FP32
   // batches.  Group c is list[off[c] .. off[c+1])
   struct BatchGroups {
