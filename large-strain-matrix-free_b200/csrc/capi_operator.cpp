@@ -420,17 +420,25 @@ lsmf_status lsmf_operator_get_table(lsmf_op *op, int which, double *host, size_t
   std::vector<char> raw(op->d_table.n);
   LSMF_CUDA(cudaStreamSynchronize(op->stream));
   LSMF_CUDA(cudaMemcpy(raw.data(), op->d_table.ptr, raw.size(), cudaMemcpyDeviceToHost));
-  for (int cell = 0; cell < L.n_cells; ++cell)
-    for (int q = 0; q < nq; ++q)
-      for (int k = 0; k < nk; ++k) {
-        // the full matrices of tables 3 and 7 from their stored upper triangles
-        const int N = which == 3 ? 6 : 9, i = k / N, j = k % N;
-        const int kk = which == 3 || which == 7 ? std::min(i, j) * N - std::min(i, j) * (std::min(i, j) - 1) / 2 + std::abs(j - i) : k;
-        const size_t src = record_index(op, cell, c0 + kk, q);
-        const double v = op->precision == LSMF_FP64 ? ((const double *)raw.data())[src]
-                                                    : (double)((const float *)raw.data())[src];
-        host[((size_t)cell * nq + q) * nk + k] = v;
-      }
+  // offsets of a value in its cell's record, once for all cells (RecLayout:
+  // record_index(cell, comp, q) = record_index(cell, 0, 0) + offset); the full
+  // matrices of tables 3 and 7 from their stored upper triangles
+  std::vector<size_t> off((size_t)nq * nk);
+  for (int q = 0; q < nq; ++q)
+    for (int k = 0; k < nk; ++k) {
+      const int N = which == 3 ? 6 : 9, i = std::min(k / N, k % N), j = std::max(k / N, k % N);
+      const int kk = which == 3 || which == 7 ? i * N - i * (i - 1) / 2 + (j - i) : k;
+      off[(size_t)q * nk + k] = record_index(op, 0, c0 + kk, q);
+    }
+  auto copy = [&](const auto *table) {
+    for (int cell = 0; cell < L.n_cells; ++cell) {
+      const auto *rec = table + record_index(op, cell, 0, 0);
+      double *out = host + (size_t)cell * off.size();
+      for (size_t i = 0; i < off.size(); ++i) out[i] = (double)rec[off[i]];
+    }
+  };
+  if (op->precision == LSMF_FP64) copy((const double *)raw.data());
+  else copy((const float *)raw.data());
   return LSMF_OK;
 }
 
