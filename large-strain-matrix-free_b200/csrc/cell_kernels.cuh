@@ -490,6 +490,25 @@ struct SF {
   }
 };
 
+// dst += the values of a lane's line, without atomics (a colour of the lattice:
+// no other lane of the launch has the line's nodes): all loads before the
+// first store, one round trip where value-by-value adds take one after the
+// other (the compiler may not move a load over a store to the same vector).
+// Entries whose component is constrained in the packed node ids are skipped.
+template <int N1, typename T>
+__device__ __forceinline__ void add_line_plain(T *dst, const int ck[N1], const T out[3][N1]) {
+  T old[N1][3];
+#pragma unroll
+  for (int k = 0; k < N1; ++k)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) old[k][i] = dst[3 * (size_t)(ck[k] & NODE_MASK) + i];
+#pragma unroll
+  for (int k = 0; k < N1; ++k)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (!((ck[k] >> (NODE_BITS + i)) & 1)) dst[3 * (size_t)(ck[k] & NODE_MASK) + i] = old[k][i] + out[i][k];
+}
+
 // --------------------------------------------------------------- physics
 // symmetric storage (0,0),(1,1),(2,2),(0,1),(0,2),(1,2)
 __device__ __forceinline__ int sym_i(int I) { return I < 3 ? I : (I == 5 ? 1 : 0); }

@@ -1095,12 +1095,14 @@ __global__ void __launch_bounds__(128) diagonal_kernel(KArgs<T> a, TabT<P, Q, T>
         out[c][k] = s;
       }
     }
-    if (valid) {
+    if (valid && a.plain) {
+      add_line_plain<N1>(a.dst, ck, out);
+    } else if (valid) {
 #pragma unroll
       for (int k = 0; k < N1; ++k)
 #pragma unroll
         for (int i = 0; i < 3; ++i)
-          if (!((ck[k] >> (NODE_BITS + i)) & 1)) scatter_add(a.dst + 3 * (size_t)(ck[k] & NODE_MASK) + i, out[i][k], a.plain);
+          if (!((ck[k] >> (NODE_BITS + i)) & 1)) atomic_add(a.dst + 3 * (size_t)(ck[k] & NODE_MASK) + i, out[i][k]);
     }
   }
 }

@@ -703,17 +703,18 @@ __global__ void __launch_bounds__(128) internal_force_kernel(const int *__restri
     double out[3][N1];
     S::integrate(tab, G, slab, lp, out);
     double acc = 0;
+    if (MODE == 0 && plain) {
+      if (valid) add_line_plain<N1>(R, ck, out);
+    } else {
 #pragma unroll
-    for (int k = 0; k < N1; ++k)
+      for (int k = 0; k < N1; ++k)
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const size_t dof = 3 * (size_t)ck[k] + i;
-        if (MODE == 1) acc += lam[dof] * out[i][k];
-        else if (valid) {
-          if (plain) R[dof] += out[i][k];
-          else atomicAdd(R + dof, out[i][k]);
+        for (int i = 0; i < 3; ++i) {
+          const size_t dof = 3 * (size_t)ck[k] + i;
+          if (MODE == 1) acc += lam[dof] * out[i][k];
+          else if (valid) atomicAdd(R + dof, out[i][k]);
         }
-      }
+    }
     if (MODE == 1) {
       // the cell's lanes in order
       __syncwarp();
