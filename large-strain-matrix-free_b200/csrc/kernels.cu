@@ -20,8 +20,11 @@ namespace lsmf {
 namespace {
 
 // ------------------------------------------------------ element-wise ops
+// dst += src on the constrained dofs.  No cell loop adds to those, so one
+// launched as its programmatic dependent may start at once.
 template <typename T>
 __global__ void constrained_add_kernel(T *dst, const T *src, const int *idx, int n) {
+  asm volatile("griddepcontrol.launch_dependents;");
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int k = idx[i];
     dst[k] += src[k];
@@ -432,6 +435,20 @@ static lsmf_status apply_chunked(const lsmf_op *op, const OpsTable *t, const Chu
   return LSMF_OK;
 }
 
+// identity rows on top of what dst holds: dst += src (mf_nh_operator.h:702-705)
+static lsmf_status add_rows(const lsmf_op *op, void *dst, const void *src) {
+  const Level &L = op->L();
+  const int nc = (int)L.constrained.size();
+  if (!nc) return LSMF_OK;
+  const int g = (nc + 255) / 256 < 4 * num_sms() ? (nc + 255) / 256 : 4 * num_sms();
+  if (op->precision == LSMF_FP64)
+    constrained_add_kernel<double><<<g, 256, 0, op->stream>>>((double *)dst, (const double *)src, L.d_constrained.ptr, nc);
+  else
+    constrained_add_kernel<float><<<g, 256, 0, op->stream>>>((float *)dst, (const float *)src, L.d_constrained.ptr, nc);
+  LSMF_CUDA(cudaGetLastError());
+  return LSMF_OK;
+}
+
 lsmf_status launch_apply(const lsmf_op *op, void *dst, const void *src, unsigned mask, bool add) {
   const Level &L = op->L();
   const OpsTable *t = table_of(op);
@@ -446,28 +463,25 @@ lsmf_status launch_apply(const lsmf_op *op, void *dst, const void *src, unsigned
       if (cp) return apply_chunked(op, t, *cp, dst, src, mask, !add && (mask & LSMF_MASK_ZERO));
     }
     const bool zero = !add && (mask & LSMF_MASK_ZERO), rows = mask & LSMF_MASK_RW;
+    // the rows come first: the cell loop adds nothing to constrained dofs
+    // (mf_nh_operator.h:702-705) and, as the dependent of the rows' launch,
+    // hides its own start behind it (vmult_add of 8^3 Q2 tensor4 FP64 in a
+    // graph: 6.09 us with the rows last, 5.56 us)
+    bool dependent = rows && (zero || !L.constrained.empty());
     if (zero && rows) LSMF_TRY(identity_rows(op, dst, src, 0, n, op->stream));
     else if (zero) LSMF_CUDA(cudaMemsetAsync(dst, 0, n * op->elem(), op->stream));
+    else if (rows) LSMF_TRY(add_rows(op, dst, src));
     LSMF_TRY(for_apply_ranges(op, mask, [&](CellRange r) {
       // the scatter of the first launch has to wait for the rows, that of
       // every further group of batches for the group before (small levels
       // are bound by the launches: 16^3 Q2 has 12 groups)
-      r.dependent = r.cells ? r.dependent : zero && rows;
+      r.dependent = r.dependent || dependent;
+      dependent = false;
       return t->apply(op, dst, src, mask, r);
     }));
-    if (zero && rows) return LSMF_OK;
+    return LSMF_OK;
   }
-  // constrained rows: dst += src (mf_nh_operator.h:702-705)
-  const int nc = (int)L.constrained.size();
-  if (nc && (mask & LSMF_MASK_RW)) {
-    const int g = (nc + 255) / 256 < 4 * num_sms() ? (nc + 255) / 256 : 4 * num_sms();
-    if (op->precision == LSMF_FP64)
-      constrained_add_kernel<double><<<g, 256, 0, op->stream>>>((double *)dst, (const double *)src, L.d_constrained.ptr, nc);
-    else
-      constrained_add_kernel<float><<<g, 256, 0, op->stream>>>((float *)dst, (const float *)src, L.d_constrained.ptr, nc);
-    LSMF_CUDA(cudaGetLastError());
-  }
-  return LSMF_OK;
+  return (mask & LSMF_MASK_RW) ? add_rows(op, dst, src) : LSMF_OK;
 }
 
 // Cell loop of a partitioned FP64 vmult with the interface exchange fused
