@@ -102,24 +102,27 @@ lsmf_status identity_rows(const lsmf_op *op, void *dst, const void *src, size_t 
 
 // node-sum scatter: dst (+)= the sum over the node's cells, in increasing
 // cell order, of the node's slot in the per-cell buffer (a fixed order: the
-// result is the same from call to call)
+// result is the same from call to call), and with `rows` the identity rows:
+// the slots of constrained dofs hold zeros, src is added there (as a launch of
+// their own after this one the rows cost 1-2 us on small levels and 8 of 365
+// us at 60^3 Q2 tensor4 FP64)
 template <typename T>
 __global__ void node_sum_kernel(T *dst, const T *__restrict__ buf, const int *__restrict__ off,
-                                const int *__restrict__ ent, int n_nodes, int add) {
+                                const int *__restrict__ ent, int n_nodes, int add, const T *__restrict__ src,
+                                const uint8_t *__restrict__ cmask, int rows) {
   for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < n_nodes; n += gridDim.x * blockDim.x) {
-    T s0 = 0, s1 = 0, s2 = 0;
+    T s[3] = {T(0), T(0), T(0)};
     const int e1 = __ldg(off + n + 1);
     for (int e = __ldg(off + n); e < e1; ++e) {
       const int b = __ldg(ent + e);
-      s0 += buf[b];
-      s1 += buf[b + 1];
-      s2 += buf[b + 2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) s[i] += buf[b + i];
     }
-    T *d = dst + 3 * (size_t)n;
-    if (add) {
-      d[0] += s0; d[1] += s1; d[2] += s2;
-    } else {
-      d[0] = s0; d[1] = s1; d[2] = s2;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const size_t d = 3 * (size_t)n + i;
+      if (rows && __ldg(cmask + d)) s[i] += __ldg(src + d);
+      dst[d] = add ? dst[d] + s[i] : s[i];
     }
   }
 }
@@ -251,7 +254,7 @@ static bool node_sum_path(const lsmf_op *op, unsigned mask) {
 
 // cell loop into the operator's cell buffer, then dst (+)= node sums
 static lsmf_status apply_node_sum(const lsmf_op *op, const OpsTable *t, void *dst, const void *src, unsigned mask,
-                                  bool add) {
+                                  bool add, bool rows) {
   const Level &L = op->L();
   if (!op->d_cellbuf.ptr || !L.d_node_cell_off.ptr) {
     set_error("node-sum scatter selected without its buffers");
@@ -261,12 +264,13 @@ static lsmf_status apply_node_sum(const lsmf_op *op, const OpsTable *t, void *ds
   r.cellbuf = op->d_cellbuf.ptr;
   LSMF_TRY(t->apply(op, dst, src, mask, r));
   const int g = std::min((L.n_nodes + 255) / 256, 8 * num_sms());
-  if (op->precision == LSMF_FP64)
-    node_sum_kernel<double><<<g, 256, 0, op->stream>>>((double *)dst, (const double *)op->d_cellbuf.ptr,
-                                                      L.d_node_cell_off.ptr, L.d_node_cell_ent.ptr, L.n_nodes, add);
-  else
-    node_sum_kernel<float><<<g, 256, 0, op->stream>>>((float *)dst, (const float *)op->d_cellbuf.ptr,
-                                                     L.d_node_cell_off.ptr, L.d_node_cell_ent.ptr, L.n_nodes, add);
+  auto sum = [&](auto zero) {
+    using T = decltype(zero);
+    node_sum_kernel<T><<<g, 256, 0, op->stream>>>((T *)dst, (const T *)op->d_cellbuf.ptr, L.d_node_cell_off.ptr,
+                                                  L.d_node_cell_ent.ptr, L.n_nodes, add, (const T *)src, L.d_cmask.ptr, rows);
+  };
+  if (op->precision == LSMF_FP64) sum(0.0);
+  else sum(0.0f);
   LSMF_CUDA(cudaGetLastError());
   return LSMF_OK;
 }
@@ -454,34 +458,30 @@ lsmf_status launch_apply(const lsmf_op *op, void *dst, const void *src, unsigned
   const OpsTable *t = table_of(op);
   if (!t) return LSMF_ERR_UNSUPPORTED;
   const size_t n = (size_t)L.n_dofs();
-  if (node_sum_path(op, mask)) {
-    LSMF_TRY(apply_node_sum(op, t, dst, src, mask, add || !(mask & LSMF_MASK_ZERO)));
-  } else {
-    if (chunkable(op, mask)) {
-      const ChunkPlan *cp = nullptr;
-      LSMF_TRY(chunk_plan(op, chunk_count(op), &cp));
-      if (cp) return apply_chunked(op, t, *cp, dst, src, mask, !add && (mask & LSMF_MASK_ZERO));
-    }
-    const bool zero = !add && (mask & LSMF_MASK_ZERO), rows = mask & LSMF_MASK_RW;
-    // the rows come first: the cell loop adds nothing to constrained dofs
-    // (mf_nh_operator.h:702-705) and, as the dependent of the rows' launch,
-    // hides its own start behind it (vmult_add of 8^3 Q2 tensor4 FP64 in a
-    // graph: 6.09 us with the rows last, 5.56 us)
-    bool dependent = rows && (zero || !L.constrained.empty());
-    if (zero && rows) LSMF_TRY(identity_rows(op, dst, src, 0, n, op->stream));
-    else if (zero) LSMF_CUDA(cudaMemsetAsync(dst, 0, n * op->elem(), op->stream));
-    else if (rows) LSMF_TRY(add_rows(op, dst, src));
-    LSMF_TRY(for_apply_ranges(op, mask, [&](CellRange r) {
-      // the scatter of the first launch has to wait for the rows, that of
-      // every further group of batches for the group before (small levels
-      // are bound by the launches: 16^3 Q2 has 12 groups)
-      r.dependent = r.dependent || dependent;
-      dependent = false;
-      return t->apply(op, dst, src, mask, r);
-    }));
-    return LSMF_OK;
+  // (the node-sum path applies to full cell loops: gather and scatter, rows too)
+  if (node_sum_path(op, mask)) return apply_node_sum(op, t, dst, src, mask, add || !(mask & LSMF_MASK_ZERO), true);
+  if (chunkable(op, mask)) {
+    const ChunkPlan *cp = nullptr;
+    LSMF_TRY(chunk_plan(op, chunk_count(op), &cp));
+    if (cp) return apply_chunked(op, t, *cp, dst, src, mask, !add && (mask & LSMF_MASK_ZERO));
   }
-  return (mask & LSMF_MASK_RW) ? add_rows(op, dst, src) : LSMF_OK;
+  const bool zero = !add && (mask & LSMF_MASK_ZERO), rows = mask & LSMF_MASK_RW;
+  // the rows come first: the cell loop adds nothing to constrained dofs
+  // (mf_nh_operator.h:702-705) and, as the dependent of the rows' launch,
+  // hides its own start behind it (vmult_add of 8^3 Q2 tensor4 FP64 in a
+  // graph: 6.09 us with the rows last, 5.56 us)
+  bool dependent = rows && (zero || !L.constrained.empty());
+  if (zero && rows) LSMF_TRY(identity_rows(op, dst, src, 0, n, op->stream));
+  else if (zero) LSMF_CUDA(cudaMemsetAsync(dst, 0, n * op->elem(), op->stream));
+  else if (rows) LSMF_TRY(add_rows(op, dst, src));
+  return for_apply_ranges(op, mask, [&](CellRange r) {
+    // the scatter of the first launch has to wait for the rows, that of
+    // every further group of batches for the group before (small levels
+    // are bound by the launches: 16^3 Q2 has 12 groups)
+    r.dependent = r.dependent || dependent;
+    dependent = false;
+    return t->apply(op, dst, src, mask, r);
+  });
 }
 
 // Cell loop of a partitioned FP64 vmult with the interface exchange fused
@@ -511,7 +511,7 @@ lsmf_status launch_apply_cells(const lsmf_op *op, void *dst, const void *src) {
   const OpsTable *t = table_of(op);
   if (!t) return LSMF_ERR_UNSUPPORTED;
   const unsigned mask = LSMF_MASK_RW | LSMF_MASK_SF | LSMF_MASK_QD;
-  if (node_sum_path(op, mask)) return apply_node_sum(op, t, dst, src, mask, true);
+  if (node_sum_path(op, mask)) return apply_node_sum(op, t, dst, src, mask, true, false);
   if (chunkable(op, mask)) {
     // the chunks' cell loops only, concurrent (nothing to zero)
     const ChunkPlan *cp = nullptr;
