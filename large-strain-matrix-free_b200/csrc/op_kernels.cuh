@@ -566,13 +566,17 @@ __device__ __forceinline__ void line_point(T G[3][3], int s, const R &slice, con
 }
 
 // Blocks of 128 threads the register allocation leaves room for: three (168
-// registers, 12 warps per SM) up to degree 2, where the working set fits
-// (60^3 Q2 FP64: tensor4 311 -> 303 us, scalar 367 -> 348, scalar_referential
-// 338 -> 329; 96^3 Q1 scalar 331 -> 315, formulation 0 387 -> 349; four
-// blocks, 128 registers, spill: tensor4 363), and for tensor2 at degree 3
-// (167 -> 161); two from there on (255 registers; 36^3 Q4 tensor4 376
-// against 438 us) and for the FP32 scalar_referential Q2 kernel (194 against
-// 210 us).
+// registers, 12 warps per SM) up to degree 2 (60^3 Q2 FP64: tensor4 311 -> 303
+// us, scalar 367 -> 348, scalar_referential 338 -> 329; 96^3 Q1 scalar 331 ->
+// 315, formulation 0 387 -> 349; four blocks, 128 registers, spill: tensor4
+// 363), and for tensor2 at degree 3 (167 -> 161); two from there on (255
+// registers; 36^3 Q4 tensor4 376 against 438 us) and for the FP32
+// scalar_referential Q2 kernel (194 against 210 us).  The Q2 kernels of the
+// scalar types do not fit in 168 registers: they spill 116-220 bytes a thread
+// in FP64, 184 (formulation 1) and 352 (formulation 0) in FP32, and three
+// blocks are the better choice in spite of it, but for FP32 formulation 0: 60^3
+// FP32 formulation 1 207 us against 213 with two blocks (no spills),
+// formulation 0 249 against 244.
 template <int P, int VAR, bool FP32>
 constexpr int line_min_blocks() {
   if (P == 2 && VAR == VAR_SCALAR_REF && FP32) return 2;
@@ -600,11 +604,9 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   const int D = RING ? a.ring : 0;
   const uint32_t slice_bytes = (uint32_t)(a.slice_elems * sizeof(E));
   const size_t warp_bytes = line_warp_bytes<P, Q, T, SCALAR>(D, slice_bytes);
-  if (smem_short(WPB * warp_bytes, a.flag)) {
-    // the launch is not to end before the one whose dependent it is
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    return;
-  }
+  // too little shared memory: no unit is taken (a return here instead of this
+  // cost small levels up to 0.3 us)
+  const bool none = smem_short(WPB * warp_bytes, a.flag);
   // A colour group's successor waits for this whole launch before its first
   // scatter, so it may start, load and compute from here on (colour8 vmult
   // tensor4 FP64 at Q2: 8^3 53.9 -> 23.9 us, 60^3 452 -> 420 us)
@@ -614,7 +616,7 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   T *slab = (T *)(wbase + D * slice_bytes + 16 * ((D + 1) / 2));
   T *park = slab + S::SZ + lp.ln;  // entry (s, c, e) at ((s * 3 + c) * 3 + e) * LW
   const int gw = blockIdx.x * WPB + warp, nw = gridDim.x * WPB;
-  const int n_units = COL ? a.n_batches : UM::units(a.n_cells);
+  const int n_units = none ? 0 : COL ? a.n_batches : UM::units(a.n_cells);
   // batch of a unit, counted from a.cell0 (a multiple of the batch size)
   auto batch = [&](int w) -> int { return COL ? __ldg(a.cells + w) : w; };
   auto batch_ptr = [&](int w) -> const E * { return a.table + (size_t)(a.cell0 / RL::B + batch(w)) * a.batch_elems; };
@@ -625,7 +627,7 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   };
   if (RING) {
     pol = evict_first_policy();
-    if (lane == 0) {
+    if (lane == 0 && gw < n_units) {
       for (int d = 0; d < D; ++d) mbar_init(&bar[d], 1);
       mbar_init_fence();
     }
@@ -684,6 +686,10 @@ __global__ void __launch_bounds__(128, line_min_blocks<P, VAR, Num<T>::H == 2>()
   if (gw < n_units) {
     prefetch(gw);
     prefetch_ref(gw);
+  } else {
+    // a launch is not to end before the one whose dependent it is, also
+    // where none of its warps has a unit
+    asm volatile("griddepcontrol.wait;" ::: "memory");
   }
   for (int w = gw; w < n_units; w += nw) {
     int ck[H][N1];
