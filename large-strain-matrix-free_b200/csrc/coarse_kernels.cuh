@@ -1,7 +1,6 @@
 // Coarse-level solver kernel, included by op_kernels.cuh inside its
-// namespace: the Chebyshev iteration of a level whose cell records fit in
-// the shared memory of all SMs together (coarse_plan.h), as one cooperative
-// launch.
+// namespace: the Chebyshev iteration of a level whose cells one CTA per SM
+// takes (coarse_plan.h), as one cooperative launch.
 //
 // The coarse solve of the V-cycle takes hundreds of Chebyshev steps on a few
 // thousand cells.  As two launches per step (cell loop, update) a step is
@@ -204,32 +203,32 @@ struct Packet<double> {
   }
 };
 
-// The cell operator of a CTA: one unit of cells per working warp, records
-// and index lists loaded once.
+// The cell operator of a CTA: one unit of CPW cells per working warp, one cell
+// per lane in both precisions, records and index lists loaded once.
 template <int P, int Q, typename T, int VAR>
 struct CoarseCells {
   using E = typename Num<T>::S;
-  static constexpr int H = Num<T>::H, TH = table_halves<E>();
+  static constexpr int TH = table_halves<E>();
   using TR = CoarseTraits<P, Q, T, VAR>;
   using S = typename TR::S;
   using RL = RecLayout<P, Q, TH>;
-  static constexpr int N1 = P + 1, NN = S::NN, L = S::L, CPW = S::CPW, LW = S::LW, B = CPW * H;
+  static constexpr int N1 = P + 1, NN = S::NN, L = S::L, CPW = S::CPW, LW = S::LW;
   static constexpr int XS = coarse_stride<E>();
-  static_assert(H == 1, "one cell per lane");
+  static_assert(Num<T>::H == 1, "one cell per lane");
   static_assert(CPW * NN * XS <= S::SZ, "the cells' results fit in the slab");
   const TabT<P, Q, T> &tab;
   LanePos<Q> lp;
   T *rec, *ref, *slab, *park;
   int SS;
   bool ref_per_cell, active;
-  int lid[H][N1];
+  int lid[N1];
   T mu, lambda, kappa;
 
   __device__ __forceinline__ CoarseCells(const KArgs<E> &a, const TabT<P, Q, T> &t, const CoarseArgs<E> &ca, unsigned char *smem)
       : tab(t) {
     const int warp = threadIdx.x >> 5, cta = blockIdx.x;
     const int n_cells = ca.counts[4 * cta];
-    active = warp < ca.warps && warp * B < n_cells;
+    active = warp < ca.warps && warp * CPW < n_cells;
     ref_per_cell = a.ref_per_cell != 0;
     SS = a.slice_elems / TH;
     unsigned char *base = smem + (size_t)warp * ca.unit_bytes;
@@ -238,51 +237,28 @@ struct CoarseCells {
     slab = (T *)(base + coarse_out_offset<P, Q, T, VAR>(a.slice_elems));
     park = (T *)((unsigned char *)slab + coarse_slab_bytes<P, Q, T, VAR>()) + lp.ln;
     if (!active) return;
-    E m[3][H];
-    const E *src[H], *rsrc[H];
-    const int *cn[H];
+    const int slot = warp * CPW + lp.r;
+    const int ce = ca.cells[(size_t)cta * ca.cells_per_cta + slot], cell = ce < 0 ? -1 - ce : ce;
+    material<E>(a.mu[cell], a.nu, mu, lambda, kappa);
+    const E *src = a.table + RL::base(cell, a.batch_elems) + lp.t * TH;
+    const uint16_t *l = ca.lid + ((size_t)cta * ca.cells_per_cta + slot) * NN + lp.t;
 #pragma unroll
-    for (int h = 0; h < H; ++h) {
-      const int slot = warp * B + lp.r * H + h;
-      const int ce = ca.cells[(size_t)cta * ca.cells_per_cta + slot], cell = ce < 0 ? -1 - ce : ce;
-      material<E>(a.mu[cell], a.nu, m[0][h], m[1][h], m[2][h]);
-      src[h] = a.table + RL::base(cell, a.batch_elems) + lp.t * TH;
-      rsrc[h] = a.table + RL::ref(cell, a.batch_elems, a.slice_elems);
-      cn[h] = a.cell_nodes + (size_t)cell * NN + lp.t;
-      const uint16_t *l = ca.lid + ((size_t)cta * ca.cells_per_cta + slot) * NN + lp.t;
-#pragma unroll
-      for (int k = 0; k < N1; ++k) lid[h][k] = XS * l[k * L];
-    }
-    mu = join_of<T>(m[0], H - 1);
-    lambda = join_of<T>(m[1], H - 1);
-    kappa = join_of<T>(m[2], H - 1);
+    for (int k = 0; k < N1; ++k) lid[k] = XS * l[k * L];
     const int ncomp = TR::SCALAR && ref_per_cell ? C_VAR + 1 : variant_ncomp(VAR);
     for (int s = 0; s < Q; ++s)
-      for (int c = 0; c < ncomp; ++c) {
-        E x[H];
-#pragma unroll
-        for (int h = 0; h < H; ++h) x[h] = src[h][(size_t)s * a.slice_elems + c * RL::CS];
-        rec[s * SS + c * LW + lp.ln] = join_of<T>(x, H - 1);
-      }
+      for (int c = 0; c < ncomp; ++c) rec[s * SS + c * LW + lp.ln] = src[(size_t)s * a.slice_elems + c * RL::CS];
     if constexpr (TR::SCALAR) {
-      if (ref_per_cell && lp.t == 0)
-        for (int i = 0; i < 9; ++i) {
-          E x[H];
-#pragma unroll
-          for (int h = 0; h < H; ++h) x[h] = rsrc[h][i * RL::RS];
-          ref[i * CPW + lp.r] = join_of<T>(x, H - 1);
-        }
+      if (ref_per_cell && lp.t == 0) {
+        const E *r = a.table + RL::ref(cell, a.batch_elems, a.slice_elems);
+        for (int i = 0; i < 9; ++i) ref[i * CPW + lp.r] = r[i * RL::RS];
+      }
       // the displacement gradients do not change during the solve
       T vu[3][N1], G[Q][3][3];
+      const int *cn = a.cell_nodes + (size_t)cell * NN + lp.t;
 #pragma unroll
       for (int k = 0; k < N1; ++k)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          E x[H];
-#pragma unroll
-          for (int h = 0; h < H; ++h) x[h] = a.u[3 * (size_t)(cn[h][k * L] & NODE_MASK) + i];
-          vu[i][k] = join_of<T>(x, H - 1);
-        }
+        for (int i = 0; i < 3; ++i) vu[i][k] = a.u[3 * (size_t)(cn[k * L] & NODE_MASK) + i];
       S::eval(tab, vu, slab, lp, G);
 #pragma unroll
       for (int s = 0; s < Q; ++s)
@@ -300,7 +276,7 @@ struct CoarseCells {
 #pragma unroll
     for (int k = 0; k < N1; ++k) {
       E x[3];
-      ld3(xg + lid[0][k], x);
+      ld3(xg + lid[k], x);
 #pragma unroll
       for (int i = 0; i < 3; ++i) v[i][k] = x[i];
     }

@@ -1,5 +1,6 @@
 // Work distribution of the coarse-level solver: a level small enough that
-// its cell records fit in the shared memory of all SMs together is solved by
+// one CTA per SM takes all its cells (one batch per warp, and their records
+// in shared memory) is solved by
 // one cooperative kernel (coarse_kernels.cuh).  Every CTA keeps a compact
 // group of cells, sums their contributions to its nodes in shared memory and
 // exchanges only the sums of the nodes it shares with other CTAs.
