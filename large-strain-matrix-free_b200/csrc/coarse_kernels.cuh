@@ -502,11 +502,7 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
     rhok = rhokp;
     if (!nodes.receive((unsigned)k, a.wait_tries)) dead = 1;
     __syncthreads();
-    if (dead) {
-      coarse_no_solution(ca);
-      if (threadIdx.x == 0) atomicOr(a.flag, FLAG_TIMEOUT);
-      return;
-    }
+    if (dead) break;
     nodes.finish();
 #pragma unroll
     for (int q = 0; q < NPT; ++q) {
@@ -522,6 +518,11 @@ __global__ void __launch_bounds__(COARSE_THREADS, 1)
       nodes.put_x(q, x[q]);
     }
     __syncthreads();
+  }
+  if (dead) {
+    coarse_no_solution(ca);
+    if (threadIdx.x == 0) atomicOr(a.flag, FLAG_TIMEOUT);
+    return;
   }
 #pragma unroll
   for (int q = 0; q < NPT; ++q) {
